@@ -42,7 +42,7 @@ L2_BYTES = 126 * 2 ** 20
 METRIC = "stencil Gpts/s (Gray-Scott 7-point, 512^3 sparse grid)"
 UNIT = "Gpts/s"
 ALG_BYTES_PER_PT = 17
-# the library's default launch configuration of the pipelined 8^3 kernel (automatic ring depth)
+# the library's default launch configuration of the 7-point kernel on 8^3 chunks
 DEFAULT_CTAS_PER_SM, DEFAULT_STAGES = "auto", "auto"
 WORKLOADS = ("gs512", "heat128", "insert1024", "batched256", "served", "ghost512", "conv1000", "conv2b")
 
@@ -647,7 +647,7 @@ def run_batched256(args, dist: Dist):
         for k in range(4):
             g.applyStencils(sgb.HEAT7, [k % 2], [1 - k % 2], [W.HEAT_DT])
     torch.cuda.synchronize()
-    # plain drop-in use: one applyStencils launch per grid per step (the pipelined kernel)
+    # plain drop-in use: one applyStencils launch per grid per step (the same kernel)
     p0, p1 = _events()
     p0.record()
     for g in grids:

@@ -1,9 +1,9 @@
 """Launch autotuner for the batched stencil step.
 
-Candidates: chunk edge 8 (pipelined kernel: one 32-thread warp per
-512-point chunk, each warp with its own staging ring, 2-6 CTAs of two warps
-per SM or the automatic choice -1, ring depth 3, 4 or the automatic depth
--1) and chunk edge 4
+Candidates: chunk edge 8 (16 or 32 threads per 512-point chunk, by the
+staging depth: 4 for eight z slices per group of 16 threads, 3 for four, -1
+by the batch's size; at most 4, 6 or 8 CTAs of 128 threads per SM, or -1 for
+no limit) and chunk edge 4
 (one-chunk-per-CTA tile kernel: 256 threads per 64-point chunk).  Each
 candidate runs a few timed batch steps (CUDA events) on a sample of the
 grids, rebuilt with its chunk edge; the fastest per active point wins.
@@ -84,8 +84,9 @@ def autotune(specs: Sequence[Spec], kind: int, params, steps: int = 10, device: 
                 b.set_launch_config(c, s)
             t = _time_steps(b, steps)
             nsps = t / steps / max(pts, 1) * 1e9
-            # 8^3: one consumer warp per chunk in the pipelined kernel; 4^3: one 256-thread CTA per chunk
-            row = {"chunk_edge": ce, "ctas_per_sm": c, "stages": s, "threads_per_chunk": 32 if ce == 8 else 256,
+            # 8^3: groups of 16 threads, one or two per chunk; 4^3: one 256-thread CTA per chunk
+            row = {"chunk_edge": ce, "ctas_per_sm": c, "stages": s,
+                   "threads_per_chunk": (16 if s >= 4 else 32) if ce == 8 else 256,
                    "ns_per_point_step": round(nsps, 5)}
             table.append(row)
             if best is None or nsps < best["ns_per_point_step"]:

@@ -168,8 +168,7 @@ static int batch_launch(sgb_batch* b, int64_t t, cudaStream_t s) {
     L.use_tile = 0;
     L.stages = b->stages;
     L.num_sms = b->num_sms;
-    const int cps = b->ctas_per_sm > 0 ? b->ctas_per_sm : auto_ctas_per_sm(b->kind);
-    L.ctas = (unsigned)std::max<int64_t>(1, std::min<int64_t>(b->n, (int64_t)b->num_sms * cps));
+    L.ctas_per_sm = b->ctas_per_sm;
     for (int k = 0; k < 2; ++k)
         for (int j = 0; j < 2; ++j) {
             const int p = j < b->np ? j : 0;

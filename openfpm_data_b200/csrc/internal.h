@@ -302,8 +302,8 @@ struct sgb_grid {
 
     sgb::DevBuf err;      // unsigned device error word
     int num_sms = 148;
-    int ctas_per_sm = 0;  // 0: automatic per stencil kind (auto_ctas_per_sm)
-    int stages = 0;       // 0: deepest staging ring that keeps ctas_per_sm CTAs resident
+    int ctas_per_sm = 0;  // 0: no limit on the CTAs per SM of the 7-point kernel
+    int stages = 0;       // z slices it stages per lane group (3: four, more: eight); 0: by the grid's size
 };
 
 namespace sgb {

@@ -1,0 +1,402 @@
+// 7-point stencils (HEAT7, GS7) on 8^3 chunks, for single grids and batches
+// and for any chunk ids.
+//
+// Reference path: applyStencilInPlace (src/SparseGridGpu/SparseGridGpu.hpp:
+// 954-1048) launches one 512-thread CTA per chunk; loadGhostBlock_impl<1>
+// (src/SparseGridGpu/SparseGridGpu_ker_util.hpp:487-564) gathers the 10^3
+// tile point by point and substitutes the background where a mask byte is 0.
+//
+// Work: 16 lanes take ZS (4 or 8) z slices of one chunk; lane l owns the x
+// quad l % 2 of row l / 2 and marches z with z - 1 / z / z + 1 in registers.
+// All of a group's loads are issued at once: its rows and the two y-face rows
+// of every slice by cp.async into a tile in shared memory (80 floats per
+// slice, so that the y neighbours of every lane are plain 16-byte shared
+// loads), the outer x cells and the two z faces into registers.  The x
+// neighbour of a chunk sits at the next or previous position under x-fastest
+// ids, so most x cells are read from the neighbouring group's tile; the one
+// block barrier is there for them.  Blocks do one round and leave: the
+// latencies of one block are covered by the others on the SM, and every block
+// pulls the masks and neighbour rows of a block one wave ahead into L2.
+//
+// Sparsity: a quad none of whose points exists is neither read nor written
+// (points with mask byte 0 hold the background in HBM, which grid.cu and
+// HEAT7's stores keep), so a step moves about the bytes of the existing rows
+// and not of whole chunks.
+//
+// What bounds it: HBM for large grids, where the power cap is reached with
+// it; latency and block turnover for one to four waves of blocks.  Measured
+// on one B200 (us per step, the earlier kernel, a ring of bulk copies per
+// warp over whole chunks, in brackets): Gray-Scott 512^3, 40 balls, 18,932
+// chunks 29.3 (39.2); Gray-Scott 900^3, 200 balls 121-130 (189); heat 48
+// grids of edge 32-384 199-215 = 5.7-6.1 TB/s (331); heat 509x301x211 6.2
+// (9.8); heat 256^3 on Morton ids 5.3 (36.0, one CTA per chunk).  Tried and
+// slower: rows read straight into registers through L1 without the tile
+// (31.4 / heat 228-256), a persistent form with two tiles per group (27.9 for
+// Gray-Scott, but heat 309-330), whole-chunk L2 prefetch (36.5-38.7: the
+// absent rows are fetched too).
+#include <algorithm>
+
+#include "stencil.cuh"
+
+namespace sgb {
+
+constexpr int kStarThreads = 128, kStarGroups = kStarThreads / 16;
+
+// Plain (coherent) global loads: under programmatic dependent launch a block
+// may start before the step that wrote these fields has finished, so the
+// read-only path, which asks for data that is constant while the kernel runs,
+// is not used for fields.
+__device__ __forceinline__ float4 ldf4(const float* p) {
+    float4 v;
+    asm("ld.global.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float ldf1(const float* p) {
+    float v;
+    asm("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+// Waits for the launch before this one; the returned value orders the loads that use it behind the wait.
+__device__ __forceinline__ int64_t grid_dependency_wait() {
+    int64_t z;
+    asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;\n\tmov.u64 %0, 0;" : "=l"(z)::"memory");
+    return z;
+}
+
+__device__ __forceinline__ float4 splat4(float b) { return make_float4(b, b, b, b); }
+
+// Two float32 values in one 64-bit register pair and the packed arithmetic on them (each half rounds as the
+// scalar instruction does).
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pk(float a, float b) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 upk(f32x2 v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+struct Quad {
+    f32x2 a, b;  // points 0, 1 and 2, 3
+};
+__device__ __forceinline__ Quad quad(const float4& v) { return {pk(v.x, v.y), pk(v.z, v.w)}; }
+
+// 7-point Laplacian of an x quad: lap7k of stencil.cuh point by point, the same operations in the same order.
+template <int KIND>
+__device__ __forceinline__ Quad lap_quad(const float4& c, float xm, float xp, const float4& ym, const float4& yp,
+                                         const float4& zm, const float4& zp) {
+    const Quad qym = quad(ym), qyp = quad(yp), qzm = quad(zm), qzp = quad(zp);
+    // the x sums take unaligned pairs: scalar
+    const f32x2 xa = pk(__fadd_rn(xm, c.y), __fadd_rn(c.x, c.z)), xb = pk(__fadd_rn(c.y, c.w), __fadd_rn(c.z, xp));
+    Quad l;
+    if (KIND == SGB_HEAT7) {
+        const f32x2 m6 = pk(-6.0f, -6.0f);
+        const Quad qc = quad(c);
+        l.a = fma2(m6, qc.a, xa);
+        l.b = fma2(m6, qc.b, xb);
+    } else {
+        // -6 c rounds on its own: scalar products, which the assembler leaves apart from the packed sum
+        l.a = add2(pk(__fmul_rn(-6.0f, c.x), __fmul_rn(-6.0f, c.y)), xa);
+        l.b = add2(pk(__fmul_rn(-6.0f, c.z), __fmul_rn(-6.0f, c.w)), xb);
+    }
+    l.a = add2(add2(l.a, add2(qym.a, qyp.a)), add2(qzm.a, qzp.a));
+    l.b = add2(add2(l.b, add2(qym.b, qyp.b)), add2(qzm.b, qzp.b));
+    return l;
+}
+
+// gs_update of two points.
+__device__ __forceinline__ void gs_update2(f32x2 u, f32x2 v, f32x2 lu, f32x2 lv, const GridInfo& g, f32x2& un, f32x2& vn) {
+    const f32x2 uvv = mul2(mul2(u, v), v);
+    const f32x2 one = pk(1.0f, 1.0f), sgn = 0x8000000080000000ull;
+    f32x2 du = fma2(pk(g.Du, g.Du), lu, uvv ^ sgn);
+    du = fma2(pk(g.F, g.F), add2(one, u ^ sgn), du);
+    f32x2 dv = fma2(pk(g.Dv, g.Dv), lv, uvv);
+    dv = fma2(pk(g.nFK, g.nFK), v, dv);
+    un = fma2(pk(g.dt, g.dt), du, u);
+    vn = fma2(pk(g.dt, g.dt), dv, v);
+}
+
+// The update of one x quad and its stores.  m4: the quad's mask bytes; act bit k: point k takes the update.
+template <int KIND, int NP>
+__device__ __forceinline__ void star_store(const float4 (&c)[NP], const Quad (&lap)[NP], uint32_t m4, uint32_t act,
+                                           const GridInfo& gi, const float (&bd)[NP], float* d0, float* d1) {
+    Quad w[NP];
+    const Quad c0 = quad(c[0]);
+    if (KIND == SGB_HEAT7) {
+        const f32x2 dt = pk(gi.dt, gi.dt);
+        w[0].a = fma2(dt, lap[0].a, c0.a);
+        w[0].b = fma2(dt, lap[0].b, c0.b);
+    } else {
+        const Quad c1 = quad(c[NP - 1]);
+        gs_update2(c0.a, c1.a, lap[0].a, lap[NP - 1].a, gi, w[0].a, w[NP - 1].a);
+        gs_update2(c0.b, c1.b, lap[0].b, lap[NP - 1].b, gi, w[0].b, w[NP - 1].b);
+    }
+    float4 o[NP];
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+        const float2 lo = upk(w[p].a), hi = upk(w[p].b);
+        o[p] = make_float4(lo.x, lo.y, hi.x, hi.y);
+    }
+    if (act != 0xfu) {
+        const bool e0 = m4 & 0xffu, e1 = m4 & 0xff00u, e2 = m4 & 0xff0000u, e3 = m4 & 0xff000000u;
+        if (KIND == SGB_HEAT7) {
+            // inactive points: an existing one keeps its value, the others take the destination's background
+            o[0].x = (act & 1u) ? o[0].x : (e0 ? c[0].x : bd[0]);
+            o[0].y = (act & 2u) ? o[0].y : (e1 ? c[0].y : bd[0]);
+            o[0].z = (act & 4u) ? o[0].z : (e2 ? c[0].z : bd[0]);
+            o[0].w = (act & 8u) ? o[0].w : (e3 ? c[0].w : bd[0]);
+        } else {
+            const uint32_t ex = (e0 ? 1u : 0u) | (e1 ? 2u : 0u) | (e2 ? 4u : 0u) | (e3 ? 8u : 0u);
+            if (ex & ~act) {  // existing inactive points (padding, outside the box) are left alone
+                const float u4[4] = {o[0].x, o[0].y, o[0].z, o[0].w};
+                const float v4[4] = {o[NP - 1].x, o[NP - 1].y, o[NP - 1].z, o[NP - 1].w};
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (act >> k & 1u) {
+                        d0[k] = u4[k];
+                        d1[k] = v4[k];
+                    }
+                return;
+            }
+            // points that do not exist take the destination's background, which no read can tell from
+            // what they hold: one whole store
+#pragma unroll
+            for (int p = 0; p < NP; ++p) {
+                o[p].x = (act & 1u) ? o[p].x : bd[p];
+                o[p].y = (act & 2u) ? o[p].y : bd[p];
+                o[p].z = (act & 4u) ? o[p].z : bd[p];
+                o[p].w = (act & 8u) ? o[p].w : bd[p];
+            }
+        }
+    }
+    *reinterpret_cast<float4*>(d0) = o[0];
+    if (NP > 1) *reinterpret_cast<float4*>(d1) = o[NP - 1];
+}
+
+// Bits of the quad's active points: EXIST and not PADDING, inside the box.
+template <bool BOX>
+__device__ __forceinline__ uint32_t active_bits(uint32_t m4, const StencilParams& prm, int x, int y, int z) {
+    // per byte: bit 0 set and bit 1 clear
+    if (!BOX && m4 == 0x01010101u) return 0xfu;
+    uint32_t a = m4 & ~(m4 >> 1) & 0x01010101u;
+    a = (a | a >> 7 | a >> 14 | a >> 21) & 0xfu;
+    if (BOX) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (!in_box(prm, x + k, y, z)) a &= ~(1u << k);
+    }
+    return a;
+}
+
+// A group's part of shared memory: rows -1 .. 8 of ZS slices, per field.
+template <int NP, int ZS>
+struct StarTile {
+    float row[NP][ZS][80];
+};
+
+template <int KIND, int NP, bool BOX, bool BATCH, int ZS, int MINB>
+__global__ void __launch_bounds__(kStarThreads, MINB)
+    k_star7_e8(FieldSet fs, const uint8_t* __restrict__ mask, const int32_t* __restrict__ nn,
+               const int64_t* __restrict__ keys, const int32_t* __restrict__ gid, const GridInfo* __restrict__ grids,
+               GridInfo g0, int64_t n, Geometry geo, StencilParams prm, int64_t t, int fill, int ahead) {
+    constexpr int PARTS = 8 / ZS;
+    extern __shared__ __align__(16) unsigned char star_smem[];
+    StarTile<NP, ZS>* const tiles = reinterpret_cast<StarTile<NP, ZS>*>(star_smem);
+    const int grp = threadIdx.x >> 4;
+    StarTile<NP, ZS>& T = tiles[grp];
+    const int64_t dep = grid_dependency_wait();
+    mask += dep;
+    nn += dep;
+    const int l16 = threadIdx.x & 15, y = l16 >> 1, xq = l16 & 1;
+    const int o0 = y * 8 + xq * 4;
+    const int64_t total = n * PARTS;
+    const int64_t it = (int64_t)blockIdx.x * kStarGroups + grp;
+    bool live = it < total;
+    const int64_t c = live ? it / PARTS : 0;
+    const int zb = PARTS == 1 ? 0 : (int)(it % PARTS) * ZS;
+    GridInfo gb;
+    int par = 0;
+    if (BATCH) {
+        gb = grids[gid[c]];
+        live = live && t >= gb.start && t < gb.start + gb.nsteps;
+        par = (int)((t - gb.start) & 1);
+    }
+    const GridInfo& gi = BATCH ? gb : g0;
+    uint32_t m[ZS];  // mask bytes of the lane's quads
+    const uint8_t* mp = mask + c * 512 + zb * 64 + o0;
+#pragma unroll
+    for (int z = 0; z < ZS; ++z) m[z] = live ? __ldg(reinterpret_cast<const uint32_t*>(mp + z * 64)) : 0u;
+    const int4 na = __ldg(reinterpret_cast<const int4*>(nn + c * 8));
+    const int2 nz = __ldg(reinterpret_cast<const int2*>(nn + c * 8 + 4));
+    const float* src[NP];
+    float bs[NP], bd[NP];  // backgrounds of the source and destination fields
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+        src[p] = (par ? fs.in[1][p] : fs.in[0][p]) + dep;
+        bs[p] = par ? gi.bck[1][p] : gi.bck[0][p];
+        bd[p] = par ? gi.bck[0][p] : gi.bck[1][p];
+    }
+    const int64_t oc = c * 512 + zb * 64 + o0;
+#pragma unroll
+    for (int z = 0; z < ZS; ++z)
+#pragma unroll
+        for (int p = 0; p < NP; ++p) {
+            float* d = &T.row[p][z][8 + o0];
+            if (m[z]) cp_async16(d, src[p] + oc + z * 64);
+            else *reinterpret_cast<float4*>(d) = splat4(bs[p]);
+        }
+    // y faces: lanes 0..7 the -y side, 8..15 the +y side, quad xq of slice (l16 % 8) / 2 + 4 k
+    {
+        const int side = l16 >> 3, zq = (l16 & 7) >> 1;
+        const int32_t ny = side ? na.w : na.z;
+#pragma unroll
+        for (int z = zq; z < ZS; z += 4)
+#pragma unroll
+            for (int p = 0; p < NP; ++p) {
+                float* d = &T.row[p][z][(side ? 72 : 0) + xq * 4];
+                if (live && ny >= 0)
+                    cp_async16(d, src[p] + (int64_t)ny * 512 + (zb + z) * 64 + (side ? 0 : 56) + xq * 4);
+                else *reinterpret_cast<float4*>(d) = splat4(bs[p]);
+            }
+    }
+    cp_async_commit();
+    // the group `ahead` items on: its mask bytes and neighbour row on their way to L2 (3 % at 512^3)
+    if (l16 < 2 && it + ahead < total) {
+        const int64_t ai = it + ahead, ac = ai / PARTS;
+        if (l16 == 0) {
+            const uint8_t* q = mask + ac * 512 + (PARTS == 1 ? 0 : (int)(ai % PARTS) * ZS * 64);
+            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(q), "r"(ZS * 64) : "memory");
+        } else {
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(nn + ac * 8) : "memory");
+        }
+    }
+    // an x neighbour at the next position is another tile of this block
+    const int32_t nx = xq ? na.y : na.x;
+    const int gq = grp / PARTS + (xq ? 1 : -1);
+    const bool in_cta = live && nx >= 0 && nx == c + (xq ? 1 : -1) && gq >= 0 && gq < kStarGroups / PARTS;
+    const float* xs = &tiles[grp + (in_cta ? (xq ? PARTS : -PARTS) : 0)].row[0][0][8 + y * 8 + (xq ? 0 : 7)];
+    const int64_t ox = (int64_t)nx * 512 + zb * 64 + y * 8 + (xq ? 0 : 7);
+    const int64_t ozm = zb > 0 ? oc - 64 : (nz.x >= 0 ? (int64_t)nz.x * 512 + 448 + o0 : -1);
+    const int64_t ozp = zb + ZS < 8 ? oc + ZS * 64 : (nz.y >= 0 ? (int64_t)nz.y * 512 + o0 : -1);
+    float4 zm[NP], zl[NP], cv[NP];
+    float xh[ZS][NP];
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+        zm[p] = splat4(bs[p]);
+        zl[p] = splat4(bs[p]);
+        if (m[0] && ozm >= 0) zm[p] = ldf4(src[p] + ozm);
+        if (m[ZS - 1] && ozp >= 0) zl[p] = ldf4(src[p] + ozp);
+    }
+#pragma unroll
+    for (int z = 0; z < ZS; ++z)
+#pragma unroll
+        for (int p = 0; p < NP; ++p) {
+            xh[z][p] = bs[p];
+            if (m[z] && nx >= 0 && !in_cta) xh[z][p] = ldf1(src[p] + ox + z * 64);
+        }
+    int32_t cx = 0, cy = 0, cz = 0;
+    if (BOX) {
+        int64_t o[3];
+        chunk_origin(geo, keys[c], o);
+        cx = (int32_t)o[0] + xq * 4;
+        cy = (int32_t)o[1] + y;
+        cz = (int32_t)o[2] + zb;
+    }
+    float* dst[NP];
+#pragma unroll
+    for (int p = 0; p < NP; ++p) dst[p] = (par ? fs.out[1][p] : fs.out[0][p]) + oc;
+    cp_async_wait_all();
+    __syncthreads();
+#pragma unroll
+    for (int p = 0; p < NP; ++p) cv[p] = *reinterpret_cast<const float4*>(&T.row[p][0][8 + o0]);
+#pragma unroll
+    for (int z = 0; z < ZS; ++z) {
+        Quad lap[NP];
+        float4 zp[NP];
+#pragma unroll
+        for (int p = 0; p < NP; ++p) {
+            zp[p] = z + 1 < ZS ? *reinterpret_cast<const float4*>(&T.row[p][z + 1 < ZS ? z + 1 : 0][8 + o0]) : zl[p];
+            const float4 ym = *reinterpret_cast<const float4*>(&T.row[p][z][o0]);
+            const float4 yp = *reinterpret_cast<const float4*>(&T.row[p][z][16 + o0]);
+            // the inner x cell is the partner quad's edge
+            const float got = __shfl_xor_sync(0xffffffffu, xq ? cv[p].x : cv[p].w, 1);
+            float xo = xh[z][p];
+            if (in_cta) xo = xs[(p * ZS + z) * 80];
+            lap[p] = lap_quad<KIND>(cv[p], xq ? got : xo, xq ? xo : got, ym, yp, zm[p], zp[p]);
+        }
+        if (m[z] || (KIND == SGB_HEAT7 && fill && live)) {
+            const uint32_t act = active_bits<BOX>(m[z], prm, cx, cy, cz + z);
+            star_store<KIND, NP>(cv, lap, m[z], act, gi, bd, dst[0] + z * 64, dst[NP - 1] + z * 64);
+        }
+#pragma unroll
+        for (int p = 0; p < NP; ++p) {
+            zm[p] = cv[p];
+            cv[p] = zp[p];
+        }
+    }
+}
+
+template <int KIND, int NP, bool BOX, bool BATCH, int ZS, int MINB>
+static int launch_star(const LaunchDesc& L, cudaStream_t s) {
+    auto kern = k_star7_e8<KIND, NP, BOX, BATCH, ZS, MINB>;
+    const int64_t items = L.n * (8 / ZS);
+    size_t smem = sizeof(StarTile<NP, ZS>) * kStarGroups;
+    // a caller's limit on the CTAs per SM: each CTA takes its share of the SM's shared memory
+    if (L.ctas_per_sm > 0) smem = std::max(smem, (size_t)(227 * 1024 / L.ctas_per_sm - 1024) & ~(size_t)127);
+    SGB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)((items + kStarGroups - 1) / kStarGroups));
+    cfg.blockDim = dim3(kStarThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    // consecutive steps overlap one launch's ramp-up with the previous one's tail
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const int ahead = L.num_sms * 7 * kStarGroups;  // about the groups resident at a time
+    SGB_CUDA(cudaLaunchKernelEx(&cfg, kern, L.fs, L.mask, L.nn, L.keys, L.gid, L.grids, L.g0, L.n, L.geo, L.prm, L.t,
+                                L.fill, ahead));
+    return SGB_OK;
+}
+
+template <int KIND, int NP, int ZS, int MINB>
+static int launch_star_kind(const LaunchDesc& L, cudaStream_t s) {
+    constexpr int BATCHB = KIND == SGB_GS7 && ZS == 4 ? MINB - 1 : MINB;  // the grid entry takes registers
+    if (L.grids) return launch_star<KIND, NP, false, true, ZS, BATCHB>(L, s);
+    if (L.prm.has_box) return launch_star<KIND, NP, true, false, ZS, MINB>(L, s);
+    return launch_star<KIND, NP, false, false, ZS, MINB>(L, s);
+}
+
+// Slices per group.  Eight halve the z-face loads and the instructions per point, four fill the chip with half
+// as many chunks.  Heat: eight from two full waves of such blocks on (us per step, 4 against 8: 5,637 chunks
+// 5.3 / 8.0, 18,932 chunks 12.8 / 12.5, 33,000 chunks 33.3 / 31.7, 300,000 chunks 241 / 212).  Gray-Scott
+// keeps four: the same time within 2 % at every size, and eight need 41 KB and 92 registers a block.  (Heat
+// with eight slices fits 8 blocks of 128 threads on an SM, with four 10; Gray-Scott 7: no spills.)
+int launch_star7(const LaunchDesc& L, cudaStream_t s) {
+    bool eight = L.kind == SGB_HEAT7 && L.n >= (int64_t)2 * L.num_sms * 8 * kStarGroups;
+    if (L.stages > 0) eight = L.stages >= 4;
+    if (L.kind == SGB_GS7)
+        return eight ? launch_star_kind<SGB_GS7, 2, 8, 4>(L, s) : launch_star_kind<SGB_GS7, 2, 4, 7>(L, s);
+    return eight ? launch_star_kind<SGB_HEAT7, 1, 8, 8>(L, s) : launch_star_kind<SGB_HEAT7, 1, 4, 10>(L, s);
+}
+
+}  // namespace sgb

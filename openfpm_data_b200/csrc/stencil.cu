@@ -6,9 +6,9 @@
 // the 10^3 tile with one scalar load per point, the user functor computes,
 // storeBlock writes back.
 //
-// Here 7-point stencils on 8^3 chunks run the pipelined kernel of
-// stencil8.cu; this file holds the generic one-chunk-per-CTA tile kernel
-// (BOX27, 4^3 chunks, cross-checks), parameter handling and dispatch.
+// Here 7-point stencils on 8^3 chunks run the kernel of star7.cu; this file
+// holds the generic one-chunk-per-CTA tile kernel (4^3 chunks, cross-checks),
+// Conv3x3x3 on 8^3 chunks, parameter handling and dispatch.
 //
 // The same kernels run a batch of grids concatenated into one block map: a
 // per-chunk grid id selects the grid's parameters and its ping-pong buffer
@@ -522,9 +522,7 @@ GridInfo grid_info_of(const StencilParams& prm) {
 
 int launch_fields(const LaunchDesc& L, cudaStream_t s) {
     if (L.n == 0) return SGB_OK;
-    // the pipelined kernel takes the x halo from the neighbouring index positions, which hold the
-    // x neighbours only under the x-fastest chunk ids
-    if (L.kind != SGB_BOX27 && L.edge == 8 && !L.use_tile && !L.geo.zorder) return launch_e8(L, s);
+    if (L.kind != SGB_BOX27 && L.edge == 8 && !L.use_tile) return launch_star7(L, s);
     if (L.kind == SGB_BOX27 && L.edge == 8 && !L.use_tile && !L.grids) {
         // 4 CTAs of four warps per SM are resident (128 registers a thread)
         const int64_t want = (L.n + kW27Warps - 1) / kW27Warps;
@@ -571,8 +569,7 @@ int launch_stencil_impl(sgb_grid* g, int kind, const int* src, const int* dst, c
     L.use_tile = use_tile;
     L.stages = g->stages;
     L.num_sms = g->num_sms;
-    const int cps = g->ctas_per_sm > 0 ? g->ctas_per_sm : auto_ctas_per_sm(kind);
-    L.ctas = (unsigned)std::max<int64_t>(1, std::min<int64_t>(g->n, (int64_t)g->num_sms * cps));
+    L.ctas_per_sm = g->ctas_per_sm;
     for (int b = 0; b < 2; ++b)
         for (int j = 0; j < 2; ++j) {
             L.fs.in[b][j] = g->data[src[j < np ? j : 0]].as<float>();
@@ -589,6 +586,7 @@ int launch_stencil_impl(sgb_grid* g, int kind, const int* src, const int* dst, c
     L.geo = g->geo;
     L.prm = prm;
     L.t = 0;
+    L.fill = kind == SGB_HEAT7 && !g->clean[dst[0]];
     L.err = g->err.as<unsigned>();
     SGB_TRY(launch_fields(L, s));
     if (kind == SGB_HEAT7) g->clean[dst[0]] = true;  // every point of dst was written from the tile
@@ -614,7 +612,7 @@ int sgb_apply_stencil(sgb_grid* g, int kind, const int* src, const int* dst, con
 }
 
 // Same as sgb_apply_stencil through the generic one-chunk-per-CTA kernel
-// (cross-check of the pipelined kernel; not part of the drop-in surface).
+// (cross-check of the 8^3 kernel; not part of the drop-in surface).
 int sgb_apply_stencil_tiled(sgb_grid* g, int kind, const int* src, const int* dst, const float* params, int nparams,
                             const int64_t* box, sgb_stream s) {
     if (!g) return SGB_EINVAL;

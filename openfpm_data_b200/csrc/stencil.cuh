@@ -63,15 +63,10 @@ __device__ __forceinline__ void gs_update(float u, float v, float lu, float lv, 
     vn = __fmaf_rn(p.dt, dv, v);
 }
 
-// CTAs per SM of the pipelined 8^3 kernel when the caller leaves it automatic
-// (measured on the 512^3 grids: Gray-Scott runs best with 6 two-warp CTAs
-// and 3-deep rings resident, heat with 8).
-inline int auto_ctas_per_sm(int kind) { return kind == SGB_GS7 ? 6 : 8; }
-
 // Everything one stencil launch needs.
 struct LaunchDesc {
-    int kind, edge, use_tile, stages, num_sms;
-    unsigned ctas;
+    int kind, edge, use_tile, num_sms;
+    int stages, ctas_per_sm;  // sgb_set_launch_config; 0: automatic
     FieldSet fs;
     const uint8_t* mask;
     const int32_t* nn;
@@ -84,11 +79,12 @@ struct LaunchDesc {
     Geometry geo;
     StencilParams prm;
     int64_t t;
+    int fill;                // HEAT7: quads without an existing point are written too (dst may hold anything there)
     unsigned* err;
 };
 
 int launch_fields(const LaunchDesc& L, cudaStream_t s);
-int launch_e8(const LaunchDesc& L, cudaStream_t s);  // pipelined 8^3 kernel (stencil8.cu)
+int launch_star7(const LaunchDesc& L, cudaStream_t s);  // 8^3 chunks, any chunk ids (star7.cu)
 GridInfo grid_info_of(const StencilParams& prm);
 
 // Capture `body(stream)` into a CUDA graph, launch it on `s`, wait for it.

@@ -1,0 +1,75 @@
+"""The 7-point kernel on 8^3 chunks against the one-chunk-per-CTA kernel, bit for bit: both evaluate the same
+float32 operations in the same order, so no tolerance is needed."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def sgb():
+    import openfpm_data_b200 as m
+    m.load()
+    return m
+
+
+def _grid(sgb, size, nchunks, lin, seed, density=0.5):
+    """A grid of about nchunks random chunks, a part of whose points exist, some of them padding."""
+    rng = np.random.default_rng(seed)
+    b = [-(-s // 8) for s in size]
+    pick = rng.permutation(b[0] * b[1] * b[2])[:nchunks]
+    bc = np.stack([pick % b[0], pick // b[0] % b[1], pick // (b[0] * b[1])], axis=1)
+    if lin == "zmb":
+        spread = lambda v: sum(((v >> i) & 1) << (3 * i) for i in range(8))  # noqa: E731
+        key = spread(bc[:, 0]) | spread(bc[:, 1]) << 1 | spread(bc[:, 2]) << 2
+    else:
+        key = pick
+    order = np.argsort(key)
+    key, bc = key[order].astype(np.int64), bc[order]
+    p = np.arange(512)
+    xyz = bc[:, None, :] * 8 + np.stack([p % 8, p // 8 % 8, p // 64], axis=1)[None]
+    rows = rng.random((len(key), 64, 1)) < 0.8  # whole x rows are missing too
+    ex = (rng.random((len(key), 64, 8)) < density) & rows
+    ex = ex.reshape(len(key), 512) & (xyz < np.array(size)).all(axis=2)
+    pad = ex & (rng.random(ex.shape) < 0.1)
+    mask = (ex | pad << 1).astype(np.uint8).reshape(-1)
+    g = sgb.SparseGridGpu(size, ["f32"] * 4, edge=8, linearizer=lin)
+    for q, v in enumerate([0.25, -1.5, 3.0, 0.5]):
+        g.setBackgroundValue(q, v)
+    g.load_map(key, [rng.standard_normal(len(mask)).astype(np.float32) for _ in range(4)], mask)
+    return g
+
+
+@pytest.mark.parametrize("stages", [3, 4])
+@pytest.mark.parametrize("lin,size,nchunks", [
+    ("smb", (8, 8, 8), 1), ("smb", (70, 20, 9), 7), ("smb", (130, 33, 30), 60), ("smb", (157, 61, 90), 1500),
+    ("zmb", (64, 64, 64), 300), ("zmb", (75, 50, 41), 200)])
+@pytest.mark.parametrize("kind", ["HEAT7", "GS7"])
+def test_star7_equals_tiled(sgb, kind, lin, size, nchunks, stages):
+    prm = [0.1] if kind == "HEAT7" else [0.16, 0.08, 0.035, 0.065, 1.0]
+    src, dst = ([0], [2]) if kind == "HEAT7" else ([0, 1], [2, 3])
+    for box in (None, ((3, 2, 1), (size[0] - 4, size[1] - 3, size[2] - 2))):
+        out = []
+        for tiled in (True, False):
+            g = _grid(sgb, size, nchunks, lin, 7)
+            g.setLaunchConfig(-1, stages)
+            m = g.private_get_mask_array()  # also: no property counts as background-clean any more
+            g.applyStencils(getattr(sgb, kind), src, dst, prm, box=box, tiled=tiled)
+            g.check_device_errors()
+            keep = torch.from_numpy(np.ones(m.numel(), bool)).cuda() if kind == "HEAT7" else (m & 1).bool()
+            out.append([g.private_get_data_array(d)[keep].cpu() for d in dst])
+        for a, b in zip(*out):
+            assert torch.equal(a.view(torch.int32), b.view(torch.int32))
+
+
+def test_star7_eight_slices_by_size(sgb):
+    """Past two waves of blocks the automatic choice changes; the steps stay the same."""
+    g = _grid(sgb, (240, 240, 240), 20000, "smb", 3)
+    got = []
+    for stages in (3, -1):
+        g.setLaunchConfig(-1, stages)
+        g.applyStencils(sgb.HEAT7, [0], [2], [0.1])
+        got.append(g.private_get_data_array(2).clone())
+    assert torch.equal(*got)
+    g.check_device_errors()
