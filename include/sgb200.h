@@ -222,8 +222,9 @@ int sgb_apply_stencil(sgb_grid* g, int kind, const int* src, const int* dst, con
 
 /* nsteps stencil applications alternating src->dst and dst->src (the
  * reference's ping-pong loop, src/SparseGridGpu/tests/
- * SparseGridGpu_tests.cu:499-503), launched as one captured CUDA graph.
- * On return *final_is_dst is 1 when the last step wrote the dst properties. */
+ * SparseGridGpu_tests.cu:499-503): one launch per step, each overlapping the
+ * tail of the one before, or one launch for all steps of a small grid.
+ * use_graph != 0: the call waits for a grid of one launch per step.  On return *final_is_dst is 1 when the last step wrote the dst properties. */
 int sgb_run_steps(sgb_grid* g, int kind, const int* src, const int* dst, const float* params, int nparams,
                   int nsteps, int use_graph, int* final_is_dst, sgb_stream s);
 

@@ -87,38 +87,4 @@ int launch_fields(const LaunchDesc& L, cudaStream_t s);
 int launch_star7(const LaunchDesc& L, cudaStream_t s);  // 8^3 chunks, any chunk ids (star7.cu)
 GridInfo grid_info_of(const StencilParams& prm);
 
-// Capture `body(stream)` into a CUDA graph, launch it on `s`, wait for it.
-template <typename F>
-int run_graph(F body, cudaStream_t s) {
-    cudaStream_t cap;
-    SGB_CUDA(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t exec = nullptr;
-    int st = SGB_OK;
-    cudaError_t e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
-    if (e == cudaSuccess) {
-        st = body(cap);
-        cudaError_t e2 = cudaStreamEndCapture(cap, &graph);
-        if (st == SGB_OK && e2 != cudaSuccess) st = cuda_status(e2, "cudaStreamEndCapture");
-    } else {
-        st = cuda_status(e, "cudaStreamBeginCapture");
-    }
-    if (st == SGB_OK) {
-        e = cudaGraphInstantiate(&exec, graph, 0);
-        if (e != cudaSuccess) st = cuda_status(e, "cudaGraphInstantiate");
-    }
-    if (st == SGB_OK) {
-        e = cudaGraphLaunch(exec, s);
-        if (e != cudaSuccess) st = cuda_status(e, "cudaGraphLaunch");
-    }
-    if (st == SGB_OK) {
-        e = cudaStreamSynchronize(s);
-        if (e != cudaSuccess) st = cuda_status(e, "cudaStreamSynchronize");
-    }
-    if (exec) cudaGraphExecDestroy(exec);
-    if (graph) cudaGraphDestroy(graph);
-    cudaStreamDestroy(cap);
-    return st;
-}
-
 }  // namespace sgb
