@@ -3,8 +3,7 @@
 Candidates: chunk edge 8 (16 or 32 threads per 512-point chunk, by the
 staging depth: 4 for eight z slices per group of 16 threads, 3 for four, -1
 by the batch's size; at most 4, 6 or 8 CTAs of 128 threads per SM, or -1 for
-no limit) and chunk edge 4
-(one-chunk-per-CTA tile kernel: 256 threads per 64-point chunk).  Each
+no limit) and chunk edge 4 (16 threads per 64-point chunk).  Each
 candidate runs a few timed batch steps (CUDA events) on a sample of the
 grids, rebuilt with its chunk edge; the fastest per active point wins.
 """
@@ -84,9 +83,9 @@ def autotune(specs: Sequence[Spec], kind: int, params, steps: int = 10, device: 
                 b.set_launch_config(c, s)
             t = _time_steps(b, steps)
             nsps = t / steps / max(pts, 1) * 1e9
-            # 8^3: groups of 16 threads, one or two per chunk; 4^3: one 256-thread CTA per chunk
+            # groups of 16 threads: one or two per 8^3 chunk, one per 4^3 chunk
             row = {"chunk_edge": ce, "ctas_per_sm": c, "stages": s,
-                   "threads_per_chunk": (16 if s >= 4 else 32) if ce == 8 else 256,
+                   "threads_per_chunk": 32 if ce == 8 and s < 4 else 16,
                    "ns_per_point_step": round(nsps, 5)}
             table.append(row)
             if best is None or nsps < best["ns_per_point_step"]:

@@ -1,5 +1,5 @@
-// 7-point stencils (HEAT7, GS7) on 8^3 chunks, for single grids and batches
-// and for any chunk ids.
+// 7-point stencils (HEAT7, GS7), for single grids and batches and for any
+// chunk ids: first 8^3 chunks, 4^3 chunks below.
 //
 // Reference path: applyStencilInPlace (src/SparseGridGpu/SparseGridGpu.hpp:
 // 954-1048) launches one 512-thread CTA per chunk; loadGhostBlock_impl<1>
@@ -353,6 +353,91 @@ __global__ void __launch_bounds__(kStarThreads, MINB)
     }
 }
 
+// 4^3 chunks: 16 lanes take one chunk, lane l the x row (y, z) = (l % 4, l / 4), all of whose neighbours are
+// read straight from global memory (rows inside the chunk and of the chunks before and after it hit the lines
+// that the block's other lanes load).  The one-CTA-per-chunk gather that served these chunks before kept 64 of
+// 256 threads busy: Gray-Scott 250x190x131, 24,003 chunks and 1.33 M points, 65.7 us per step, now 6.46 (3.5
+// TB/s of the points' bytes; 4 to 8 blocks per SM run the same).  Bound by latency: two waves of blocks.
+template <int KIND, int NP, bool BOX, bool BATCH, int MINB>
+__global__ void __launch_bounds__(kStarThreads, MINB)
+    k_star7_e4(FieldSet fs, const uint8_t* __restrict__ mask, const int32_t* __restrict__ nn,
+               const int64_t* __restrict__ keys, const int32_t* __restrict__ gid, const GridInfo* __restrict__ grids,
+               GridInfo g0, int64_t n, Geometry geo, StencilParams prm, int64_t t, int fill) {
+    const int64_t dep = grid_dependency_wait();
+    mask += dep;
+    nn += dep;
+    const int l16 = threadIdx.x & 15, y = l16 & 3, z = l16 >> 2;
+    const int64_t c = (int64_t)blockIdx.x * kStarGroups + (threadIdx.x >> 4);
+    if (c >= n) return;
+    GridInfo gb;
+    int par = 0;
+    if (BATCH) {
+        gb = grids[gid[c]];
+        if (!(t >= gb.start && t < gb.start + gb.nsteps)) return;
+        par = (int)((t - gb.start) & 1);
+    }
+    const GridInfo& gi = BATCH ? gb : g0;
+    const uint32_t m = __ldg(reinterpret_cast<const uint32_t*>(mask + c * 64 + l16 * 4));
+    if (!m && !(KIND == SGB_HEAT7 && fill)) return;  // the row holds no point
+    const int4 na = __ldg(reinterpret_cast<const int4*>(nn + c * 8));
+    const int2 nz = __ldg(reinterpret_cast<const int2*>(nn + c * 8 + 4));
+    const int64_t oc = c * 64 + l16 * 4;
+    const int64_t oxm = (int64_t)na.x * 64 + l16 * 4 + 3, oxp = (int64_t)na.y * 64 + l16 * 4;
+    const int64_t oym = y > 0 ? oc - 4 : (na.z >= 0 ? (int64_t)na.z * 64 + z * 16 + 12 : -1);
+    const int64_t oyp = y < 3 ? oc + 4 : (na.w >= 0 ? (int64_t)na.w * 64 + z * 16 : -1);
+    const int64_t ozm = z > 0 ? oc - 16 : (nz.x >= 0 ? (int64_t)nz.x * 64 + 48 + y * 4 : -1);
+    const int64_t ozp = z < 3 ? oc + 16 : (nz.y >= 0 ? (int64_t)nz.y * 64 + y * 4 : -1);
+    float4 cv[NP];
+    Quad lap[NP];
+    float bd[NP];
+    float* dst[NP];
+    float4 ym[NP], yp[NP], zm[NP], zp[NP];
+    float xm[NP], xp[NP];
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+        const float* src = (par ? fs.in[1][p] : fs.in[0][p]) + dep;
+        const float bs = par ? gi.bck[1][p] : gi.bck[0][p];
+        dst[p] = (par ? fs.out[1][p] : fs.out[0][p]) + oc;
+        bd[p] = par ? gi.bck[0][p] : gi.bck[1][p];
+        ym[p] = yp[p] = zm[p] = zp[p] = splat4(bs);
+        xm[p] = xp[p] = bs;
+        cv[p] = ldf4(src + oc);
+        if (oym >= 0) ym[p] = ldf4(src + oym);
+        if (oyp >= 0) yp[p] = ldf4(src + oyp);
+        if (ozm >= 0) zm[p] = ldf4(src + ozm);
+        if (ozp >= 0) zp[p] = ldf4(src + ozp);
+        if (na.x >= 0) xm[p] = ldf1(src + oxm);
+        if (na.y >= 0) xp[p] = ldf1(src + oxp);
+    }
+#pragma unroll
+    for (int p = 0; p < NP; ++p) lap[p] = lap_quad<KIND>(cv[p], xm[p], xp[p], ym[p], yp[p], zm[p], zp[p]);
+    int32_t cx = 0, cy = 0, cz = 0;
+    if (BOX) {
+        int64_t o[3];
+        chunk_origin(geo, keys[c], o);
+        cx = (int32_t)o[0];
+        cy = (int32_t)o[1] + y;
+        cz = (int32_t)o[2] + z;
+    }
+    star_store<KIND, NP>(cv, lap, m, active_bits<BOX>(m, prm, cx, cy, cz), gi, bd, dst[0], dst[NP - 1]);
+}
+
+// Consecutive steps overlap one launch's ramp-up with the previous one's tail.
+struct StarLaunch {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    StarLaunch(int64_t groups, size_t smem, cudaStream_t s) {
+        cfg.gridDim = dim3((unsigned)((groups + kStarGroups - 1) / kStarGroups));
+        cfg.blockDim = dim3(kStarThreads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = s;
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+    }
+};
+
 template <int KIND, int NP, bool BOX, bool BATCH, int ZS, int MINB>
 static int launch_star(const LaunchDesc& L, cudaStream_t s) {
     auto kern = k_star7_e8<KIND, NP, BOX, BATCH, ZS, MINB>;
@@ -361,19 +446,9 @@ static int launch_star(const LaunchDesc& L, cudaStream_t s) {
     // a caller's limit on the CTAs per SM: each CTA takes its share of the SM's shared memory
     if (L.ctas_per_sm > 0) smem = std::max(smem, (size_t)(227 * 1024 / L.ctas_per_sm - 1024) & ~(size_t)127);
     SGB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)((items + kStarGroups - 1) / kStarGroups));
-    cfg.blockDim = dim3(kStarThreads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    // consecutive steps overlap one launch's ramp-up with the previous one's tail
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    StarLaunch l(items, smem, s);
     const int ahead = L.num_sms * 7 * kStarGroups;  // about the groups resident at a time
-    SGB_CUDA(cudaLaunchKernelEx(&cfg, kern, L.fs, L.mask, L.nn, L.keys, L.gid, L.grids, L.g0, L.n, L.geo, L.prm, L.t,
+    SGB_CUDA(cudaLaunchKernelEx(&l.cfg, kern, L.fs, L.mask, L.nn, L.keys, L.gid, L.grids, L.g0, L.n, L.geo, L.prm, L.t,
                                 L.fill, ahead));
     return SGB_OK;
 }
@@ -386,12 +461,28 @@ static int launch_star_kind(const LaunchDesc& L, cudaStream_t s) {
     return launch_star<KIND, NP, false, false, ZS, MINB>(L, s);
 }
 
+template <int KIND, int NP, bool BOX, bool BATCH>
+static int launch_e4(const LaunchDesc& L, cudaStream_t s) {
+    StarLaunch l(L.n, 0, s);
+    SGB_CUDA(cudaLaunchKernelEx(&l.cfg, k_star7_e4<KIND, NP, BOX, BATCH, KIND == SGB_GS7 ? 6 : 10>, L.fs, L.mask, L.nn,
+                                L.keys, L.gid, L.grids, L.g0, L.n, L.geo, L.prm, L.t, L.fill));
+    return SGB_OK;
+}
+
+template <int KIND, int NP>
+static int launch_e4_kind(const LaunchDesc& L, cudaStream_t s) {
+    if (L.grids) return launch_e4<KIND, NP, false, true>(L, s);
+    if (L.prm.has_box) return launch_e4<KIND, NP, true, false>(L, s);
+    return launch_e4<KIND, NP, false, false>(L, s);
+}
+
 // Slices per group.  Eight halve the z-face loads and the instructions per point, four fill the chip with half
 // as many chunks.  Heat: eight from two full waves of such blocks on (us per step, 4 against 8: 5,637 chunks
 // 5.3 / 8.0, 18,932 chunks 12.8 / 12.5, 33,000 chunks 33.3 / 31.7, 300,000 chunks 241 / 212).  Gray-Scott
 // keeps four: the same time within 2 % at every size, and eight need 41 KB and 92 registers a block.  (Heat
 // with eight slices fits 8 blocks of 128 threads on an SM, with four 10; Gray-Scott 7: no spills.)
 int launch_star7(const LaunchDesc& L, cudaStream_t s) {
+    if (L.edge == 4) return L.kind == SGB_GS7 ? launch_e4_kind<SGB_GS7, 2>(L, s) : launch_e4_kind<SGB_HEAT7, 1>(L, s);
     bool eight = L.kind == SGB_HEAT7 && L.n >= (int64_t)2 * L.num_sms * 8 * kStarGroups;
     if (L.stages > 0) eight = L.stages >= 4;
     if (L.kind == SGB_GS7)

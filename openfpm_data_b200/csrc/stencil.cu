@@ -6,9 +6,9 @@
 // the 10^3 tile with one scalar load per point, the user functor computes,
 // storeBlock writes back.
 //
-// Here 7-point stencils on 8^3 chunks run the kernel of star7.cu; this file
-// holds the generic one-chunk-per-CTA tile kernel (4^3 chunks, cross-checks),
-// Conv3x3x3 on 8^3 chunks, parameter handling and dispatch.
+// Here 7-point stencils run the kernels of star7.cu; this file holds the
+// generic one-chunk-per-CTA tile kernel (Conv3x3x3 on 4^3 chunks,
+// cross-checks), Conv3x3x3 on 8^3 chunks, parameter handling and dispatch.
 //
 // The same kernels run a batch of grids concatenated into one block map: a
 // per-chunk grid id selects the grid's parameters and its ping-pong buffer
@@ -38,7 +38,7 @@ namespace sgb {
 // Any edge, any of the three stencils: one CTA per chunk (grid-stride), the
 // (edge+2)^3 tile gathered with one load per cell, as the reference's
 // loadGhostBlock does, with NNFull edge/corner cells taken from the right
-// neighbour.  Used for BOX27, for 4^3 chunks and as a cross-check.
+// neighbour.  Used for BOX27 on 4^3 chunks and as a cross-check.
 template <int KIND, int E>
 __global__ void __launch_bounds__(256) k_stencil_tile(FieldSet fs, const uint8_t* __restrict__ mask,
                                                       const int32_t* __restrict__ nn, const int64_t* __restrict__ keys,
@@ -522,7 +522,7 @@ GridInfo grid_info_of(const StencilParams& prm) {
 
 int launch_fields(const LaunchDesc& L, cudaStream_t s) {
     if (L.n == 0) return SGB_OK;
-    if (L.kind != SGB_BOX27 && L.edge == 8 && !L.use_tile) return launch_star7(L, s);
+    if (L.kind != SGB_BOX27 && !L.use_tile) return launch_star7(L, s);
     if (L.kind == SGB_BOX27 && L.edge == 8 && !L.use_tile && !L.grids) {
         // 4 CTAs of four warps per SM are resident (128 registers a thread)
         const int64_t want = (L.n + kW27Warps - 1) / kW27Warps;

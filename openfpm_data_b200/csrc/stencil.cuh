@@ -84,7 +84,7 @@ struct LaunchDesc {
 };
 
 int launch_fields(const LaunchDesc& L, cudaStream_t s);
-int launch_star7(const LaunchDesc& L, cudaStream_t s);  // 8^3 chunks, any chunk ids (star7.cu)
+int launch_star7(const LaunchDesc& L, cudaStream_t s);  // 7-point kernels, any chunk ids (star7.cu)
 GridInfo grid_info_of(const StencilParams& prm);
 
 }  // namespace sgb

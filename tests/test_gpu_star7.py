@@ -1,4 +1,4 @@
-"""The 7-point kernel on 8^3 chunks against the one-chunk-per-CTA kernel, bit for bit: both evaluate the same
+"""The 7-point kernels against the one-chunk-per-CTA kernel, bit for bit: both evaluate the same
 float32 operations in the same order, so no tolerance is needed."""
 import numpy as np
 import pytest
@@ -14,10 +14,10 @@ def sgb():
     return m
 
 
-def _grid(sgb, size, nchunks, lin, seed, density=0.5):
+def _grid(sgb, size, nchunks, lin, seed, density=0.5, e=8):
     """A grid of about nchunks random chunks, a part of whose points exist, some of them padding."""
     rng = np.random.default_rng(seed)
-    b = [-(-s // 8) for s in size]
+    b = [-(-s // e) for s in size]
     pick = rng.permutation(b[0] * b[1] * b[2])[:nchunks]
     bc = np.stack([pick % b[0], pick // b[0] % b[1], pick // (b[0] * b[1])], axis=1)
     if lin == "zmb":
@@ -27,32 +27,32 @@ def _grid(sgb, size, nchunks, lin, seed, density=0.5):
         key = pick
     order = np.argsort(key)
     key, bc = key[order].astype(np.int64), bc[order]
-    p = np.arange(512)
-    xyz = bc[:, None, :] * 8 + np.stack([p % 8, p // 8 % 8, p // 64], axis=1)[None]
-    rows = rng.random((len(key), 64, 1)) < 0.8  # whole x rows are missing too
-    ex = (rng.random((len(key), 64, 8)) < density) & rows
-    ex = ex.reshape(len(key), 512) & (xyz < np.array(size)).all(axis=2)
+    p = np.arange(e ** 3)
+    xyz = bc[:, None, :] * e + np.stack([p % e, p // e % e, p // e ** 2], axis=1)[None]
+    rows = rng.random((len(key), e * e, 1)) < 0.8  # whole x rows are missing too
+    ex = (rng.random((len(key), e * e, e)) < density) & rows
+    ex = ex.reshape(len(key), e ** 3) & (xyz < np.array(size)).all(axis=2)
     pad = ex & (rng.random(ex.shape) < 0.1)
     mask = (ex | pad << 1).astype(np.uint8).reshape(-1)
-    g = sgb.SparseGridGpu(size, ["f32"] * 4, edge=8, linearizer=lin)
+    g = sgb.SparseGridGpu(size, ["f32"] * 4, edge=e, linearizer=lin)
     for q, v in enumerate([0.25, -1.5, 3.0, 0.5]):
         g.setBackgroundValue(q, v)
     g.load_map(key, [rng.standard_normal(len(mask)).astype(np.float32) for _ in range(4)], mask)
     return g
 
 
-@pytest.mark.parametrize("stages", [3, 4])
+@pytest.mark.parametrize("e,stages", [(8, 3), (8, 4), (4, -1)])
 @pytest.mark.parametrize("lin,size,nchunks", [
     ("smb", (8, 8, 8), 1), ("smb", (70, 20, 9), 7), ("smb", (130, 33, 30), 60), ("smb", (157, 61, 90), 1500),
     ("zmb", (64, 64, 64), 300), ("zmb", (75, 50, 41), 200)])
 @pytest.mark.parametrize("kind", ["HEAT7", "GS7"])
-def test_star7_equals_tiled(sgb, kind, lin, size, nchunks, stages):
+def test_star7_equals_tiled(sgb, kind, lin, size, nchunks, e, stages):
     prm = [0.1] if kind == "HEAT7" else [0.16, 0.08, 0.035, 0.065, 1.0]
     src, dst = ([0], [2]) if kind == "HEAT7" else ([0, 1], [2, 3])
     for box in (None, ((3, 2, 1), (size[0] - 4, size[1] - 3, size[2] - 2))):
         out = []
         for tiled in (True, False):
-            g = _grid(sgb, size, nchunks, lin, 7)
+            g = _grid(sgb, size, nchunks, lin, 7, e=e)
             g.setLaunchConfig(-1, stages)
             m = g.private_get_mask_array()  # also: no property counts as background-clean any more
             g.applyStencils(getattr(sgb, kind), src, dst, prm, box=box, tiled=tiled)
