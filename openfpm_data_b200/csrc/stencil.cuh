@@ -85,6 +85,9 @@ struct LaunchDesc {
 
 int launch_fields(const LaunchDesc& L, cudaStream_t s);
 int launch_star7(const LaunchDesc& L, cudaStream_t s);  // 7-point kernels, any chunk ids (star7.cu)
+// All steps of a small grid's solve in one launch (solve.cu); SGB_ENOTSUP: not for this grid.
+int run_steps_cluster(sgb_grid* g, int kind, const int* src, const int* dst, const StencilParams& fwd, int nsteps,
+                      cudaStream_t s);
 GridInfo grid_info_of(const StencilParams& prm);
 
 }  // namespace sgb

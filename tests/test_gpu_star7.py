@@ -73,3 +73,23 @@ def test_star7_eight_slices_by_size(sgb):
         got.append(g.private_get_data_array(2).clone())
     assert torch.equal(*got)
     g.check_device_errors()
+
+
+@pytest.mark.parametrize("nchunks", [1, 2, 5, 17, 33, 160, 161, 256, 257])
+@pytest.mark.parametrize("kind", ["HEAT7", "GS7"])
+def test_solve_in_one_launch_equals_steps(sgb, kind, nchunks):
+    """run_steps of a small grid (both sides of the size limit) against single steps of the tile kernel."""
+    prm = [0.1] if kind == "HEAT7" else [0.16, 0.08, 0.035, 0.065, 1.0]
+    a, b = ([0], [2]) if kind == "HEAT7" else ([0, 1], [2, 3])
+    size = (75, 80, 70) if nchunks < 100 else (100, 99, 75)
+    for nsteps in (2, 9):
+        g, h = (_grid(sgb, size, nchunks, "smb", 11, density=0.9) for _ in range(2))
+        fin = g.run_steps(getattr(sgb, kind), a, b, prm, nsteps)
+        for k in range(nsteps):
+            h.applyStencils(getattr(sgb, kind), a if k % 2 == 0 else b, b if k % 2 == 0 else a, prm, tiled=True)
+        assert fin == (nsteps % 2 == 1)
+        g.check_device_errors()
+        ex = (g.private_get_mask_array() & 1).bool()
+        for q in a + b:  # the last state and the one before it
+            x, w = g.private_get_data_array(q)[ex], h.private_get_data_array(q)[ex]
+            assert torch.equal(x.view(torch.int32), w.view(torch.int32))
