@@ -160,7 +160,7 @@ static int batch_upload_grids(sgb_batch* b, cudaStream_t s) {
     return SGB_OK;
 }
 
-static int batch_launch(sgb_batch* b, int64_t t, cudaStream_t s) {
+static int batch_launch(sgb_batch* b, int64_t t, cudaStream_t s, bool chained) {
     LaunchDesc L;
     std::memset(&L, 0, sizeof(L));
     L.kind = b->kind;
@@ -185,6 +185,7 @@ static int batch_launch(sgb_batch* b, int64_t t, cudaStream_t s) {
     L.geo.edge = b->edge;
     L.geo.bs = b->edge * b->edge * b->edge;
     L.t = t;
+    L.chained = chained;
     L.err = b->err.as<unsigned>();
     return launch_fields(L, s);
 }
@@ -349,7 +350,7 @@ int sgb_batch_step(sgb_batch* b, int nsteps, int use_graph, sgb_stream stream) {
         st = SGB_OK;
         cudaError_t e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
         if (e == cudaSuccess) {
-            for (int k = 0; k < nsteps && st == SGB_OK; ++k) st = batch_launch(b, T0 + k, cap);
+            for (int k = 0; k < nsteps && st == SGB_OK; ++k) st = batch_launch(b, T0 + k, cap, k > 0);
             const cudaError_t e2 = cudaStreamEndCapture(cap, &graph);
             if (st == SGB_OK && e2 != cudaSuccess) st = cuda_status(e2, "cudaStreamEndCapture");
         } else {
@@ -383,7 +384,7 @@ int sgb_batch_step(sgb_batch* b, int nsteps, int use_graph, sgb_stream stream) {
         cudaStreamDestroy(cap);
     } else {
         st = SGB_OK;
-        for (int k = 0; k < nsteps && st == SGB_OK; ++k) st = batch_launch(b, b->T + k, s);
+        for (int k = 0; k < nsteps && st == SGB_OK; ++k) st = batch_launch(b, b->T + k, s, k > 0);
     }
     if (st == SGB_OK) b->T += nsteps;
     return st;

@@ -319,8 +319,9 @@ int launch_points_box27_sparse(sgb_grid* g, const int* src, const int* dst, cons
                                cudaStream_t s);
 
 // stencil.cu
+// chained: follows a launch over the same masks and neighbours in the same call
 int launch_stencil(sgb_grid* g, int kind, const int* src, const int* dst, const StencilParams& prm,
-                   cudaStream_t s);
+                   cudaStream_t s, bool chained = false);
 int make_params(sgb_grid* g, int kind, const int* src, const int* dst, const float* params, int nparams,
                 const int64_t* box, StencilParams& prm);
 

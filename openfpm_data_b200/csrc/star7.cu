@@ -52,15 +52,18 @@ template <int KIND, int NP, bool BOX, bool BATCH, int ZS, int MINB>
 __global__ void __launch_bounds__(kStarThreads, MINB)
     k_star7_e8(FieldSet fs, const uint8_t* __restrict__ mask, const int32_t* __restrict__ nn,
                const int64_t* __restrict__ keys, const int32_t* __restrict__ gid, const GridInfo* __restrict__ grids,
-               GridInfo g0, int64_t n, Geometry geo, StencilParams prm, int64_t t, int fill, int ahead) {
+               GridInfo g0, int64_t n, Geometry geo, StencilParams prm, int64_t t, int fill, int chained, int ahead) {
     constexpr int PARTS = 8 / ZS;
     extern __shared__ __align__(16) unsigned char star_smem[];
     StarTile<NP, ZS>* const tiles = reinterpret_cast<StarTile<NP, ZS>*>(star_smem);
     const int grp = threadIdx.x >> 4;
     StarTile<NP, ZS>& T = tiles[grp];
-    const int64_t dep = grid_dependency_wait();
-    mask += dep;
-    nn += dep;
+    grid_launch_dependents();
+    if (!chained) {  // a chained launch follows one of the same map: its masks and neighbours stand already
+        const int64_t first = grid_dependency_wait();
+        mask += first;
+        nn += first;
+    }
     const int l16 = threadIdx.x & 15, y = l16 >> 1, xq = l16 & 1;
     const int o0 = y * 8 + xq * 4;
     const int64_t total = n * PARTS;
@@ -82,6 +85,7 @@ __global__ void __launch_bounds__(kStarThreads, MINB)
     for (int z = 0; z < ZS; ++z) m[z] = live ? __ldg(reinterpret_cast<const uint32_t*>(mp + z * 64)) : 0u;
     const int4 na = __ldg(reinterpret_cast<const int4*>(nn + c * 8));
     const int2 nz = __ldg(reinterpret_cast<const int2*>(nn + c * 8 + 4));
+    const int64_t dep = grid_dependency_wait();
     const float* src[NP];
     float bs[NP], bd[NP];  // backgrounds of the source and destination fields
 #pragma unroll
@@ -199,10 +203,13 @@ template <int KIND, int NP, bool BOX, bool BATCH, int MINB>
 __global__ void __launch_bounds__(kStarThreads, MINB)
     k_star7_e4(FieldSet fs, const uint8_t* __restrict__ mask, const int32_t* __restrict__ nn,
                const int64_t* __restrict__ keys, const int32_t* __restrict__ gid, const GridInfo* __restrict__ grids,
-               GridInfo g0, int64_t n, Geometry geo, StencilParams prm, int64_t t, int fill) {
-    const int64_t dep = grid_dependency_wait();
-    mask += dep;
-    nn += dep;
+               GridInfo g0, int64_t n, Geometry geo, StencilParams prm, int64_t t, int fill, int chained) {
+    grid_launch_dependents();
+    if (!chained) {  // a chained launch follows one of the same map: its masks and neighbours stand already
+        const int64_t first = grid_dependency_wait();
+        mask += first;
+        nn += first;
+    }
     const int l16 = threadIdx.x & 15, y = l16 & 3, z = l16 >> 2;
     const int64_t c = (int64_t)blockIdx.x * kStarGroups + (threadIdx.x >> 4);
     if (c >= n) return;
@@ -224,6 +231,7 @@ __global__ void __launch_bounds__(kStarThreads, MINB)
     const int64_t oyp = y < 3 ? oc + 4 : (na.w >= 0 ? (int64_t)na.w * 64 + z * 16 : -1);
     const int64_t ozm = z > 0 ? oc - 16 : (nz.x >= 0 ? (int64_t)nz.x * 64 + 48 + y * 4 : -1);
     const int64_t ozp = z < 3 ? oc + 16 : (nz.y >= 0 ? (int64_t)nz.y * 64 + y * 4 : -1);
+    const int64_t dep = grid_dependency_wait();
     float4 cv[NP];
     Quad lap[NP];
     float bd[NP];
@@ -282,11 +290,11 @@ static int launch_star(const LaunchDesc& L, cudaStream_t s) {
     size_t smem = sizeof(StarTile<NP, ZS>) * kStarGroups;
     // a caller's limit on the CTAs per SM: each CTA takes its share of the SM's shared memory
     if (L.ctas_per_sm > 0) smem = std::max(smem, (size_t)(227 * 1024 / L.ctas_per_sm - 1024) & ~(size_t)127);
-    SGB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > 48 * 1024) SGB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     StarLaunch l(items, smem, s);
     const int ahead = L.num_sms * 7 * kStarGroups;  // about the groups resident at a time
     SGB_CUDA(cudaLaunchKernelEx(&l.cfg, kern, L.fs, L.mask, L.nn, L.keys, L.gid, L.grids, L.g0, L.n, L.geo, L.prm, L.t,
-                                L.fill, ahead));
+                                L.fill, L.chained, ahead));
     return SGB_OK;
 }
 
@@ -302,7 +310,7 @@ template <int KIND, int NP, bool BOX, bool BATCH>
 static int launch_e4(const LaunchDesc& L, cudaStream_t s) {
     StarLaunch l(L.n, 0, s);
     SGB_CUDA(cudaLaunchKernelEx(&l.cfg, k_star7_e4<KIND, NP, BOX, BATCH, KIND == SGB_GS7 ? 6 : 10>, L.fs, L.mask, L.nn,
-                                L.keys, L.gid, L.grids, L.g0, L.n, L.geo, L.prm, L.t, L.fill));
+                                L.keys, L.gid, L.grids, L.g0, L.n, L.geo, L.prm, L.t, L.fill, L.chained));
     return SGB_OK;
 }
 

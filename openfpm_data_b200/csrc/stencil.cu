@@ -408,7 +408,7 @@ int launch_fields(const LaunchDesc& L, cudaStream_t s) {
 }
 
 int launch_stencil_impl(sgb_grid* g, int kind, const int* src, const int* dst, const StencilParams& prm,
-                        cudaStream_t s, bool use_tile) {
+                        cudaStream_t s, bool use_tile, bool chained) {
     if (g->n == 0) return SGB_OK;
     if (kind == SGB_BOX27_NS) return launch_points_box27(g, src, dst, prm, s);
     if (kind == SGB_BOX27 && !use_tile) {  // sparse chunks: the point list
@@ -443,6 +443,7 @@ int launch_stencil_impl(sgb_grid* g, int kind, const int* src, const int* dst, c
     L.geo = g->geo;
     L.prm = prm;
     L.t = 0;
+    L.chained = chained;
     L.fill = kind == SGB_HEAT7 && !g->clean[dst[0]];
     L.err = g->err.as<unsigned>();
     SGB_TRY(launch_fields(L, s));
@@ -450,8 +451,9 @@ int launch_stencil_impl(sgb_grid* g, int kind, const int* src, const int* dst, c
     return SGB_OK;
 }
 
-int launch_stencil(sgb_grid* g, int kind, const int* src, const int* dst, const StencilParams& prm, cudaStream_t s) {
-    return launch_stencil_impl(g, kind, src, dst, prm, s, false);
+int launch_stencil(sgb_grid* g, int kind, const int* src, const int* dst, const StencilParams& prm, cudaStream_t s,
+                   bool chained) {
+    return launch_stencil_impl(g, kind, src, dst, prm, s, false, chained);
 }
 
 }  // namespace sgb
@@ -475,7 +477,7 @@ int sgb_apply_stencil_tiled(sgb_grid* g, int kind, const int* src, const int* ds
     if (!g) return SGB_EINVAL;
     StencilParams prm;
     SGB_TRY(make_params(g, kind, src, dst, params, nparams, box, prm));
-    return launch_stencil_impl(g, kind, src, dst, prm, (cudaStream_t)s, true);
+    return launch_stencil_impl(g, kind, src, dst, prm, (cudaStream_t)s, true, false);
 }
 
 int sgb_run_steps(sgb_grid* g, int kind, const int* src, const int* dst, const float* params, int nparams, int nsteps,
@@ -507,8 +509,8 @@ int sgb_run_steps(sgb_grid* g, int kind, const int* src, const int* dst, const f
     // every call took 5-10 us per step on the host before the first step ran (31 heat steps of 6.2 us: 524 us),
     // a launch takes about 2 us beside the step before it.  use_graph also asks for the wait at the end.
     for (int k = 0; k < nsteps; ++k) {
-        if (k % 2 == 0) SGB_TRY(launch_stencil(g, kind, src, dst, fwd, s));
-        else SGB_TRY(launch_stencil(g, kind, dst, src, bwd, s));
+        if (k % 2 == 0) SGB_TRY(launch_stencil(g, kind, src, dst, fwd, s, k > 0));
+        else SGB_TRY(launch_stencil(g, kind, dst, src, bwd, s, k > 0));
     }
     if (use_graph) SGB_CUDA(cudaStreamSynchronize(s));
     return SGB_OK;

@@ -80,6 +80,7 @@ struct LaunchDesc {
     StencilParams prm;
     int64_t t;
     int fill;                // HEAT7: quads without an existing point are written too (dst may hold anything there)
+    int chained;             // follows a launch over the same masks and neighbours in the same call
     unsigned* err;
 };
 
