@@ -14,7 +14,8 @@
 //   4. when new chunks appear: merged index, old chunks moved to their new
 //      positions (128-bit copies), new chunks set to background / empty mask
 //   5. per point: A = op(A, old) when the point exists, mask |= EXIST
-// One device->host read of three counters sizes the new map.
+// One device->host read of three counters and the error word sizes the new
+// map.
 #include <algorithm>
 #include <cstring>
 
@@ -30,19 +31,69 @@ constexpr int kRsTile = kRsThreads * kRsRounds;  // 4096 keys per CTA
 
 constexpr int kRsMaxBuckets = 1024;  // digits of up to 10 bits
 
-template <typename K>
-__global__ void k_rs_hist(const K* keys, int64_t n, int shift, unsigned dmask, int nbuckets, uint32_t* hist,
-                          int ntiles) {
+// Digit counts of every tile, hist[tile][digit].  T: the staged 64-bit linear ids in pass 0, K afterwards.
+template <typename T, typename K>
+__global__ void __launch_bounds__(kRsThreads) k_rs_hist(const T* __restrict__ keys, int64_t n, int shift, unsigned dmask,
+                                                         int nbuckets, uint32_t* __restrict__ hist) {
     __shared__ uint32_t h[kRsMaxBuckets];
-    for (int i = threadIdx.x; i < nbuckets; i += blockDim.x) h[i] = 0;
+    for (int i = threadIdx.x; i < nbuckets; i += kRsThreads) h[i] = 0;
+    const int64_t base = (int64_t)blockIdx.x * kRsTile + threadIdx.x;
+    K k[kRsRounds];  // all loads in flight at once
+#pragma unroll
+    for (int r = 0; r < kRsRounds; ++r) k[r] = base + r * kRsThreads < n ? (K)keys[base + r * kRsThreads] : K(0);
     __syncthreads();
-    const int64_t base = (int64_t)blockIdx.x * kRsTile;
-    for (int k = threadIdx.x; k < kRsTile; k += blockDim.x) {
-        int64_t i = base + k;
-        if (i < n) atomicAdd(&h[(unsigned)(keys[i] >> shift) & dmask], 1u);
+#pragma unroll
+    for (int r = 0; r < kRsRounds; ++r)
+        if (base + r * kRsThreads < n) atomicAdd(&h[(unsigned)(k[r] >> shift) & dmask], 1u);
+    __syncthreads();
+    for (int d = threadIdx.x; d < nbuckets; d += kRsThreads) hist[(size_t)blockIdx.x * nbuckets + d] = h[d];
+}
+
+// Counts to exclusive prefixes over the tiles, digit by digit, in place; tot[d]: the digit's count over all
+// tiles.  A CTA takes 32 digits (one per lane) and splits the tiles over its 32 warps; every access is one
+// coalesced line.
+__global__ void __launch_bounds__(1024) k_rs_rowscan(uint32_t* hist, int ntiles, int nbuckets, uint32_t* tot) {
+    __shared__ uint32_t sums[32][33];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int d = blockIdx.x * 32 + lane;
+    const int per = (ntiles + 31) / 32, t0 = min(ntiles, w * per), t1 = min(ntiles, t0 + per);
+    uint32_t sum = 0;
+    if (d < nbuckets)
+#pragma unroll 8
+        for (int t = t0; t < t1; ++t) sum += hist[(size_t)t * nbuckets + d];
+    sums[w][lane] = sum;
+    __syncthreads();
+    uint32_t run = 0;
+    for (int k = 0; k < w; ++k) run += sums[k][lane];
+    if (d >= nbuckets) return;
+    if (w == 31) tot[d] = run + sum;
+    for (int t = t0; t < t1; t += 8) {
+        uint32_t c[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) c[k] = t + k < t1 ? hist[(size_t)(t + k) * nbuckets + d] : 0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            if (t + k < t1) {
+                hist[(size_t)(t + k) * nbuckets + d] = run;
+                run += c[k];
+            }
     }
+}
+
+// Exclusive scan of one value per thread over the CTA; wsum: one word per warp.
+__device__ __forceinline__ uint32_t rs_block_scan(uint32_t v, uint32_t* wsum) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t u = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += u;
+    }
+    if (lane == 31) wsum[warp] = incl;
     __syncthreads();
-    for (int d = threadIdx.x; d < nbuckets; d += blockDim.x) hist[(size_t)d * ntiles + blockIdx.x] = h[d];
+    uint32_t run = incl - v;
+    for (int w = 0; w < warp; ++w) run += wsum[w];
+    return run;
 }
 
 // Stable scatter: items keep their order inside each digit.  Tile order is
@@ -51,6 +102,12 @@ __global__ void k_rs_hist(const K* keys, int64_t n, int shift, unsigned dmask, i
 // The tile is then staged in shared memory in digit order and written out
 // run by run, so that consecutive threads store consecutive positions of a
 // digit's output range instead of one scattered 4-byte store per item.
+//
+// Bound by latency (ranking rounds, shared memory), 3.3 CTAs per SM at 2 M
+// keys: 27 us (50 us with the loads inside the ranking rounds and one
+// uncoalesced offset read per item).  The loads of a tile all go out before the
+// first ranking round, and the digits' output positions are read once per
+// digit, coalesced.
 template <typename K>
 __host__ __device__ constexpr size_t rs_union_bytes() {
     return (size_t)kRsWarps * kRsMaxBuckets * 4 > (size_t)kRsTile * (sizeof(K) + 4)
@@ -59,33 +116,40 @@ __host__ __device__ constexpr size_t rs_union_bytes() {
 }
 template <typename K>
 __host__ __device__ constexpr size_t rs_scatter_smem() {
-    return rs_union_bytes<K>() + (size_t)kRsMaxBuckets * 4 + kRsWarps * 4;
+    return rs_union_bytes<K>() + (size_t)kRsMaxBuckets * 8 + 2 * kRsWarps * 4;
 }
 
-template <typename K>
-__global__ void __launch_bounds__(kRsThreads) k_rs_scatter(const K* kin, const uint32_t* vin, K* kout, uint32_t* vout,
-                                                            int64_t n, int shift, unsigned dmask, int nbuckets,
-                                                            const uint32_t* offs, int ntiles) {
+template <typename T, typename K>
+__global__ void __launch_bounds__(kRsThreads) k_rs_scatter(const T* __restrict__ kin, const uint32_t* __restrict__ vin,
+                                                            K* __restrict__ kout, uint32_t* __restrict__ vout, int64_t n,
+                                                            int shift, unsigned dmask, int nbuckets,
+                                                            const uint32_t* __restrict__ offs,
+                                                            const uint32_t* __restrict__ tot_g) {
     extern __shared__ __align__(16) unsigned char rs_smem[];
     auto wcnt = reinterpret_cast<uint32_t(*)[kRsMaxBuckets]>(rs_smem);  // [kRsWarps][kRsMaxBuckets]
     K* sk = reinterpret_cast<K*>(rs_smem);                              // the same bytes, once wcnt is done
     uint32_t* sv = reinterpret_cast<uint32_t*>(rs_smem + (size_t)kRsTile * sizeof(K));
-    uint32_t* dstart = reinterpret_cast<uint32_t*>(rs_smem + rs_union_bytes<K>());
-    uint32_t* wsum = dstart + kRsMaxBuckets;
-    for (int i = threadIdx.x; i < kRsWarps * kRsMaxBuckets; i += blockDim.x) (&wcnt[0][0])[i] = 0;
-    __syncthreads();
+    uint32_t* dstart = reinterpret_cast<uint32_t*>(rs_smem + rs_union_bytes<K>());  // digit's first place in the tile
+    uint32_t* gdst = dstart + kRsMaxBuckets;  // output position of the digit's items minus dstart
+    uint32_t* wsum = gdst + kRsMaxBuckets;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t tbase = (int64_t)blockIdx.x * kRsTile;
-    const int64_t base = tbase + warp * (32 * kRsRounds);
+    const int64_t base = tbase + warp * (32 * kRsRounds) + lane;
     K key[kRsRounds];
     uint32_t val[kRsRounds], rank[kRsRounds];
+#pragma unroll
+    for (int r = 0; r < kRsRounds; ++r) {
+        const int64_t i = base + r * 32;
+        key[r] = i < n ? (K)kin[i] : K(0);
+        val[r] = i < n ? (vin ? vin[i] : (uint32_t)i) : 0u;
+    }
+    for (int i = threadIdx.x; i < kRsWarps * kRsMaxBuckets / 4; i += kRsThreads)
+        reinterpret_cast<uint4*>(&wcnt[0][0])[i] = make_uint4(0, 0, 0, 0);
+    __syncthreads();
     const unsigned lt = lanemask_lt();
 #pragma unroll
     for (int r = 0; r < kRsRounds; ++r) {
-        const int64_t i = base + r * 32 + lane;
-        const bool valid = i < n;
-        key[r] = valid ? kin[i] : K(0);
-        val[r] = valid ? (vin ? vin[i] : (uint32_t)i) : 0u;
+        const bool valid = base + r * 32 < n;
         const unsigned d = valid ? ((unsigned)(key[r] >> shift) & dmask) : 0x10000u;
         const unsigned peers = __match_any_sync(0xffffffffu, d);
         uint32_t cnt = 0;
@@ -98,12 +162,14 @@ __global__ void __launch_bounds__(kRsThreads) k_rs_scatter(const K* kin, const u
     __syncthreads();
     // per digit: the warps' counts become prefixes; thread t owns digits kPer t .. kPer t + kPer - 1
     constexpr int kPer = kRsMaxBuckets / kRsThreads;
-    uint32_t tot[kPer], tsum = 0;
+    uint32_t tot[kPer], tsum = 0, gtot[kPer], gsum = 0;
 #pragma unroll
     for (int k = 0; k < kPer; ++k) {
         const int d = threadIdx.x * kPer + k;
         uint32_t run = 0;
+        gtot[k] = d < nbuckets ? tot_g[d] : 0;
         if (d < nbuckets)
+#pragma unroll
             for (int w = 0; w < kRsWarps; ++w) {
                 const uint32_t c = wcnt[w][d];
                 wcnt[w][d] = run;
@@ -111,28 +177,24 @@ __global__ void __launch_bounds__(kRsThreads) k_rs_scatter(const K* kin, const u
             }
         tot[k] = run;
         tsum += run;
+        gsum += gtot[k];
     }
-    // the digits' first positions in the tile: an exclusive scan of the threads' sums
-    uint32_t incl = tsum;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += v;
-    }
-    if (lane == 31) wsum[warp] = incl;
-    __syncthreads();
-    uint32_t run = incl - tsum;
-    for (int w = 0; w < warp; ++w) run += wsum[w];
+    // the digits' first positions in the tile and in the output: exclusive scans of the threads' sums
+    uint32_t run = rs_block_scan(tsum, wsum), grun = rs_block_scan(gsum, wsum + kRsWarps);
 #pragma unroll
     for (int k = 0; k < kPer; ++k) {
         const int d = threadIdx.x * kPer + k;
-        if (d < nbuckets) dstart[d] = run;
+        if (d < nbuckets) {
+            dstart[d] = run;
+            gdst[d] = grun + offs[(size_t)blockIdx.x * nbuckets + d] - run;
+        }
         run += tot[k];
+        grun += gtot[k];
     }
     __syncthreads();
 #pragma unroll
     for (int r = 0; r < kRsRounds; ++r) {
-        if (base + r * 32 + lane < n) {
+        if (base + r * 32 < n) {
             const unsigned d = (unsigned)(key[r] >> shift) & dmask;
             rank[r] += dstart[d] + wcnt[warp][d];  // position in the tile, digit order
         }
@@ -140,26 +202,20 @@ __global__ void __launch_bounds__(kRsThreads) k_rs_scatter(const K* kin, const u
     __syncthreads();  // wcnt is read no more: its bytes take the staged tile
 #pragma unroll
     for (int r = 0; r < kRsRounds; ++r) {
-        if (base + r * 32 + lane < n) {
+        if (base + r * 32 < n) {
             sk[rank[r]] = key[r];
             sv[rank[r]] = val[r];
         }
     }
     __syncthreads();
     const int tn = (int)(n - tbase < kRsTile ? n - tbase : kRsTile);
+#pragma unroll 4
     for (int j = threadIdx.x; j < tn; j += kRsThreads) {
         const K k = sk[j];
-        const unsigned d = (unsigned)(k >> shift) & dmask;
-        const size_t pos = (size_t)offs[(size_t)d * ntiles + blockIdx.x] + (uint32_t)(j - dstart[d]);
+        const uint32_t pos = gdst[(unsigned)(k >> shift) & dmask] + (uint32_t)j;
         kout[pos] = k;
         vout[pos] = sv[j];
     }
-}
-
-template <typename K>
-__global__ void k_make_keys(const int64_t* lin, int64_t n, K* keys) {
-    int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i < n) keys[i] = (K)lin[i];
 }
 
 struct PropSet {
@@ -181,124 +237,288 @@ __device__ __forceinline__ T op_apply(int op, T a, T b) {
     }
 }
 
-// a = op(a, b) on raw elements of type `type` (both operands exist).
-__device__ __forceinline__ void op_raw(int type, int op, unsigned char* a, const unsigned char* b) {
+// Elements of any property type travel as raw 64-bit words.
+__device__ __forceinline__ uint64_t load_raw(int type, const unsigned char* p, int64_t i) {
     switch (type) {
-        case SGB_F32: *(float*)a = op_apply(op, *(const float*)a, *(const float*)b); break;
-        case SGB_F64: *(double*)a = op_apply(op, *(const double*)a, *(const double*)b); break;
+        case SGB_F64: return reinterpret_cast<const uint64_t*>(p)[i];
+        case SGB_U8: return p[i];
+        default: return reinterpret_cast<const uint32_t*>(p)[i];
+    }
+}
+__device__ __forceinline__ void store_raw(int type, unsigned char* p, int64_t i, uint64_t v) {
+    switch (type) {
+        case SGB_F64: reinterpret_cast<uint64_t*>(p)[i] = v; break;
+        case SGB_U8: p[i] = (unsigned char)v; break;
+        default: reinterpret_cast<uint32_t*>(p)[i] = (uint32_t)v;
+    }
+}
+// op(a, b) on raw elements of type `type` (both operands exist).
+__device__ __forceinline__ uint64_t op_raw(int type, int op, uint64_t a, uint64_t b) {
+    if (op == SGB_OP_RIGHT) return b;
+    if (op == SGB_OP_LEFT) return a;
+    switch (type) {
+        case SGB_F32: return __float_as_uint(op_apply(op, __uint_as_float((uint32_t)a), __uint_as_float((uint32_t)b)));
+        case SGB_F64:
+            return (uint64_t)__double_as_longlong(
+                op_apply(op, __longlong_as_double((long long)a), __longlong_as_double((long long)b)));
         case SGB_I32: {
-            int32_t x = *(const int32_t*)a, y = *(const int32_t*)b;
-            *(int32_t*)a = op == SGB_OP_OR ? (x | y) : op_apply(op, x, y);
-            break;
+            const int32_t x = (int32_t)(uint32_t)a, y = (int32_t)(uint32_t)b;
+            return (uint32_t)(op == SGB_OP_OR ? (x | y) : op_apply(op, x, y));
         }
         default: {
-            uint8_t x = *a, y = *b;
-            *a = op == SGB_OP_OR ? (uint8_t)(x | y) : op_apply(op, x, y);
+            const uint8_t x = (uint8_t)a, y = (uint8_t)b;
+            return (uint8_t)(op == SGB_OP_OR ? (uint8_t)(x | y) : op_apply(op, x, y));
         }
     }
 }
 
-__device__ __forceinline__ int esz(int t) { return t == SGB_F64 ? 8 : (t == SGB_U8 ? 1 : 4); }
+// Segment heads of the sorted ids: the first item of every point and of every chunk.  A tile of 2048 items
+// is eight rounds of a 256-thread CTA in index order.
+constexpr int kHdThreads = 256, kHdRounds = 8, kHdTile = kHdThreads * kHdRounds;
 
 template <typename K>
-__global__ void k_heads(const K* sk, int64_t n, int bs_shift, uint32_t* pt_head, uint32_t* blk_head) {
-    int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const K k = sk[i];
-    const bool first = i == 0;
-    const K prev = first ? k : sk[i - 1];
-    pt_head[i] = first || prev != k;
-    blk_head[i] = first || (prev >> bs_shift) != (k >> bs_shift);
-}
-
-// Per point: fold its inserts in insertion order (the sort is stable).
-template <typename K>
-__global__ void k_fold(const K* sk, const uint32_t* sidx, int64_t n, int bs_shift, const uint32_t* pt_head,
-                       const uint32_t* pt_seg, const uint32_t* blk_head, const uint32_t* blk_seg, PropSet vals,
-                       PropSet upt, int64_t* upt_key, int64_t* ublk_key) {
-    int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= n || !pt_head[i]) return;
-    const K k = sk[i];
-    const uint32_t u = pt_seg[i];
-    upt_key[u] = (int64_t)k;
-    if (blk_head[i]) ublk_key[blk_seg[i]] = (int64_t)(k >> bs_shift);
-    for (int p = 0; p < vals.nprop; ++p) {
-        if (vals.op[p] == SGB_OP_NONE) continue;
-        const int t = vals.type[p], es = esz(t);
-        alignas(8) unsigned char acc[8];
-        const unsigned char* src = vals.p[p] + (size_t)sidx[i] * es;
-        for (int b = 0; b < es; ++b) acc[b] = src[b];
-        for (int64_t j = i + 1; j < n && sk[j] == k; ++j) op_raw(t, vals.op[p], acc, vals.p[p] + (size_t)sidx[j] * es);
-        unsigned char* dst = upt.p[p] + (size_t)u * es;
-        for (int b = 0; b < es; ++b) dst[b] = acc[b];
+__device__ __forceinline__ void heads_of(const K* __restrict__ sk, int64_t n, int64_t i, int bs_shift, K& k, bool& pt,
+                                         bool& blk) {
+    pt = blk = false;
+    k = K(0);
+    if (i < n) {
+        k = sk[i];
+        const K prev = i ? sk[i - 1] : k;
+        pt = i == 0 || prev != k;
+        blk = i == 0 || (prev >> bs_shift) != (k >> bs_shift);
     }
 }
 
-__global__ void k_lookup(const int64_t* ublk_key, int64_t nslots, const uint32_t* nb_dev, const int64_t* keys,
-                         int64_t n, uint32_t* isnew) {
-    int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (b < nslots) isnew[b] = b < (int64_t)*nb_dev ? (find_key(keys, n, ublk_key[b]) < 0) : 0u;
+// Points and chunks that begin in every tile.
+template <typename K>
+__global__ void __launch_bounds__(kHdThreads) k_heads_count(const K* __restrict__ sk, int64_t n, int bs_shift,
+                                                             uint2* __restrict__ cnt) {
+    __shared__ uint32_t np, nb;
+    if (threadIdx.x == 0) np = nb = 0;
+    __syncthreads();
+    uint32_t p = 0, b = 0;
+#pragma unroll
+    for (int r = 0; r < kHdRounds; ++r) {
+        K k;
+        bool hp, hb;
+        heads_of(sk, n, (int64_t)blockIdx.x * kHdTile + r * kHdThreads + threadIdx.x, bs_shift, k, hp, hb);
+        p += hp;
+        b += hb;
+    }
+    p = __reduce_add_sync(0xffffffffu, p);
+    b = __reduce_add_sync(0xffffffffu, b);
+    if ((threadIdx.x & 31) == 0) {
+        atomicAdd(&np, p);
+        atomicAdd(&nb, b);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) cnt[blockIdx.x] = make_uint2(np, nb);
 }
 
-__global__ void k_compact_new(const int64_t* ublk_key, int64_t nb, const uint32_t* isnew, const uint32_t* rank,
-                              int64_t* newkeys) {
-    int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (b < nb && isnew[b]) newkeys[rank[b]] = ublk_key[b];
+// Exclusive scan of the tiles' counts by one CTA, in place.  WHICH 0: (points, chunks) pairs, totals to
+// counters[0], [1].  WHICH 1: new chunks per 1024-chunk tile, as many tiles as counters[1] chunks take, total to
+// counters[2]; the device error word goes along to counters[3].
+constexpr int kLkTile = 1024;
+template <int WHICH>
+__global__ void __launch_bounds__(1024) k_tile_scan(uint2* cnt, int64_t ntiles, uint32_t* counters, const unsigned* err) {
+    __shared__ uint32_t wx[32], wy[32];
+    if (WHICH == 1) ntiles = ((int64_t)counters[1] + kLkTile - 1) / kLkTile;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t cx = 0, cy = 0;
+    for (int64_t t0 = 0; t0 < ntiles; t0 += 1024) {
+        const int64_t t = t0 + threadIdx.x;
+        const uint2 v = t < ntiles ? cnt[t] : make_uint2(0, 0);
+        uint32_t x = v.x, y = v.y;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t a = __shfl_up_sync(0xffffffffu, x, o), b = __shfl_up_sync(0xffffffffu, y, o);
+            if (lane >= o) {
+                x += a;
+                y += b;
+            }
+        }
+        if (lane == 31) {
+            wx[warp] = x;
+            wy[warp] = y;
+        }
+        __syncthreads();
+        uint32_t bx = cx, by = cy;
+        for (int w = 0; w < 32; ++w) {
+            if (w < warp) {
+                bx += wx[w];
+                by += wy[w];
+            }
+            cx += wx[w];
+            cy += wy[w];
+        }
+        if (t < ntiles) cnt[t] = make_uint2(bx + x - v.x, by + y - v.y);
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        if (WHICH == 0) {
+            counters[0] = cx;
+            counters[1] = cy;
+        } else {
+            counters[2] = cx;
+            counters[3] = *err;
+        }
+    }
+}
+
+// Per point: fold its inserts in insertion order (the sort is stable).  The point's chunk (its rank among the
+// touched chunks) and offset go to upt, the reduced values to vals_out, the touched chunks' ids to ublk_key.
+template <typename K>
+__global__ void __launch_bounds__(kHdThreads) k_fold(const K* __restrict__ sk, const uint32_t* __restrict__ sidx, int64_t n,
+                                                      int bs_shift, const uint2* __restrict__ tile_off, PropSet vals,
+                                                      PropSet out, uint2* __restrict__ upt, int64_t* __restrict__ ublk_key) {
+    constexpr int W = kHdThreads / 32;
+    __shared__ uint32_t pre[kHdRounds * W];  // points | chunks << 16 that begin before (round, warp) in the tile
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t base = (int64_t)blockIdx.x * kHdTile + threadIdx.x;
+    K key[kHdRounds];
+    unsigned pb[kHdRounds], bb[kHdRounds];
+#pragma unroll
+    for (int r = 0; r < kHdRounds; ++r) {
+        bool hp, hb;
+        heads_of(sk, n, base + r * kHdThreads, bs_shift, key[r], hp, hb);
+        pb[r] = __ballot_sync(0xffffffffu, hp);
+        bb[r] = __ballot_sync(0xffffffffu, hb);
+        if (lane == 0) pre[r * W + warp] = __popc(pb[r]) | __popc(bb[r]) << 16;
+    }
+    __syncthreads();
+    if (warp == 0) {  // 64 entries, two per lane
+        const uint32_t a = pre[2 * lane], b = pre[2 * lane + 1];
+        uint32_t incl = a + b;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += v;
+        }
+        pre[2 * lane] = incl - a - b;
+        pre[2 * lane + 1] = incl - b;
+    }
+    __syncthreads();
+    const uint2 off = tile_off[blockIdx.x];
+    const unsigned lt = lanemask_lt(), le = lt | 1u << lane;
+#pragma unroll
+    for (int r = 0; r < kHdRounds; ++r) {
+        if (!(pb[r] >> lane & 1u)) continue;
+        const int64_t i = base + r * kHdThreads;
+        const K k = key[r];
+        const uint32_t pr = pre[r * W + warp];
+        const uint32_t u = off.x + (pr & 0xffffu) + __popc(pb[r] & lt);
+        const uint32_t b = off.y + (pr >> 16) + __popc(bb[r] & le) - 1;
+        upt[u] = make_uint2(b, (uint32_t)(k & (((K)1 << bs_shift) - 1)));
+        if (bb[r] >> lane & 1u) ublk_key[b] = (int64_t)(k >> bs_shift);
+        // the point's inserts are items [i, e)
+        int64_t e = i + 1;
+        while (e < n && sk[e] == k) ++e;
+        for (int p = 0; p < vals.nprop; ++p) {
+            const int op = vals.op[p], t = vals.type[p];
+            if (op == SGB_OP_NONE) continue;
+            uint64_t acc = load_raw(t, vals.p[p], sidx[op == SGB_OP_RIGHT ? e - 1 : i]);  // the last one stands
+            if (op != SGB_OP_RIGHT && op != SGB_OP_LEFT)
+                for (int64_t j = i + 1; j < e; ++j) acc = op_raw(t, op, acc, load_raw(t, vals.p[p], sidx[j]));
+            store_raw(t, out.p[p], u, acc);
+        }
+    }
+}
+
+// The touched chunks in the current index: 2 x (old chunks below its id) + (1 when it is new), and the number of
+// new ones per 1024-chunk tile.  How many there are is known on the device only.
+__global__ void __launch_bounds__(256) k_lookup(const int64_t* __restrict__ ublk_key, const uint32_t* __restrict__ counters,
+                                                 const int64_t* __restrict__ keys, int64_t n, int64_t* __restrict__ place,
+                                                 uint2* __restrict__ cnt) {
+    __shared__ uint32_t nnew;
+    const int64_t nb = counters[1];
+    for (int64_t t = blockIdx.x; t * kLkTile < nb; t += gridDim.x) {
+        if (threadIdx.x == 0) nnew = 0;
+        __syncthreads();
+        uint32_t c = 0;
+        for (int k = 0; k < kLkTile; k += 256) {
+            const int64_t b = t * kLkTile + k + threadIdx.x;
+            if (b < nb) {
+                const int64_t key = ublk_key[b];
+                const int64_t lo = lower_bound_i64(keys, n, key);
+                const bool isnew = !(lo < n && keys[lo] == key);
+                place[b] = 2 * lo + isnew;
+                c += isnew;
+            }
+        }
+        c = __reduce_add_sync(0xffffffffu, c);
+        if ((threadIdx.x & 31) == 0) atomicAdd(&nnew, c);
+        __syncthreads();
+        if (threadIdx.x == 0) cnt[t] = make_uint2(nnew, 0);
+        __syncthreads();
+    }
+}
+
+// Positions in the merged map: (old chunks below) + (new chunks below).  place[b] becomes 2 x that; the new
+// chunks also enter the new-key list and the merged index.
+__global__ void __launch_bounds__(kLkTile) k_merge_pos(const int64_t* __restrict__ ublk_key, int64_t nb, int64_t* place,
+                                                        const uint2* __restrict__ tile_off, int64_t* __restrict__ newkeys,
+                                                        int64_t* __restrict__ keys_out, int32_t* __restrict__ srcpos) {
+    __shared__ uint32_t wsum[32];
+    const int64_t b = (int64_t)blockIdx.x * kLkTile + threadIdx.x;
+    const int64_t v = b < nb ? place[b] : 0;
+    const uint32_t isnew = (uint32_t)(v & 1);
+    const uint32_t rank = tile_off[blockIdx.x].x + rs_block_scan(isnew, wsum);
+    if (b >= nb) return;
+    const int64_t pos = (v >> 1) + rank;
+    place[b] = 2 * pos;
+    if (isnew) {
+        const int64_t key = ublk_key[b];
+        newkeys[rank] = key;
+        keys_out[pos] = key;
+        srcpos[pos] = -1;
+    }
 }
 
 // New position of every old chunk: j + #(new keys below its key).
-__global__ void k_old_pos(const int64_t* keys, int64_t n, const int64_t* newkeys, int64_t nnew, int64_t* keys_out,
-                          int64_t* newpos) {
-    int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+__global__ void k_old_pos(const int64_t* __restrict__ keys, int64_t n, const int64_t* __restrict__ newkeys, int64_t nnew,
+                          int64_t* __restrict__ keys_out, int32_t* __restrict__ srcpos) {
+    const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (j >= n) return;
     const int64_t k = keys[j];
     const int64_t pos = j + lower_bound_i64(newkeys, nnew, k);
-    newpos[j] = pos;
+    srcpos[pos] = (int32_t)j;
     keys_out[pos] = k;
 }
 
-__global__ void k_new_pos(const int64_t* newkeys, int64_t nnew, const int64_t* keys, int64_t n, int64_t* keys_out,
-                          int64_t* newpos) {
-    int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (r >= nnew) return;
-    const int64_t k = newkeys[r];
-    const int64_t pos = r + lower_bound_i64(keys, n, k);
-    newpos[r] = pos;
-    keys_out[pos] = k;
-}
+struct MapSet {
+    const uint4* src[kMaxProps + 1];
+    uint4* dst[kMaxProps + 1];
+    uint4 fill[kMaxProps + 1];
+    int shift[kMaxProps + 1];  // a chunk holds 2^shift 16-byte words
+    int count;
+};
 
-// Chunk moves as a flat stream of 16-byte words: word i of the old map (of
-// chunk i >> cw_shift; a chunk holds 2^cw_shift words) goes to the same word
-// of the chunk's merged position.  Four independent copies are in flight per
-// thread and the loads are coalesced, whatever a chunk's size.
-__global__ void k_move_chunks(const uint4* __restrict__ src, uint4* __restrict__ dst, int64_t nchunks, int cw_shift,
-                              const int64_t* __restrict__ newpos) {
-    const int64_t total = nchunks << cw_shift, wmask = (int64_t(1) << cw_shift) - 1;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    for (; i + 3 * stride < total; i += 4 * stride) {
-        uint4 v[4];
-        int64_t d[4];
+// The merged map, all properties and the masks: a warp per chunk of it copies the old chunk there or fills a new
+// one (and the background chunk at position n) with backgrounds and a zero mask.  Bound by HBM: 6.8 TB/s.
+__global__ void __launch_bounds__(256) k_merge_map(MapSet ms, const int32_t* __restrict__ srcpos, int64_t n) {
+    const int lane = threadIdx.x & 31;
+    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    for (int64_t c = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; c <= n; c += nw) {
+        const int64_t s = c < n ? srcpos[c] : -1;
+        for (int p = 0; p < ms.count; ++p) {
+            const int words = 1 << ms.shift[p];
+            uint4* d = ms.dst[p] + (c << ms.shift[p]);
+            if (s < 0) {
+                for (int w = lane; w < words; w += 32) d[w] = ms.fill[p];
+                continue;
+            }
+            const uint4* q = ms.src[p] + (s << ms.shift[p]);
+            if (words == 128) {
+                uint4 v[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const int64_t j = i + k * stride;
-            v[k] = __ldcs(src + j);  // the old map is read once
-            d[k] = (__ldg(newpos + (j >> cw_shift)) << cw_shift) | (j & wmask);
+                for (int k = 0; k < 4; ++k) v[k] = __ldcs(q + lane + 32 * k);  // the old map is read once
+#pragma unroll
+                for (int k = 0; k < 4; ++k) d[lane + 32 * k] = v[k];
+            } else {
+                for (int w = lane; w < words; w += 32) d[w] = __ldcs(q + w);
+            }
         }
-#pragma unroll
-        for (int k = 0; k < 4; ++k) dst[d[k]] = v[k];
     }
-    for (; i < total; i += stride) dst[(__ldg(newpos + (i >> cw_shift)) << cw_shift) | (i & wmask)] = __ldcs(src + i);
-}
-
-// New chunks get the background pattern (or a zero mask), the same flat word stream.
-__global__ void k_fill_chunks(uint4* __restrict__ dst, int64_t nnew, int cw_shift, uint4 word,
-                              const int64_t* __restrict__ newpos) {
-    const int64_t total = nnew << cw_shift, wmask = (int64_t(1) << cw_shift) - 1;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-#pragma unroll 4
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += stride)
-        dst[(__ldg(newpos + (i >> cw_shift)) << cw_shift) | (i & wmask)] = word;
 }
 
 // The element pattern of es bytes repeated over a 16-byte word.
@@ -311,30 +531,38 @@ static uint4 replicate16(uint64_t pattern, int es) {
 }
 
 // Per unique point: reduce with the existing value, write, set EXIST.
-__global__ void k_scatter(const int64_t* upt_key, int64_t nu, int bs_shift, const int64_t* keys, int64_t n,
-                          PropSet upt, PropSet data, uint8_t* mask, int any_listed) {
-    int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+__global__ void k_scatter(const uint2* __restrict__ upt, int64_t nu, int bs_shift, const int64_t* __restrict__ place,
+                          PropSet upv, PropSet data, uint8_t* mask, int any_listed) {
+    const int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (u >= nu) return;
-    const int64_t k = upt_key[u];
-    const int64_t pos = find_key(keys, n, k >> bs_shift);
-    if (pos < 0) return;  // cannot happen: every chunk id was merged in
-    const int64_t bsm = (1ll << bs_shift) - 1;
-    const size_t idx = (size_t)pos * (bsm + 1) + (size_t)(k & bsm);
+    const uint2 q = upt[u];
+    const int64_t idx = (place[q.x] >> 1 << bs_shift) + q.y;
     const uint8_t om = mask[idx];
     for (int p = 0; p < data.nprop; ++p) {
-        if (data.op[p] == SGB_OP_NONE) continue;
-        const int t = data.type[p], es = esz(t);
-        alignas(8) unsigned char acc[8];
-        const unsigned char* a = upt.p[p] + (size_t)u * es;
-        for (int b = 0; b < es; ++b) acc[b] = a[b];
-        unsigned char* d = data.p[p] + idx * es;
-        if (om & 1) op_raw(t, data.op[p], acc, d);  // op(new, old), BlockMapGpu_kernels.cuh:294-305
-        for (int b = 0; b < es; ++b) d[b] = acc[b];
+        const int op = data.op[p], t = data.type[p];
+        if (op == SGB_OP_NONE) continue;
+        if ((om & 1) && op == SGB_OP_RIGHT) continue;  // op(new, old) = old
+        uint64_t v = load_raw(t, upv.p[p], u);
+        if ((om & 1) && op != SGB_OP_LEFT) v = op_raw(t, op, v, load_raw(t, data.p[p], idx));  // BlockMapGpu_kernels.cuh:294-305
+        store_raw(t, data.p[p], idx, v);
     }
-    if (any_listed) mask[idx] = om | 1u;
+    if (any_listed && !(om & 1)) mask[idx] = om | 1u;
 }
 
 static inline unsigned nblk(int64_t n, int t = 256) { return (unsigned)((n + t - 1) / t); }
+
+template <typename T, typename K>
+static int radix_pass(const T* kin, const uint32_t* vin, K* kout, uint32_t* vout, int64_t n, int shift, unsigned dmask,
+                      int nbuckets, uint32_t* hist, uint32_t* tot, int ntiles, cudaStream_t s) {
+    k_rs_hist<T, K><<<ntiles, kRsThreads, 0, s>>>(kin, n, shift, dmask, nbuckets, hist);
+    k_rs_rowscan<<<(nbuckets + 31) / 32, 1024, 0, s>>>(hist, ntiles, nbuckets, tot);
+    constexpr size_t smem = rs_scatter_smem<K>();
+    if (smem > 48 * 1024)
+        SGB_CUDA(cudaFuncSetAttribute(k_rs_scatter<T, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    k_rs_scatter<T, K><<<ntiles, kRsThreads, smem, s>>>(kin, vin, kout, vout, n, shift, dmask, nbuckets, hist, tot);
+    SGB_CUDA(cudaGetLastError());
+    return SGB_OK;
+}
 
 template <typename K>
 static int radix_sort(sgb_grid* g, int64_t n, int bits, K** keys_out, uint32_t** vals_out, cudaStream_t s) {
@@ -343,7 +571,6 @@ static int radix_sort(sgb_grid* g, int64_t n, int bits, K** keys_out, uint32_t**
     DevBuf& vA = g->scratch[2];
     DevBuf& vB = g->scratch[3];
     DevBuf& hist = g->scratch[4];
-    DevBuf& hoff = g->scratch[5];
     SGB_TRY(kA.ensure((size_t)n * sizeof(K)));
     SGB_TRY(kB.ensure((size_t)n * sizeof(K)));
     SGB_TRY(vA.ensure((size_t)n * 4));
@@ -354,32 +581,19 @@ static int radix_sort(sgb_grid* g, int64_t n, int bits, K** keys_out, uint32_t**
     const int dbits = bits <= 0 ? 1 : (bits + passes - 1) / passes;
     const int nbuckets = 1 << dbits;
     const unsigned dmask = (unsigned)nbuckets - 1u;
-    SGB_TRY(hist.ensure((size_t)ntiles * nbuckets * 4));
-    SGB_TRY(hoff.ensure((size_t)ntiles * nbuckets * 4));
-    k_make_keys<K><<<nblk(n), 256, 0, s>>>(g->pend_lin.as<int64_t>(), n, kA.as<K>());
-    SGB_CUDA(cudaGetLastError());
-    K* kin = kA.as<K>();
-    K* kout = kB.as<K>();
+    SGB_TRY(hist.ensure(((size_t)ntiles + 1) * nbuckets * 4));
+    uint32_t* h = hist.as<uint32_t>();
+    uint32_t* tot = h + (size_t)ntiles * nbuckets;
+    K* kbuf[2] = {kA.as<K>(), kB.as<K>()};
     uint32_t* vbuf[2] = {vA.as<uint32_t>(), vB.as<uint32_t>()};
-    for (int ps = 0; ps < passes; ++ps) {
-        const int shift = ps * dbits;
-        const uint32_t* vin = ps == 0 ? nullptr : vbuf[ps & 1];  // pass 0 ranks the insertion index itself
-        uint32_t* vout = vbuf[(ps + 1) & 1];
-        k_rs_hist<K><<<ntiles, 256, 0, s>>>(kin, n, shift, dmask, nbuckets, hist.as<uint32_t>(), ntiles);
-        SGB_CUDA(cudaGetLastError());
-        SGB_TRY(scan_exclusive_u32(hist.as<uint32_t>(), hoff.as<uint32_t>(), (int64_t)ntiles * nbuckets, nullptr,
-                                   &g->scratch[6], s));
-        constexpr size_t smem = rs_scatter_smem<K>();
-        SGB_CUDA(cudaFuncSetAttribute(k_rs_scatter<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k_rs_scatter<K><<<ntiles, kRsThreads, smem, s>>>(kin, vin, kout, vout, n, shift, dmask, nbuckets,
-                                                         hoff.as<uint32_t>(), ntiles);
-        SGB_CUDA(cudaGetLastError());
-        K* kt = kin;
-        kin = kout;
-        kout = kt;
-    }
-    *vals_out = vbuf[passes & 1];
-    *keys_out = kin;
+    // pass 0 takes the staged ids as they are and ranks the insertion index itself
+    SGB_TRY((radix_pass<int64_t, K>(g->pend_lin.as<int64_t>(), nullptr, kbuf[0], vbuf[0], n, 0, dmask, nbuckets, h, tot,
+                                    ntiles, s)));
+    for (int ps = 1; ps < passes; ++ps)
+        SGB_TRY((radix_pass<K, K>(kbuf[(ps + 1) & 1], vbuf[(ps + 1) & 1], kbuf[ps & 1], vbuf[ps & 1], n, ps * dbits, dmask,
+                                  nbuckets, h, tot, ntiles, s)));
+    *vals_out = vbuf[(passes + 1) & 1];
+    *keys_out = kbuf[(passes + 1) & 1];
     return SGB_OK;
 }
 
@@ -392,68 +606,65 @@ static int flush_impl(sgb_grid* g, const int* ops, int bits, cudaStream_t s) {
     uint32_t* sidx = nullptr;
     SGB_TRY(radix_sort<K>(g, n, bits, &sk, &sidx, s));
 
-    DevBuf& heads = g->scratch[7];
-    DevBuf& segs = g->scratch[8];
+    DevBuf& tiles = g->scratch[7];
     DevBuf& ubuf = g->scratch[9];
     DevBuf& uval = g->scratch[10];
     DevBuf& cnt = g->scratch[11];
-    SGB_TRY(heads.ensure((size_t)n * 8));
-    SGB_TRY(segs.ensure((size_t)n * 8 + 64));
+    const int64_t htiles = (n + kHdTile - 1) / kHdTile, ltiles = (n + kLkTile - 1) / kLkTile;
+    SGB_TRY(tiles.ensure((size_t)(htiles + ltiles) * 8));
     SGB_TRY(cnt.ensure(64));
-    uint32_t* pt_head = heads.as<uint32_t>();
-    uint32_t* blk_head = pt_head + n;
-    uint32_t* pt_seg = segs.as<uint32_t>();
-    uint32_t* blk_seg = pt_seg + n;
-    uint32_t* counters = cnt.as<uint32_t>();  // [0] U, [1] B, [2] NB
-    k_heads<K><<<nblk(n), 256, 0, s>>>(sk, n, bs_shift, pt_head, blk_head);
-    SGB_CUDA(cudaGetLastError());
-    SGB_TRY(scan_exclusive_u32(pt_head, pt_seg, n, counters + 0, &g->scratch[6], s));
-    SGB_TRY(scan_exclusive_u32(blk_head, blk_seg, n, counters + 1, &g->scratch[6], s));
+    uint2* htile = tiles.as<uint2>();
+    uint2* ltile = htile + htiles;
+    uint32_t* counters = cnt.as<uint32_t>();  // [0] U, [1] B, [2] NB, [3] error word
 
     // unique points / chunks: at most n of each
     size_t uval_bytes = 0;
     for (int p = 0; p < g->nprop; ++p) uval_bytes += ((size_t)n * elem_size(g->ptype[p]) + 15) & ~(size_t)15;
     SGB_TRY(uval.ensure(uval_bytes + 64));
-    // ubuf: upt_key[n] int64 | ublk_key[n] int64 | isnew[n] u32 | rank[n] u32 | newkeys[n] int64
+    // ubuf: upt[n] uint2 | ublk_key[n] int64 | place[n] int64 | newkeys[n] int64
     SGB_TRY(ubuf.ensure((size_t)n * 32 + 256));
-    int64_t* upt_key = ubuf.as<int64_t>();
-    int64_t* ublk_key = upt_key + n;
-    uint32_t* isnew = (uint32_t*)(ublk_key + n);
-    uint32_t* rank = isnew + n;
-    int64_t* newkeys = (int64_t*)(rank + n);
+    uint2* upt = ubuf.as<uint2>();
+    int64_t* ublk_key = reinterpret_cast<int64_t*>(upt + n);
+    int64_t* place = ublk_key + n;
+    int64_t* newkeys = place + n;
 
-    PropSet vals{}, upt{}, data{};
-    vals.nprop = upt.nprop = data.nprop = g->nprop;
+    PropSet vals{}, upv{}, data{};
+    vals.nprop = upv.nprop = data.nprop = g->nprop;
     size_t off = 0;
     int any_listed = 0;
     for (int p = 0; p < g->nprop; ++p) {
         vals.p[p] = g->pend_val[p].as<unsigned char>();
-        upt.p[p] = uval.as<unsigned char>() + off;
+        upv.p[p] = uval.as<unsigned char>() + off;
         off += ((size_t)n * elem_size(g->ptype[p]) + 15) & ~(size_t)15;
-        vals.type[p] = upt.type[p] = data.type[p] = g->ptype[p];
-        vals.op[p] = upt.op[p] = data.op[p] = ops[p];
+        vals.type[p] = upv.type[p] = data.type[p] = g->ptype[p];
+        vals.op[p] = upv.op[p] = data.op[p] = ops[p];
         any_listed |= ops[p] != SGB_OP_NONE;
     }
-    k_fold<K><<<nblk(n), 256, 0, s>>>(sk, sidx, n, bs_shift, pt_head, pt_seg, blk_head, blk_seg, vals, upt, upt_key,
-                                      ublk_key);
+    k_heads_count<K><<<(unsigned)htiles, kHdThreads, 0, s>>>(sk, n, bs_shift, htile);
+    k_tile_scan<0><<<1, 1024, 0, s>>>(htile, htiles, counters, nullptr);
+    k_fold<K><<<(unsigned)htiles, kHdThreads, 0, s>>>(sk, sidx, n, bs_shift, htile, vals, upv, upt, ublk_key);
+    k_lookup<<<(unsigned)std::min<int64_t>(ltiles, (int64_t)g->num_sms * 8), 256, 0, s>>>(
+        ublk_key, counters, g->keys.as<int64_t>(), g->n, place, ltile);
+    k_tile_scan<1><<<1, 1024, 0, s>>>(ltile, 0, counters, g->err.as<unsigned>());
     SGB_CUDA(cudaGetLastError());
-
-    // B is only known on the device: every slot below n is looked up, the
-    // ones at or above B report "not new".
-    k_lookup<<<nblk(n), 256, 0, s>>>(ublk_key, n, counters + 1, g->keys.as<int64_t>(), g->n, isnew);
-    SGB_CUDA(cudaGetLastError());
-    SGB_TRY(scan_exclusive_u32(isnew, rank, n, counters + 2, &g->scratch[6], s));
     SGB_TRY(g->hscratch.ensure(64));
-    SGB_CUDA(cudaMemcpyAsync(g->hscratch.p, counters, 12, cudaMemcpyDeviceToHost, s));
+    SGB_CUDA(cudaMemcpyAsync(g->hscratch.p, counters, 16, cudaMemcpyDeviceToHost, s));
     SGB_CUDA(cudaStreamSynchronize(s));
     const int64_t U = ((uint32_t*)g->hscratch.p)[0];
     const int64_t B = ((uint32_t*)g->hscratch.p)[1];
     const int64_t NB = ((uint32_t*)g->hscratch.p)[2];
+    // out-of-domain points were flagged at insert time; nothing of the map has been touched yet
+    const unsigned e = ((uint32_t*)g->hscratch.p)[3];
+    if (e & (kErrOutOfDomain | kErrPoolOverflow)) {
+        SGB_CUDA(cudaMemsetAsync(g->err.p, 0, 4, s));
+        set_error((e & kErrOutOfDomain)
+                      ? "an inserted point lies outside the grid domain; the staged inserts were dropped"
+                      : "an insert pool counted more points than its slots; the staged inserts were dropped");
+        return SGB_ERANGE;
+    }
 
     if (NB > 0) {
         const int64_t nold = g->n, nn_ = nold + NB;
-        k_compact_new<<<nblk(B), 256, 0, s>>>(ublk_key, B, isnew, rank, newkeys);
-        SGB_CUDA(cudaGetLastError());
         // second buffer set for the new map (contents are rebuilt): kept while it holds the map,
         // otherwise allocated for twice the map, so that a growing map reallocates rarely (each
         // reallocation frees and maps gigabytes and stalls the device)
@@ -467,52 +678,26 @@ static int flush_impl(sgb_grid* g, const int* ops, int bits, cudaStream_t s) {
             for (int p = 0; p < g->nprop; ++p)
                 SGB_TRY(g->data2[p].ensure((size_t)(cap2 + 1) * bs * elem_size(g->ptype[p])));
         }
-        DevBuf& posbuf = g->scratch[5];  // histogram offsets are no longer needed
-        SGB_TRY(posbuf.ensure((size_t)(nold + NB) * 8 + 64));
-        int64_t* oldpos = posbuf.as<int64_t>();
-        int64_t* npos = oldpos + nold;
-        if (nold > 0) {
-            k_old_pos<<<nblk(nold), 256, 0, s>>>(g->keys.as<int64_t>(), nold, newkeys, NB, g->keys2.as<int64_t>(),
-                                                 oldpos);
-            SGB_CUDA(cudaGetLastError());
-        }
-        k_new_pos<<<nblk(NB), 256, 0, s>>>(newkeys, NB, g->keys.as<int64_t>(), nold, g->keys2.as<int64_t>(), npos);
+        DevBuf& posbuf = g->scratch[5];
+        SGB_TRY(posbuf.ensure((size_t)nn_ * 4 + 64));
+        int32_t* srcpos = posbuf.as<int32_t>();
+        k_merge_pos<<<(unsigned)((B + kLkTile - 1) / kLkTile), kLkTile, 0, s>>>(ublk_key, B, place, ltile, newkeys,
+                                                                                 g->keys2.as<int64_t>(), srcpos);
+        if (nold > 0)
+            k_old_pos<<<nblk(nold), 256, 0, s>>>(g->keys.as<int64_t>(), nold, newkeys, NB, g->keys2.as<int64_t>(), srcpos);
         SGB_CUDA(cudaGetLastError());
-        // flat word streams: at most 16 CTAs of 256 threads per SM, no more threads than words
-        auto word_grid = [&](int64_t chunks, int cw_shift) {
-            const int64_t words = chunks << cw_shift;
-            return (unsigned)std::max<int64_t>(1, std::min<int64_t>((int64_t)g->num_sms * 16, (words + 255) / 256));
-        };
-        auto shift_of = [](int words) {  // chunk sizes in 16-byte words are powers of two
-            int sh = 0;
-            while ((1 << sh) < words) ++sh;
-            return sh;
-        };
-        const int msh = shift_of(bs / 16);
-        if ((1 << msh) != bs / 16) {  // chunk edges are powers of two, so every chunk is 2^k words
-            set_error("chunk size is not a power of two 16-byte words");
-            return SGB_ENOTSUP;
-        }
-        for (int p = 0; p < g->nprop; ++p) {
-            const int es = elem_size(g->ptype[p]);
-            const int sh = shift_of(bs * es / 16);
-            if (nold > 0) {
-                k_move_chunks<<<word_grid(nold, sh), 256, 0, s>>>(g->data[p].as<uint4>(), g->data2[p].as<uint4>(),
-                                                                  nold, sh, oldpos);
-                SGB_CUDA(cudaGetLastError());
-            }
+        MapSet ms{};
+        ms.count = g->nprop + 1;
+        for (int p = 0; p <= g->nprop; ++p) {
+            const int es = p < g->nprop ? elem_size(g->ptype[p]) : 1;
+            ms.src[p] = p < g->nprop ? g->data[p].as<uint4>() : g->mask.as<uint4>();
+            ms.dst[p] = p < g->nprop ? g->data2[p].as<uint4>() : g->mask2.as<uint4>();
             uint64_t pat = 0;
-            std::memcpy(&pat, g->bck[p], es);
-            k_fill_chunks<<<word_grid(NB, sh), 256, 0, s>>>(g->data2[p].as<uint4>(), NB, sh, replicate16(pat, es),
-                                                            npos);
-            SGB_CUDA(cudaGetLastError());
+            if (p < g->nprop) std::memcpy(&pat, g->bck[p], es);
+            ms.fill[p] = replicate16(pat, es);
+            while ((16 << ms.shift[p]) < bs * es) ++ms.shift[p];  // chunk edges are powers of two
         }
-        if (nold > 0) {
-            k_move_chunks<<<word_grid(nold, msh), 256, 0, s>>>(g->mask.as<uint4>(), g->mask2.as<uint4>(), nold, msh,
-                                                               oldpos);
-            SGB_CUDA(cudaGetLastError());
-        }
-        k_fill_chunks<<<word_grid(NB, msh), 256, 0, s>>>(g->mask2.as<uint4>(), NB, msh, make_uint4(0, 0, 0, 0), npos);
+        k_merge_map<<<(unsigned)std::min<int64_t>((nn_ + 8) / 8, (int64_t)g->num_sms * 8), 256, 0, s>>>(ms, srcpos, nn_);
         SGB_CUDA(cudaGetLastError());
         // swap buffer sets
         std::swap(g->keys, g->keys2);
@@ -520,11 +705,9 @@ static int flush_impl(sgb_grid* g, const int* ops, int bits, cudaStream_t s) {
         for (int p = 0; p < g->nprop; ++p) std::swap(g->data[p], g->data2[p]);
         g->cap = cap2;
         g->n = nn_;
-        SGB_TRY(write_background(g, g->n, s, g->data, g->mask));
     }
     for (int p = 0; p < g->nprop; ++p) data.p[p] = g->data[p].as<unsigned char>();
-    k_scatter<<<nblk(U), 256, 0, s>>>(upt_key, U, bs_shift, g->keys.as<int64_t>(), g->n, upt, data,
-                                      g->mask.as<uint8_t>(), any_listed);
+    k_scatter<<<nblk(U), 256, 0, s>>>(upt, U, bs_shift, place, upv, data, g->mask.as<uint8_t>(), any_listed);
     SGB_CUDA(cudaGetLastError());
     return SGB_OK;
 }
@@ -541,19 +724,6 @@ extern "C" int sgb_flush(sgb_grid* g, const int* ops, sgb_stream stream) {
     }
     cudaStream_t s = (cudaStream_t)stream;
     if (g->npend == 0) return SGB_OK;
-    // out-of-domain points were flagged at insert time
-    SGB_TRY(g->hscratch.ensure(64));
-    SGB_CUDA(cudaMemcpyAsync(g->hscratch.p, g->err.p, 4, cudaMemcpyDeviceToHost, s));
-    SGB_CUDA(cudaStreamSynchronize(s));
-    const unsigned e = *(unsigned*)g->hscratch.p;
-    if (e & (kErrOutOfDomain | kErrPoolOverflow)) {
-        SGB_CUDA(cudaMemsetAsync(g->err.p, 0, 4, s));
-        g->npend = 0;
-        set_error((e & kErrOutOfDomain)
-                      ? "an inserted point lies outside the grid domain; the staged inserts were dropped"
-                      : "an insert pool counted more points than its slots; the staged inserts were dropped");
-        return SGB_ERANGE;
-    }
     const int64_t maxlin = key_space(g->geo) * g->geo.bs;
     int bits = 0;
     while (bits < 63 && (int64_t(1) << bits) < maxlin) ++bits;

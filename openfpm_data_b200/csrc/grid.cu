@@ -360,8 +360,9 @@ __global__ void k_lin_from_coords(const int32_t* coords, int64_t n, Geometry geo
     if (i >= n) return;
     int64_t c[3];
     bool ok = true;
-    for (int d = 0; d < geo.dim; ++d) {
-        c[d] = coords[i * geo.dim + d];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        c[d] = coords[i * 3 + d];
         ok &= c[d] >= 0 && c[d] < geo.size[d];
     }
     if (!ok) {
@@ -370,7 +371,7 @@ __global__ void k_lin_from_coords(const int32_t* coords, int64_t n, Geometry geo
         return;
     }
     int64_t b, l;
-    point_key(geo, c, &b, &l);
+    point_key_in(geo, c, &b, &l);
     lin[i] = b * geo.bs + l;
 }
 
@@ -416,7 +417,7 @@ __global__ void k_get(const int32_t* coords, int64_t n, Geometry geo, const int6
         return;
     }
     int64_t b, l;
-    point_key(geo, c, &b, &l);
+    point_key_in(geo, c, &b, &l);
     int64_t pos = find_key(keys, nchunks, b);
     if (pos < 0) pos = nchunks;
     // BlockMapGpu_ker::get (src/SparseGridGpu/BlockMapGpu_ker.cuh:117-135)

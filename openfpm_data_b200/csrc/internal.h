@@ -207,6 +207,15 @@ __host__ __device__ inline void point_key(const Geometry& g, const int64_t* c, i
     *local = l;
 }
 
+// point_key of a point inside the domain, with shifts instead of 64-bit divisions (chunk edges are 4 or 8; a
+// negative coordinate would round the other way).  2 M coordinates: 30 us with divisions, 9 us so.
+__host__ __device__ inline void point_key_in(const Geometry& g, const int64_t* c, int64_t* key, int64_t* local) {
+    const int sh = g.edge == 8 ? 3 : 2, m = g.edge - 1;
+    const int64_t bx = c[0] >> sh, by = c[1] >> sh, bz = c[2] >> sh;
+    *key = g.zorder ? block_key(g, bx, by, bz) : bx + g.bsz[0] * (by + g.bsz[1] * bz);
+    *local = (c[0] & m) | ((c[1] & m) | (c[2] & m) << sh) << sh;
+}
+
 // Is a chunk id one of a block inside the domain?
 __host__ __device__ inline bool key_in_domain(const Geometry& g, int64_t key) {
     if (key < 0 || key >= key_space(g)) return false;

@@ -290,7 +290,7 @@ __global__ void k_unpack_stage(const unsigned char* __restrict__ buf, PackLayout
     int64_t lin = -1;
     if (ok) {
         int64_t b, l;
-        point_key(dst_geo, c, &b, &l);
+        point_key_in(dst_geo, c, &b, &l);
         lin = b * dst_geo.bs + l;
     } else {
         atomicOr(err, kErrOutOfDomain);
@@ -400,7 +400,7 @@ __global__ void k_unpack_stage_all(const unsigned char* __restrict__ buf, const 
     int64_t lin = -1;
     if (ok) {
         int64_t kb, kl;
-        point_key(dst_geo, c, &kb, &kl);
+        point_key_in(dst_geo, c, &kb, &kl);
         lin = kb * dst_geo.bs + kl;
     } else {
         atomicOr(err, kErrOutOfDomain);

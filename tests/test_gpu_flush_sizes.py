@@ -1,0 +1,56 @@
+"""Flush at the sizes where its kernels' tiles end: 2048 items (segment heads), 4096 keys (sort), 1024 touched
+chunks (lookup), against the CPU oracle; block maps, masks and values are exact."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def sgb():
+    import openfpm_data_b200 as m
+    m.load()
+    return m
+
+
+@pytest.mark.parametrize("edge", [8, 4])
+@pytest.mark.parametrize("n", [1, 31, 2047, 2048, 2049, 4096, 4097, 12289, 70000])
+@pytest.mark.parametrize("spread", [6, 120])
+def test_flush_sizes(sgb, edge, n, spread):
+    """n inserts with duplicates in a small or large part of the domain, then as many again (merge into the map).
+    float32 maxima, float64 and uint8 last / first values, int32 bit sets: no sum whose order could matter."""
+    rng = np.random.default_rng(n + spread + edge)
+    size = (130, 121, 125)
+    g = sgb.SparseGridGpu(size, ["f32", "f64", "i32", "u8"], edge=edge)
+    o = O.OracleGrid(size, edge=edge, ptypes=[O.T_F32, O.T_F64, O.T_I32, O.T_U8])
+    names = ["smax_", "sRight_", "sBitwiseOr_", "sLeft_"]
+    ops = [O.OP_MAX, O.OP_RIGHT, O.OP_OR, O.OP_LEFT]
+    for _ in range(2):
+        pts = rng.integers(0, spread, size=(n, 3)).astype(np.int64)
+        vals = [rng.standard_normal(n).astype(np.float32), rng.standard_normal(n),
+                rng.integers(0, 2 ** 31 - 1, n).astype(np.int32), rng.integers(0, 255, n).astype(np.uint8)]
+        g.insert(torch.from_numpy(pts.astype(np.int32)).cuda(), [torch.from_numpy(v).cuda() for v in vals])
+        g.flush(names)
+        o.insert_flush(pts, vals, ops)
+    keys, data, mask = g.deviceToHost()
+    okeys, odata, omask = o.export()
+    assert np.array_equal(keys, okeys) and np.array_equal(mask, omask)
+    ex = (mask & 1).astype(bool)
+    for a, b in zip(data, odata):
+        assert np.array_equal(a[ex], np.asarray(b)[ex])
+
+
+def test_flush_drops_out_of_domain(sgb):
+    """The staged points are dropped and the map stays as it was when one of them lies outside."""
+    g = sgb.SparseGridGpu((40, 40, 40), ["f32"], edge=8)
+    p = torch.tensor([[1, 2, 3], [9, 9, 9]], dtype=torch.int32, device="cuda")
+    g.insert(p, [torch.ones(2, device="cuda")])
+    g.flush(["sRight_"])
+    g.insert(torch.tensor([[20, 20, 20], [40, 0, 0]], dtype=torch.int32, device="cuda"), [torch.ones(2, device="cuda")])
+    with pytest.raises(sgb.SgbError):
+        g.flush(["sRight_"])
+    g.flush(["sRight_"])
+    assert g.countExistingElements() == 2 and g.nchunks == 2
