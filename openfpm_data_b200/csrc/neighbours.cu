@@ -176,9 +176,12 @@ __global__ void k_tag_star8(const uint64_t* bits, const int32_t* nn, int64_t n, 
     if (chunk >= n) return;
     constexpr uint64_t COL0 = 0x0101010101010101ull, COL7 = COL0 << 7;
     const int z = lane & 7;
-    const int32_t* nb = nn + chunk * 8;
+    uint4* mp = reinterpret_cast<uint4*>(mask + (size_t)chunk * 512) + lane;
+    uint4 v = *mp;  // on its way while the neighbours' bitmaps are fetched
+    const int4 na = __ldg(reinterpret_cast<const int4*>(nn + chunk * 8));
+    const int2 nz = __ldg(reinterpret_cast<const int2*>(nn + chunk * 8 + 4));
     const uint64_t W = bits[chunk * 8 + z];
-    const int32_t xm = nb[0], xp = nb[1], ym = nb[2], yp = nb[3], zm = nb[4], zp = nb[5];
+    const int32_t xm = na.x, xp = na.y, ym = na.z, yp = na.w, zm = nz.x, zp = nz.y;
     const uint64_t XM = xm >= 0 ? bits[(int64_t)xm * 8 + z] : 0;
     const uint64_t XP = xp >= 0 ? bits[(int64_t)xp * 8 + z] : 0;
     const uint64_t YM = ym >= 0 ? bits[(int64_t)ym * 8 + z] : 0;
@@ -195,21 +198,16 @@ __global__ void k_tag_star8(const uint64_t* bits, const int32_t* nn, int64_t n, 
     // lane l rewrites mask bytes [16l, 16l+16): z-slice l/4, bits 16*(l%4)..
     const uint64_t pw = __shfl_sync(0xffffffffu, pad, lane >> 2);
     const unsigned bits16 = (unsigned)(pw >> (16 * (lane & 3))) & 0xffffu;
-    uint4* mp = reinterpret_cast<uint4*>(mask + (size_t)chunk * 512) + lane;
-    uint4 v = *mp;
     unsigned w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-        unsigned out = 0;
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            unsigned m = (w[q] >> (8 * b)) & 0xffu;
-            if (m & 1u) m = ((bits16 >> (q * 4 + b)) & 1u) ? (m | 2u) : (m & ~2u);
-            out |= m << (8 * b);
-        }
-        w[q] = out;
+        // the four points' padding bits, one per byte; only bytes with EXIST change
+        const unsigned b4 = bits16 >> (4 * q) & 0xfu;
+        const unsigned p = (b4 | b4 << 7 | b4 << 14 | b4 << 21) & 0x01010101u, ex = w[q] & 0x01010101u;
+        w[q] = (w[q] & ~(ex << 1)) | (p & ex) << 1;
     }
-    *mp = make_uint4(w[0], w[1], w[2], w[3]);
+    const uint4 o = make_uint4(w[0], w[1], w[2], w[3]);
+    if (o.x != v.x || o.y != v.y || o.z != v.z || o.w != v.w) *mp = o;
 }
 
 // Generic tagBoundaries for any edge and both neighbourhoods: one CTA per

@@ -36,42 +36,35 @@ __global__ void k_ep_count(const uint64_t* __restrict__ bits, int64_t n, int bs,
     }
 }
 
-// Emission: warp per chunk, lane l owns points [l * P, l * P + P) with P = bs / 32; a warp
-// scan of the lanes' counts places each lane's ids, written in point order.  The next chunk's
-// bitmap slice and offset are loaded before the current chunk is written out.
+// Emission: a warp per chunk, 32 points per round: each round's existing points go to consecutive places, so the
+// stores are coalesced (18.9 K chunks, 6.7 M points: 41 us with 16 points per lane, 8.3 us so; 27 MB written).
+// The next chunk's bitmap and offset are loaded before the current chunk is written out.
 __global__ void k_ep_emit(const uint64_t* __restrict__ bits, int64_t n, int bs, const uint32_t* __restrict__ offs,
-                          uint32_t* out) {
+                          uint32_t* __restrict__ out) {
     constexpr unsigned kAll = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    const int P = bs >> 5, words = bs >> 6;
-    const int first = lane * P, wi = first >> 6, sh = first & 63;
-    const uint32_t pmask = P >= 32 ? ~0u : (1u << P) - 1u;
+    const int rounds = bs >> 5;
+    const uint32_t* w32 = reinterpret_cast<const uint32_t*>(bits);
+    const unsigned lt = lanemask_lt();
     int64_t c = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    uint32_t m = 0, pos = 0;
+    uint32_t m = 0, pos = 0;  // lane r holds the bitmap of round r
     if (c < n) {
-        m = (uint32_t)(__ldg(bits + c * words + wi) >> sh) & pmask;
+        m = lane < rounds ? __ldg(w32 + c * rounds + lane) : 0u;
         pos = __ldg(offs + c);
     }
     for (; c < n; c += nw) {
         const int64_t cn = c + nw;
         uint32_t mn = 0, posn = 0;
         if (cn < n) {
-            mn = (uint32_t)(__ldg(bits + cn * words + wi) >> sh) & pmask;
+            mn = lane < rounds ? __ldg(w32 + cn * rounds + lane) : 0u;
             posn = __ldg(offs + cn);
         }
-        const uint32_t cnt = __popc(m);
-        uint32_t pre = cnt;  // inclusive prefix over the lanes
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t v = __shfl_up_sync(kAll, pre, o);
-            if (lane >= o) pre += v;
-        }
-        uint32_t p = pos + pre - cnt;
-        const uint32_t base = (uint32_t)(c * bs) + (uint32_t)first;
-        while (m) {
-            out[p++] = base + (uint32_t)(__ffs(m) - 1);
-            m &= m - 1;
+        const uint32_t id = (uint32_t)(c * bs) + (uint32_t)lane;
+        for (int r = 0; r < rounds; ++r) {
+            const uint32_t w = __shfl_sync(kAll, m, r);
+            if (w >> lane & 1u) out[pos + __popc(w & lt)] = id + (uint32_t)(r * 32);
+            pos += __popc(w);
         }
         m = mn;
         pos = posn;
