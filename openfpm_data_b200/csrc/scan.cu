@@ -69,6 +69,71 @@ __global__ void k_scan_tiles(const uint32_t* in, int64_t n, const uint32_t* offs
     if (total_dev && blockIdx.x == gridDim.x - 1 && threadIdx.x == kScanThreads - 1) *total_dev = pre;
 }
 
+// Short arrays: one CTA walks them, 16384 items a round (three launches of a few CTAs each cost 10.5 us for 19 K
+// items, this 8.1 us).  VEC: 16-byte accesses, for 16-byte aligned arrays.
+constexpr int64_t kScanOneMax = 65536;
+constexpr int kScanOneItems = 16;
+template <bool VEC>
+__global__ void __launch_bounds__(1024) k_scan_one(const uint32_t* __restrict__ in, int64_t n, uint32_t* __restrict__ out,
+                                                    uint32_t* total_dev) {
+    __shared__ uint32_t ws[33];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t carry = 0;
+    for (int64_t t0 = 0; t0 < n; t0 += 1024 * kScanOneItems) {
+        const int64_t base = t0 + threadIdx.x * kScanOneItems;
+        uint32_t v[kScanOneItems], s = 0;
+        if (VEC && base + kScanOneItems <= n) {
+#pragma unroll
+            for (int k = 0; k < kScanOneItems / 4; ++k)
+                *reinterpret_cast<uint4*>(v + 4 * k) = *reinterpret_cast<const uint4*>(in + base + 4 * k);
+        } else {
+#pragma unroll
+            for (int k = 0; k < kScanOneItems; ++k) v[k] = base + k < n ? in[base + k] : 0;
+        }
+#pragma unroll
+        for (int k = 0; k < kScanOneItems; ++k) {
+            const uint32_t c = v[k];
+            v[k] = s;
+            s += c;
+        }
+        uint32_t incl = s;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t u = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += u;
+        }
+        if (lane == 31) ws[warp] = incl;
+        __syncthreads();
+        if (warp == 0) {
+            const uint32_t w = ws[lane];
+            uint32_t x = w;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t u = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= o) x += u;
+            }
+            ws[lane] = x - w;
+            if (lane == 31) ws[32] = x;
+        }
+        __syncthreads();
+        const uint32_t pre = carry + ws[warp] + incl - s;
+        carry += ws[32];
+#pragma unroll
+        for (int k = 0; k < kScanOneItems; ++k) v[k] += pre;
+        if (VEC && base + kScanOneItems <= n) {
+#pragma unroll
+            for (int k = 0; k < kScanOneItems / 4; ++k)
+                *reinterpret_cast<uint4*>(out + base + 4 * k) = *reinterpret_cast<uint4*>(v + 4 * k);
+        } else {
+#pragma unroll
+            for (int k = 0; k < kScanOneItems; ++k)
+                if (base + k < n) out[base + k] = v[k];
+        }
+        __syncthreads();
+    }
+    if (total_dev && threadIdx.x == 0) *total_dev = carry;
+}
+
 // tmp must provide scratch for the tile sums of every level.
 int scan_exclusive_u32(const uint32_t* in, uint32_t* out, int64_t n, uint32_t* total_dev, DevBuf* tmp,
                        cudaStream_t s) {
@@ -76,12 +141,14 @@ int scan_exclusive_u32(const uint32_t* in, uint32_t* out, int64_t n, uint32_t* t
         if (total_dev) SGB_CUDA(cudaMemsetAsync(total_dev, 0, 4, s));
         return SGB_OK;
     }
-    const int64_t tiles = (n + kScanTile - 1) / kScanTile;
-    if (tiles == 1) {
-        k_scan_tiles<<<1, kScanThreads, 0, s>>>(in, n, nullptr, out, total_dev);
+    if (n <= kScanOneMax) {
+        const bool vec = ((uintptr_t)in | (uintptr_t)out) % 16 == 0;
+        if (vec) k_scan_one<true><<<1, 1024, 0, s>>>(in, n, out, total_dev);
+        else k_scan_one<false><<<1, 1024, 0, s>>>(in, n, out, total_dev);
         SGB_CUDA(cudaGetLastError());
         return SGB_OK;
     }
+    const int64_t tiles = (n + kScanTile - 1) / kScanTile;
     SGB_TRY(tmp->reserve((size_t)tiles * 4 * 2 + 64));
     uint32_t* sums = tmp->as<uint32_t>();
     uint32_t* offs = sums + tiles;
