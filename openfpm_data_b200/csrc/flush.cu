@@ -96,18 +96,31 @@ __device__ __forceinline__ uint32_t rs_block_scan(uint32_t v, uint32_t* wsum) {
     return run;
 }
 
+// The warp's lanes with the same digit, by one ballot per digit bit (__match_any_sync, whose time grows with the
+// distinct values in the warp, makes a 2 M key pass with random digits 4 us longer).
+__device__ __forceinline__ unsigned digit_peers(unsigned d, bool valid, unsigned dmask) {
+    unsigned peers = __ballot_sync(0xffffffffu, valid);
+#pragma unroll
+    for (int b = 0; b < 10; ++b) {
+        if (!(dmask >> b & 1u)) break;  // uniform
+        const unsigned m = __ballot_sync(0xffffffffu, d >> b & 1u);
+        peers &= (d >> b & 1u) ? m : ~m;
+    }
+    return peers;
+}
+
 // Stable scatter: items keep their order inside each digit.  Tile order is
-// (warp, round, lane) == index order; ranks inside a warp come from
-// __match_any_sync peer groups, counts across warps from a shared prefix.
+// (warp, round, lane) == index order; ranks inside a warp come from the peer
+// groups of equal digits, counts across warps from a shared prefix.
 // The tile is then staged in shared memory in digit order and written out
 // run by run, so that consecutive threads store consecutive positions of a
 // digit's output range instead of one scattered 4-byte store per item.
 //
 // Bound by latency (ranking rounds, shared memory), 3.3 CTAs per SM at 2 M
-// keys: 27 us (50 us with the loads inside the ranking rounds and one
-// uncoalesced offset read per item).  The loads of a tile all go out before the
-// first ranking round, and the digits' output positions are read once per
-// digit, coalesced.
+// keys: 25-30 us (50 us with __match_any_sync, the loads inside the ranking
+// rounds and one uncoalesced offset read per item).  The keys of a tile all go
+// out before the first ranking round, the digits' output positions are read
+// once per digit, coalesced, and 64 registers let four CTAs share an SM.
 template <typename K>
 __host__ __device__ constexpr size_t rs_union_bytes() {
     return (size_t)kRsWarps * kRsMaxBuckets * 4 > (size_t)kRsTile * (sizeof(K) + 4)
@@ -120,7 +133,7 @@ __host__ __device__ constexpr size_t rs_scatter_smem() {
 }
 
 template <typename T, typename K>
-__global__ void __launch_bounds__(kRsThreads) k_rs_scatter(const T* __restrict__ kin, const uint32_t* __restrict__ vin,
+__global__ void __launch_bounds__(kRsThreads, sizeof(K) == 4 ? 4 : 2) k_rs_scatter(const T* __restrict__ kin, const uint32_t* __restrict__ vin,
                                                             K* __restrict__ kout, uint32_t* __restrict__ vout, int64_t n,
                                                             int shift, unsigned dmask, int nbuckets,
                                                             const uint32_t* __restrict__ offs,
@@ -136,12 +149,11 @@ __global__ void __launch_bounds__(kRsThreads) k_rs_scatter(const T* __restrict__
     const int64_t tbase = (int64_t)blockIdx.x * kRsTile;
     const int64_t base = tbase + warp * (32 * kRsRounds) + lane;
     K key[kRsRounds];
-    uint32_t val[kRsRounds], rank[kRsRounds];
+    uint32_t rank[kRsRounds];
 #pragma unroll
     for (int r = 0; r < kRsRounds; ++r) {
         const int64_t i = base + r * 32;
         key[r] = i < n ? (K)kin[i] : K(0);
-        val[r] = i < n ? (vin ? vin[i] : (uint32_t)i) : 0u;
     }
     for (int i = threadIdx.x; i < kRsWarps * kRsMaxBuckets / 4; i += kRsThreads)
         reinterpret_cast<uint4*>(&wcnt[0][0])[i] = make_uint4(0, 0, 0, 0);
@@ -150,8 +162,8 @@ __global__ void __launch_bounds__(kRsThreads) k_rs_scatter(const T* __restrict__
 #pragma unroll
     for (int r = 0; r < kRsRounds; ++r) {
         const bool valid = base + r * 32 < n;
-        const unsigned d = valid ? ((unsigned)(key[r] >> shift) & dmask) : 0x10000u;
-        const unsigned peers = __match_any_sync(0xffffffffu, d);
+        const unsigned d = (unsigned)(key[r] >> shift) & dmask;
+        const unsigned peers = digit_peers(d, valid, dmask);
         uint32_t cnt = 0;
         if (valid) cnt = wcnt[warp][d];
         rank[r] = cnt + __popc(peers & lt);
@@ -160,6 +172,12 @@ __global__ void __launch_bounds__(kRsThreads) k_rs_scatter(const T* __restrict__
         __syncwarp();
     }
     __syncthreads();
+    uint32_t val[kRsRounds];  // needed from here on
+#pragma unroll
+    for (int r = 0; r < kRsRounds; ++r) {
+        const int64_t i = base + r * 32;
+        val[r] = i < n ? (vin ? vin[i] : (uint32_t)i) : 0u;
+    }
     // per digit: the warps' counts become prefixes; thread t owns digits kPer t .. kPer t + kPer - 1
     constexpr int kPer = kRsMaxBuckets / kRsThreads;
     uint32_t tot[kPer], tsum = 0, gtot[kPer], gsum = 0;
@@ -272,6 +290,19 @@ __device__ __forceinline__ uint64_t op_raw(int type, int op, uint64_t a, uint64_
     }
 }
 
+// The rest of a point's inserts folded into its first one, in insertion order.  A call: inlined into the unrolled
+// rounds of its users it takes 218 registers.
+__device__ __noinline__ uint64_t fold_rest(int type, int op, uint64_t acc, const unsigned char* vals,
+                                           const uint32_t* __restrict__ sidx, uint32_t len) {
+    for (uint32_t j = 1; j < len; ++j) acc = op_raw(type, op, acc, load_raw(type, vals, sidx[j]));
+    return acc;
+}
+__device__ __noinline__ uint64_t fold_rest16(int type, int op, uint64_t acc, const unsigned char* vals,
+                                             const uint16_t* sidx, uint32_t len) {
+    for (uint32_t j = 1; j < len; ++j) acc = op_raw(type, op, acc, load_raw(type, vals, sidx[j]));
+    return acc;
+}
+
 // Segment heads of the sorted ids: the first item of every point and of every chunk.  A tile of 2048 items
 // is eight rounds of a 256-thread CTA in index order.
 constexpr int kHdThreads = 256, kHdRounds = 8, kHdTile = kHdThreads * kHdRounds;
@@ -368,7 +399,7 @@ __global__ void __launch_bounds__(1024) k_tile_scan(uint2* cnt, int64_t ntiles, 
 // Per point: fold its inserts in insertion order (the sort is stable).  The point's chunk (its rank among the
 // touched chunks) and offset go to upt, the reduced values to vals_out, the touched chunks' ids to ublk_key.
 template <typename K>
-__global__ void __launch_bounds__(kHdThreads) k_fold(const K* __restrict__ sk, const uint32_t* __restrict__ sidx, int64_t n,
+__global__ void __launch_bounds__(kHdThreads, 3) k_fold(const K* __restrict__ sk, const uint32_t* __restrict__ sidx, int64_t n,
                                                       int bs_shift, const uint2* __restrict__ tile_off, PropSet vals,
                                                       PropSet out, uint2* __restrict__ upt, int64_t* __restrict__ ublk_key) {
     constexpr int W = kHdThreads / 32;
@@ -400,33 +431,54 @@ __global__ void __launch_bounds__(kHdThreads) k_fold(const K* __restrict__ sk, c
     __syncthreads();
     const uint2 off = tile_off[blockIdx.x];
     const unsigned lt = lanemask_lt(), le = lt | 1u << lane;
+    // round by round: the point's rank, how many inserts it has, and its first and last one's staging index
+    uint32_t u[kHdRounds], len[kHdRounds], first[kHdRounds], last[kHdRounds];
 #pragma unroll
     for (int r = 0; r < kHdRounds; ++r) {
+        len[r] = 0;
         if (!(pb[r] >> lane & 1u)) continue;
         const int64_t i = base + r * kHdThreads;
         const K k = key[r];
         const uint32_t pr = pre[r * W + warp];
-        const uint32_t u = off.x + (pr & 0xffffu) + __popc(pb[r] & lt);
         const uint32_t b = off.y + (pr >> 16) + __popc(bb[r] & le) - 1;
-        upt[u] = make_uint2(b, (uint32_t)(k & (((K)1 << bs_shift) - 1)));
+        u[r] = off.x + (pr & 0xffffu) + __popc(pb[r] & lt);
+        upt[u[r]] = make_uint2(b, (uint32_t)(k & (((K)1 << bs_shift) - 1)));
         if (bb[r] >> lane & 1u) ublk_key[b] = (int64_t)(k >> bs_shift);
-        // the point's inserts are items [i, e)
-        int64_t e = i + 1;
-        while (e < n && sk[e] == k) ++e;
-        for (int p = 0; p < vals.nprop; ++p) {
-            const int op = vals.op[p], t = vals.type[p];
-            if (op == SGB_OP_NONE) continue;
-            uint64_t acc = load_raw(t, vals.p[p], sidx[op == SGB_OP_RIGHT ? e - 1 : i]);  // the last one stands
+        const unsigned next = pb[r] & ~le;  // the next point begins at that lane, or past the warp's items
+        uint32_t c = next ? (uint32_t)(__ffs(next) - 1 - lane) : (uint32_t)(32 - lane);
+        if (!next)
+            while (i + c < n && sk[i + c] == k) ++c;
+        len[r] = i + c < n ? c : (uint32_t)(n - i);
+        first[r] = sidx[i];
+        last[r] = len[r] > 1 ? sidx[i + len[r] - 1] : first[r];
+    }
+    for (int p = 0; p < vals.nprop; ++p) {
+        const int op = vals.op[p], t = vals.type[p];
+        if (op == SGB_OP_NONE) continue;
+        auto reduce = [&](auto zero) {
+            using T = decltype(zero);
+            const T* src = reinterpret_cast<const T*>(vals.p[p]);
+            T* dst = reinterpret_cast<T*>(out.p[p]);
+            T v[kHdRounds];  // all of the thread's values in flight at once
+#pragma unroll
+            for (int r = 0; r < kHdRounds; ++r) v[r] = len[r] ? src[op == SGB_OP_RIGHT ? last[r] : first[r]] : zero;
             if (op != SGB_OP_RIGHT && op != SGB_OP_LEFT)
-                for (int64_t j = i + 1; j < e; ++j) acc = op_raw(t, op, acc, load_raw(t, vals.p[p], sidx[j]));
-            store_raw(t, out.p[p], u, acc);
-        }
+#pragma unroll
+                for (int r = 0; r < kHdRounds; ++r)
+                    if (len[r] > 1) v[r] = (T)fold_rest(t, op, v[r], vals.p[p], sidx + base + r * kHdThreads, len[r]);
+#pragma unroll
+            for (int r = 0; r < kHdRounds; ++r)
+                if (len[r]) dst[u[r]] = v[r];
+        };
+        if (t == SGB_F64) reduce(uint64_t(0));
+        else if (t == SGB_U8) reduce(uint8_t(0));
+        else reduce(uint32_t(0));
     }
 }
 
 // The touched chunks in the current index: 2 x (old chunks below its id) + (1 when it is new), and the number of
 // new ones per 1024-chunk tile.  How many there are is known on the device only.
-__global__ void __launch_bounds__(256) k_lookup(const int64_t* __restrict__ ublk_key, const uint32_t* __restrict__ counters,
+__global__ void __launch_bounds__(kLkTile) k_lookup(const int64_t* __restrict__ ublk_key, const uint32_t* __restrict__ counters,
                                                  const int64_t* __restrict__ keys, int64_t n, int64_t* __restrict__ place,
                                                  uint2* __restrict__ cnt) {
     __shared__ uint32_t nnew;
@@ -435,15 +487,13 @@ __global__ void __launch_bounds__(256) k_lookup(const int64_t* __restrict__ ublk
         if (threadIdx.x == 0) nnew = 0;
         __syncthreads();
         uint32_t c = 0;
-        for (int k = 0; k < kLkTile; k += 256) {
-            const int64_t b = t * kLkTile + k + threadIdx.x;
-            if (b < nb) {
-                const int64_t key = ublk_key[b];
-                const int64_t lo = lower_bound_i64(keys, n, key);
-                const bool isnew = !(lo < n && keys[lo] == key);
-                place[b] = 2 * lo + isnew;
-                c += isnew;
-            }
+        const int64_t b = t * kLkTile + threadIdx.x;
+        if (b < nb) {
+            const int64_t key = ublk_key[b];
+            const int64_t lo = lower_bound_i64(keys, n, key);
+            const bool isnew = !(lo < n && keys[lo] == key);
+            place[b] = 2 * lo + isnew;
+            c = isnew;
         }
         c = __reduce_add_sync(0xffffffffu, c);
         if ((threadIdx.x & 31) == 0) atomicAdd(&nnew, c);
@@ -530,12 +580,9 @@ static uint4 replicate16(uint64_t pattern, int es) {
     return w;
 }
 
-// Per unique point: reduce with the existing value, write, set EXIST.
-__global__ void k_scatter(const uint2* __restrict__ upt, int64_t nu, int bs_shift, const int64_t* __restrict__ place,
-                          PropSet upv, PropSet data, uint8_t* mask, int any_listed) {
-    const int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (u >= nu) return;
-    const uint2 q = upt[u];
+// A unique point: reduce with the existing value, write, set EXIST.
+__device__ __forceinline__ void write_point(uint2 q, int64_t u, int bs_shift, const int64_t* place, const PropSet& upv,
+                                            const PropSet& data, uint8_t* mask, int any_listed) {
     const int64_t idx = (place[q.x] >> 1 << bs_shift) + q.y;
     const uint8_t om = mask[idx];
     for (int p = 0; p < data.nprop; ++p) {
@@ -547,6 +594,199 @@ __global__ void k_scatter(const uint2* __restrict__ upt, int64_t nu, int bs_shif
         store_raw(t, data.p[p], idx, v);
     }
     if (any_listed && !(om & 1)) mask[idx] = om | 1u;
+}
+
+__global__ void k_scatter(const uint2* __restrict__ upt, int64_t nu, int bs_shift, const int64_t* __restrict__ place,
+                          PropSet upv, PropSet data, uint8_t* mask, int any_listed) {
+    const int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (u < nu) write_point(upt[u], u, bs_shift, place, upv, data, mask, any_listed);
+}
+
+// ------------------------------------------------------------------ small flushes in one launch
+// Up to 8192 staged points: one CTA sorts them in shared memory (digits of at most 8 bits, eight items per thread),
+// folds the points' inserts, looks the touched chunks up and, when none of them is new, writes the results back --
+// what the kernels above do in 14 launches of a few CTAs, each bound by its launch and memory latency.  (5003
+// points into a 128^3 map, whole call: 123 us with those, 92 us so.)
+constexpr int kSmThreads = 1024, kSmItems = 8, kSmMax = kSmThreads * kSmItems, kSmBuckets = 256;
+
+template <typename K>
+constexpr size_t small_smem() {
+    // keys, indexes, per-warp digit counts, digit starts
+    return (size_t)kSmMax * (sizeof(K) + 2) + (size_t)32 * kSmBuckets * 2 + (size_t)kSmBuckets * 4 * 5;
+}
+
+template <typename K>
+__global__ void __launch_bounds__(kSmThreads) k_flush_small(const int64_t* __restrict__ lin, int n, int passes, int dbits,
+                                                             int bs_shift, PropSet vals, PropSet out, PropSet data,
+                                                             uint8_t* mask, int any_listed, const int64_t* __restrict__ keys,
+                                                             int64_t nold, uint2* upt, int64_t* ublk_key, int64_t* place,
+                                                             uint2* ltile, uint32_t* counters, const unsigned* err) {
+    extern __shared__ __align__(16) unsigned char sm_raw[];
+    K* sk = reinterpret_cast<K*>(sm_raw);
+    uint16_t* si = reinterpret_cast<uint16_t*>(sk + kSmMax);
+    auto wcnt = reinterpret_cast<uint16_t(*)[kSmBuckets]>(si + kSmMax);  // [32 warps]
+    auto part = reinterpret_cast<uint32_t(*)[kSmBuckets]>(wcnt + 32);    // [4]: sums of eight warps each
+    uint32_t* dstart = &part[4][0];
+    __shared__ uint32_t ws[33];
+    __shared__ unsigned bad;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const unsigned lt = lanemask_lt(), dmask = (1u << dbits) - 1u;
+    if (tid == 0) bad = *err & (kErrOutOfDomain | kErrPoolOverflow);
+    K key[kSmItems];
+    uint32_t idx[kSmItems], rank[kSmItems];
+    const int base = warp * 32 * kSmItems + lane;  // items in (warp, round, lane) order
+#pragma unroll
+    for (int r = 0; r < kSmItems; ++r) {
+        const int i = base + 32 * r;
+        key[r] = i < n ? (K)lin[i] : K(0);
+        idx[r] = (uint32_t)i;
+    }
+    for (int ps = 0; ps < passes; ++ps) {
+        const int shift = ps * dbits;
+        reinterpret_cast<uint4*>(wcnt)[tid] = make_uint4(0, 0, 0, 0);
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < kSmItems; ++r) {
+            const bool valid = base + 32 * r < n;
+            const unsigned d = (unsigned)(key[r] >> shift) & dmask;
+            const unsigned peers = digit_peers(d, valid, dmask);
+            uint32_t c = 0;
+            if (valid) c = wcnt[warp][d];
+            rank[r] = c + __popc(peers & lt);
+            __syncwarp();
+            if (valid && lane == __ffs(peers) - 1) wcnt[warp][d] = (uint16_t)(c + __popc(peers));
+            __syncwarp();
+        }
+        __syncthreads();
+        {  // counts to prefixes over the warps: a thread takes one digit of eight warps
+            const int d = tid & (kSmBuckets - 1), q = tid >> 8;
+            uint32_t sum = 0;
+#pragma unroll
+            for (int w = 0; w < 8; ++w) sum += wcnt[q * 8 + w][d];
+            part[q][d] = sum;
+            __syncthreads();
+            uint32_t run = 0;
+            for (int k = 0; k < q; ++k) run += part[k][d];
+#pragma unroll
+            for (int w = 0; w < 8; ++w) {
+                const uint32_t c = wcnt[q * 8 + w][d];
+                wcnt[q * 8 + w][d] = (uint16_t)run;
+                run += c;
+            }
+            if (warp == 0) {  // the digits' starts: eight digits per lane
+                uint32_t t[8], s = 0;
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    const int e = lane * 8 + k;
+                    t[k] = s;
+                    s += part[0][e] + part[1][e] + part[2][e] + part[3][e];
+                }
+                uint32_t incl = s;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t u = __shfl_up_sync(0xffffffffu, incl, o);
+                    if (lane >= o) incl += u;
+                }
+#pragma unroll
+                for (int k = 0; k < 8; ++k) dstart[lane * 8 + k] = t[k] + incl - s;
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < kSmItems; ++r)
+            if (base + 32 * r < n) {
+                const unsigned d = (unsigned)(key[r] >> shift) & dmask;
+                const uint32_t pos = dstart[d] + wcnt[warp][d] + rank[r];
+                sk[pos] = key[r];
+                si[pos] = (uint16_t)idx[r];
+            }
+        __syncthreads();
+        if (ps + 1 < passes)
+#pragma unroll
+            for (int r = 0; r < kSmItems; ++r)
+                if (base + 32 * r < n) {
+                    key[r] = sk[base + 32 * r];
+                    idx[r] = si[base + 32 * r];
+                }
+    }
+    // heads: a thread takes eight consecutive items; ranks by one scan (points | chunks << 16)
+    const int i0 = tid * kSmItems;
+    uint32_t hp = 0, hb = 0;  // bit k: item i0 + k begins a point / a chunk
+#pragma unroll
+    for (int k = 0; k < kSmItems; ++k) {
+        const int i = i0 + k;
+        if (i < n) {
+            const K c = sk[i], p = i ? sk[i - 1] : c;
+            if (i == 0 || c != p) hp |= 1u << k;
+            if (i == 0 || (c >> bs_shift) != (p >> bs_shift)) hb |= 1u << k;
+        }
+    }
+    const uint32_t mine = __popc(hp) | (uint32_t)__popc(hb) << 16;
+    const uint32_t before = rs_block_scan(mine, ws);
+    if (tid == kSmThreads - 1) ws[32] = before + mine;
+    __syncthreads();
+    const uint32_t U = ws[32] & 0xffffu, B = ws[32] >> 16;
+    uint32_t len[kSmItems], first[kSmItems], last[kSmItems];
+    const uint32_t u0 = before & 0xffffu, b0 = before >> 16;
+#pragma unroll
+    for (int k = 0; k < kSmItems; ++k) {
+        len[k] = 0;
+        if (!(hp >> k & 1u)) continue;
+        const int i = i0 + k;
+        const K c = sk[i];
+        const uint32_t b = b0 + __popc(hb & ((2u << k) - 1u)) - 1;
+        upt[u0 + __popc(hp & ((1u << k) - 1u))] = make_uint2(b, (uint32_t)(c & (((K)1 << bs_shift) - 1)));
+        if (hb >> k & 1u) ublk_key[b] = (int64_t)(c >> bs_shift);
+        int e = i + 1;
+        while (e < n && sk[e] == c) ++e;
+        len[k] = (uint32_t)(e - i);
+        first[k] = si[i];
+        last[k] = si[e - 1];
+    }
+    for (int p = 0; p < vals.nprop; ++p) {
+        const int op = vals.op[p], t = vals.type[p];
+        if (op == SGB_OP_NONE) continue;
+        auto reduce = [&](auto zero) {
+            using T = decltype(zero);
+            const T* src = reinterpret_cast<const T*>(vals.p[p]);
+            T* dst = reinterpret_cast<T*>(out.p[p]);
+            T v[kSmItems];
+#pragma unroll
+            for (int k = 0; k < kSmItems; ++k) v[k] = len[k] ? src[op == SGB_OP_RIGHT ? last[k] : first[k]] : zero;
+            if (op != SGB_OP_RIGHT && op != SGB_OP_LEFT)
+#pragma unroll
+                for (int k = 0; k < kSmItems; ++k)
+                    if (len[k] > 1) v[k] = (T)fold_rest16(t, op, v[k], vals.p[p], si + i0 + k, len[k]);
+#pragma unroll
+            for (int k = 0; k < kSmItems; ++k)
+                if (len[k]) dst[u0 + __popc(hp & ((1u << k) - 1u))] = v[k];
+        };
+        if (t == SGB_F64) reduce(uint64_t(0));
+        else if (t == SGB_U8) reduce(uint8_t(0));
+        else reduce(uint32_t(0));
+    }
+    __syncthreads();
+    // the touched chunks in the current index (as k_lookup), 1024 at a time
+    uint32_t nnew = 0;
+    for (uint32_t t = 0; t * kLkTile < B; ++t) {
+        const uint32_t b = t * kLkTile + tid;
+        bool isnew = false;
+        if (b < B) {
+            const int64_t k = ublk_key[b], lo = lower_bound_i64(keys, nold, k);
+            isnew = !(lo < nold && keys[lo] == k);
+            place[b] = 2 * lo + isnew;
+        }
+        if (tid == 0) ltile[t] = make_uint2(nnew, 0);
+        nnew += (uint32_t)__syncthreads_count(isnew);
+    }
+    if (tid == 0) {
+        counters[0] = U;
+        counters[1] = B;
+        counters[2] = nnew;
+        counters[3] = *err;
+    }
+    if (nnew == 0 && !bad)  // every chunk is there: write the points back now
+        for (uint32_t u = tid; u < U; u += kSmThreads) write_point(upt[u], u, bs_shift, place, out, data, mask, any_listed);
 }
 
 static inline unsigned nblk(int64_t n, int t = 256) { return (unsigned)((n + t - 1) / t); }
@@ -602,9 +842,7 @@ static int flush_impl(sgb_grid* g, const int* ops, int bits, cudaStream_t s) {
     const int64_t n = g->npend;
     const int bs = g->geo.bs;
     const int bs_shift = bs == 512 ? 9 : 6;
-    K* sk = nullptr;
-    uint32_t* sidx = nullptr;
-    SGB_TRY(radix_sort<K>(g, n, bits, &sk, &sidx, s));
+    const bool small = n <= kSmMax;
 
     DevBuf& tiles = g->scratch[7];
     DevBuf& ubuf = g->scratch[9];
@@ -640,12 +878,25 @@ static int flush_impl(sgb_grid* g, const int* ops, int bits, cudaStream_t s) {
         vals.op[p] = upv.op[p] = data.op[p] = ops[p];
         any_listed |= ops[p] != SGB_OP_NONE;
     }
-    k_heads_count<K><<<(unsigned)htiles, kHdThreads, 0, s>>>(sk, n, bs_shift, htile);
-    k_tile_scan<0><<<1, 1024, 0, s>>>(htile, htiles, counters, nullptr);
-    k_fold<K><<<(unsigned)htiles, kHdThreads, 0, s>>>(sk, sidx, n, bs_shift, htile, vals, upv, upt, ublk_key);
-    k_lookup<<<(unsigned)std::min<int64_t>(ltiles, (int64_t)g->num_sms * 8), 256, 0, s>>>(
-        ublk_key, counters, g->keys.as<int64_t>(), g->n, place, ltile);
-    k_tile_scan<1><<<1, 1024, 0, s>>>(ltile, 0, counters, g->err.as<unsigned>());
+    for (int p = 0; p < g->nprop; ++p) data.p[p] = g->data[p].as<unsigned char>();
+    if (small) {
+        const int passes = std::max(1, (bits + 7) / 8), dbits = std::max(1, (bits + passes - 1) / passes);
+        constexpr size_t smem = small_smem<K>();
+        SGB_CUDA(cudaFuncSetAttribute(k_flush_small<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        k_flush_small<K><<<1, kSmThreads, smem, s>>>(g->pend_lin.as<int64_t>(), (int)n, passes, dbits, bs_shift, vals, upv, data,
+                                                     g->mask.as<uint8_t>(), any_listed, g->keys.as<int64_t>(), g->n, upt,
+                                                     ublk_key, place, ltile, counters, g->err.as<unsigned>());
+    } else {
+        K* sk = nullptr;
+        uint32_t* sidx = nullptr;
+        SGB_TRY(radix_sort<K>(g, n, bits, &sk, &sidx, s));
+        k_heads_count<K><<<(unsigned)htiles, kHdThreads, 0, s>>>(sk, n, bs_shift, htile);
+        k_tile_scan<0><<<1, 1024, 0, s>>>(htile, htiles, counters, nullptr);
+        k_fold<K><<<(unsigned)htiles, kHdThreads, 0, s>>>(sk, sidx, n, bs_shift, htile, vals, upv, upt, ublk_key);
+        k_lookup<<<(unsigned)std::min<int64_t>(ltiles, (int64_t)g->num_sms * 2), kLkTile, 0, s>>>(
+            ublk_key, counters, g->keys.as<int64_t>(), g->n, place, ltile);
+        k_tile_scan<1><<<1, 1024, 0, s>>>(ltile, 0, counters, g->err.as<unsigned>());
+    }
     SGB_CUDA(cudaGetLastError());
     SGB_TRY(g->hscratch.ensure(64));
     SGB_CUDA(cudaMemcpyAsync(g->hscratch.p, counters, 16, cudaMemcpyDeviceToHost, s));
@@ -706,6 +957,7 @@ static int flush_impl(sgb_grid* g, const int* ops, int bits, cudaStream_t s) {
         g->cap = cap2;
         g->n = nn_;
     }
+    if (small && NB == 0) return SGB_OK;  // written back already
     for (int p = 0; p < g->nprop; ++p) data.p[p] = g->data[p].as<unsigned char>();
     k_scatter<<<nblk(U), 256, 0, s>>>(upt, U, bs_shift, place, upv, data, g->mask.as<uint8_t>(), any_listed);
     SGB_CUDA(cudaGetLastError());
