@@ -64,6 +64,25 @@ __global__ void k_fill_i32(int32_t* out, int64_t count, int32_t v) {
     if (i < count) out[i] = v;
 }
 
+// Up to four equally long copies in one launch, 16-byte words (chunks are multiples of 16 bytes).
+struct CopySet {
+    const uint4* src[4];
+    uint4* dst[4];
+    int count;
+};
+__global__ void __launch_bounds__(256) k_copy_set(CopySet cs, int64_t words) {
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < words; i += stride) {
+        uint4 v[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (k < cs.count) v[k] = __ldcs(cs.src[k] + i);
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (k < cs.count) cs.dst[k][i] = v[k];
+    }
+}
+
 static int batch_reserve(sgb_batch* b, int64_t chunks) {
     if (chunks <= b->cap) return SGB_OK;
     int64_t nc = std::max<int64_t>(chunks, b->cap + b->cap / 2);
@@ -406,13 +425,20 @@ int sgb_batch_extract(sgb_batch* b, int slot, sgb_grid* g, int* final_is_dst, sg
     int64_t done = 0;
     sgb_batch_slot_steps(b, slot, &done);
     if (final_is_dst) *final_is_dst = (int)(done & 1);
-    // buffer 0 mirrors the src properties, buffer 1 the dst properties
+    // buffer 0 mirrors the src properties, buffer 1 the dst properties; all of them in one launch (a copy call per
+    // property and slot: 48 heat slots with 20 steps before them 5.08 ms, 4.82 ms so)
+    CopySet cs{};
     for (int p = 0; p < b->np; ++p) {
         if (sl.src[p] >= g->nprop || sl.dst[p] >= g->nprop) return SGB_EINVAL;
-        SGB_CUDA(cudaMemcpyAsync(g->data[sl.src[p]].p, b->field[0][p].as<float>() + sl.off * bs, sl.n * bs * 4,
-                                 cudaMemcpyDeviceToDevice, s));
-        SGB_CUDA(cudaMemcpyAsync(g->data[sl.dst[p]].p, b->field[1][p].as<float>() + sl.off * bs, sl.n * bs * 4,
-                                 cudaMemcpyDeviceToDevice, s));
+        for (int k = 0; k < 2; ++k) {
+            cs.src[cs.count] = reinterpret_cast<const uint4*>(b->field[k][p].as<float>() + sl.off * bs);
+            cs.dst[cs.count++] = g->data[k ? sl.dst[p] : sl.src[p]].as<uint4>();
+        }
+    }
+    const int64_t words = sl.n * bs / 4;
+    if (words > 0) {
+        k_copy_set<<<(unsigned)std::min<int64_t>((words + 255) / 256, (int64_t)b->num_sms * 8), 256, 0, s>>>(cs, words);
+        SGB_CUDA(cudaGetLastError());
     }
     return SGB_OK;
 }
