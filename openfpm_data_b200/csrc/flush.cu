@@ -25,25 +25,27 @@
 namespace sgb {
 
 constexpr int kRsWarps = 8;
-constexpr int kRsRounds = 16;
 constexpr int kRsThreads = kRsWarps * 32;
-constexpr int kRsTile = kRsThreads * kRsRounds;  // 4096 keys per CTA
+// Items per thread of a tile, RR: sixteen, or four while such tiles do not outnumber the CTAs that the chip holds:
+// a tile's time is mostly its ranking rounds and latencies (the ghost exchange of 84 K points: 363 us with
+// sixteen, 350 with four).
+constexpr int kRsRounds = 16, kRsRoundsFew = 4;
 
 constexpr int kRsMaxBuckets = 1024;  // digits of up to 10 bits
 
 // Digit counts of every tile, hist[tile][digit].  T: the staged 64-bit linear ids in pass 0, K afterwards.
-template <typename T, typename K>
+template <int RR, typename T, typename K>
 __global__ void __launch_bounds__(kRsThreads) k_rs_hist(const T* __restrict__ keys, int64_t n, int shift, unsigned dmask,
                                                          int nbuckets, uint32_t* __restrict__ hist) {
     __shared__ uint32_t h[kRsMaxBuckets];
     for (int i = threadIdx.x; i < nbuckets; i += kRsThreads) h[i] = 0;
-    const int64_t base = (int64_t)blockIdx.x * kRsTile + threadIdx.x;
-    K k[kRsRounds];  // all loads in flight at once
+    const int64_t base = (int64_t)blockIdx.x * (kRsThreads * RR) + threadIdx.x;
+    K k[RR];  // all loads in flight at once
 #pragma unroll
-    for (int r = 0; r < kRsRounds; ++r) k[r] = base + r * kRsThreads < n ? (K)keys[base + r * kRsThreads] : K(0);
+    for (int r = 0; r < RR; ++r) k[r] = base + r * kRsThreads < n ? (K)keys[base + r * kRsThreads] : K(0);
     __syncthreads();
 #pragma unroll
-    for (int r = 0; r < kRsRounds; ++r)
+    for (int r = 0; r < RR; ++r)
         if (base + r * kRsThreads < n) atomicAdd(&h[(unsigned)(k[r] >> shift) & dmask], 1u);
     __syncthreads();
     for (int d = threadIdx.x; d < nbuckets; d += kRsThreads) hist[(size_t)blockIdx.x * nbuckets + d] = h[d];
@@ -121,37 +123,39 @@ __device__ __forceinline__ unsigned digit_peers(unsigned d, bool valid, unsigned
 // rounds and one uncoalesced offset read per item).  The keys of a tile all go
 // out before the first ranking round, the digits' output positions are read
 // once per digit, coalesced, and 64 registers let four CTAs share an SM.
-template <typename K>
+template <int RR, typename K>
 __host__ __device__ constexpr size_t rs_union_bytes() {
+    constexpr int kRsTile = kRsThreads * RR;
     return (size_t)kRsWarps * kRsMaxBuckets * 4 > (size_t)kRsTile * (sizeof(K) + 4)
                ? (size_t)kRsWarps * kRsMaxBuckets * 4
                : (size_t)kRsTile * (sizeof(K) + 4);
 }
-template <typename K>
+template <int RR, typename K>
 __host__ __device__ constexpr size_t rs_scatter_smem() {
-    return rs_union_bytes<K>() + (size_t)kRsMaxBuckets * 8 + 2 * kRsWarps * 4;
+    return rs_union_bytes<RR, K>() + (size_t)kRsMaxBuckets * 8 + 2 * kRsWarps * 4;
 }
 
-template <typename T, typename K>
+template <int RR, typename T, typename K>
 __global__ void __launch_bounds__(kRsThreads, sizeof(K) == 4 ? 4 : 2) k_rs_scatter(const T* __restrict__ kin, const uint32_t* __restrict__ vin,
                                                             K* __restrict__ kout, uint32_t* __restrict__ vout, int64_t n,
                                                             int shift, unsigned dmask, int nbuckets,
                                                             const uint32_t* __restrict__ offs,
                                                             const uint32_t* __restrict__ tot_g) {
+    constexpr int kRsTile = kRsThreads * RR;
     extern __shared__ __align__(16) unsigned char rs_smem[];
     auto wcnt = reinterpret_cast<uint32_t(*)[kRsMaxBuckets]>(rs_smem);  // [kRsWarps][kRsMaxBuckets]
     K* sk = reinterpret_cast<K*>(rs_smem);                              // the same bytes, once wcnt is done
     uint32_t* sv = reinterpret_cast<uint32_t*>(rs_smem + (size_t)kRsTile * sizeof(K));
-    uint32_t* dstart = reinterpret_cast<uint32_t*>(rs_smem + rs_union_bytes<K>());  // digit's first place in the tile
+    uint32_t* dstart = reinterpret_cast<uint32_t*>(rs_smem + rs_union_bytes<RR, K>());  // digit's first place in the tile
     uint32_t* gdst = dstart + kRsMaxBuckets;  // output position of the digit's items minus dstart
     uint32_t* wsum = gdst + kRsMaxBuckets;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t tbase = (int64_t)blockIdx.x * kRsTile;
-    const int64_t base = tbase + warp * (32 * kRsRounds) + lane;
-    K key[kRsRounds];
-    uint32_t rank[kRsRounds];
+    const int64_t base = tbase + warp * (32 * RR) + lane;
+    K key[RR];
+    uint32_t rank[RR];
 #pragma unroll
-    for (int r = 0; r < kRsRounds; ++r) {
+    for (int r = 0; r < RR; ++r) {
         const int64_t i = base + r * 32;
         key[r] = i < n ? (K)kin[i] : K(0);
     }
@@ -160,7 +164,7 @@ __global__ void __launch_bounds__(kRsThreads, sizeof(K) == 4 ? 4 : 2) k_rs_scatt
     __syncthreads();
     const unsigned lt = lanemask_lt();
 #pragma unroll
-    for (int r = 0; r < kRsRounds; ++r) {
+    for (int r = 0; r < RR; ++r) {
         const bool valid = base + r * 32 < n;
         const unsigned d = (unsigned)(key[r] >> shift) & dmask;
         const unsigned peers = digit_peers(d, valid, dmask);
@@ -172,9 +176,9 @@ __global__ void __launch_bounds__(kRsThreads, sizeof(K) == 4 ? 4 : 2) k_rs_scatt
         __syncwarp();
     }
     __syncthreads();
-    uint32_t val[kRsRounds];  // needed from here on
+    uint32_t val[RR];  // needed from here on
 #pragma unroll
-    for (int r = 0; r < kRsRounds; ++r) {
+    for (int r = 0; r < RR; ++r) {
         const int64_t i = base + r * 32;
         val[r] = i < n ? (vin ? vin[i] : (uint32_t)i) : 0u;
     }
@@ -211,7 +215,7 @@ __global__ void __launch_bounds__(kRsThreads, sizeof(K) == 4 ? 4 : 2) k_rs_scatt
     }
     __syncthreads();
 #pragma unroll
-    for (int r = 0; r < kRsRounds; ++r) {
+    for (int r = 0; r < RR; ++r) {
         if (base + r * 32 < n) {
             const unsigned d = (unsigned)(key[r] >> shift) & dmask;
             rank[r] += dstart[d] + wcnt[warp][d];  // position in the tile, digit order
@@ -219,7 +223,7 @@ __global__ void __launch_bounds__(kRsThreads, sizeof(K) == 4 ? 4 : 2) k_rs_scatt
     }
     __syncthreads();  // wcnt is read no more: its bytes take the staged tile
 #pragma unroll
-    for (int r = 0; r < kRsRounds; ++r) {
+    for (int r = 0; r < RR; ++r) {
         if (base + r * 32 < n) {
             sk[rank[r]] = key[r];
             sv[rank[r]] = val[r];
@@ -303,9 +307,9 @@ __device__ __noinline__ uint64_t fold_rest16(int type, int op, uint64_t acc, con
     return acc;
 }
 
-// Segment heads of the sorted ids: the first item of every point and of every chunk.  A tile of 2048 items
-// is eight rounds of a 256-thread CTA in index order.
-constexpr int kHdThreads = 256, kHdRounds = 8, kHdTile = kHdThreads * kHdRounds;
+// Segment heads of the sorted ids: the first item of every point and of every chunk.  A tile of 1024 items
+// is four rounds of a 256-thread CTA in index order (eight rounds: 8 us more per 2 M points, fewer CTAs in flight).
+constexpr int kHdThreads = 256, kHdRounds = 4, kHdTile = kHdThreads * kHdRounds;
 
 template <typename K>
 __device__ __forceinline__ void heads_of(const K* __restrict__ sk, int64_t n, int64_t i, int bs_shift, K& k, bool& pt,
@@ -399,7 +403,7 @@ __global__ void __launch_bounds__(1024) k_tile_scan(uint2* cnt, int64_t ntiles, 
 // Per point: fold its inserts in insertion order (the sort is stable).  The point's chunk (its rank among the
 // touched chunks) and offset go to upt, the reduced values to vals_out, the touched chunks' ids to ublk_key.
 template <typename K>
-__global__ void __launch_bounds__(kHdThreads, 3) k_fold(const K* __restrict__ sk, const uint32_t* __restrict__ sidx, int64_t n,
+__global__ void __launch_bounds__(kHdThreads, 4) k_fold(const K* __restrict__ sk, const uint32_t* __restrict__ sidx, int64_t n,
                                                       int bs_shift, const uint2* __restrict__ tile_off, PropSet vals,
                                                       PropSet out, uint2* __restrict__ upt, int64_t* __restrict__ ublk_key) {
     constexpr int W = kHdThreads / 32;
@@ -417,16 +421,16 @@ __global__ void __launch_bounds__(kHdThreads, 3) k_fold(const K* __restrict__ sk
         if (lane == 0) pre[r * W + warp] = __popc(pb[r]) | __popc(bb[r]) << 16;
     }
     __syncthreads();
-    if (warp == 0) {  // 64 entries, two per lane
-        const uint32_t a = pre[2 * lane], b = pre[2 * lane + 1];
-        uint32_t incl = a + b;
+    static_assert(kHdRounds * W == 32, "one entry per lane");
+    if (warp == 0) {
+        const uint32_t a = pre[lane];
+        uint32_t incl = a;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
             if (lane >= o) incl += v;
         }
-        pre[2 * lane] = incl - a - b;
-        pre[2 * lane + 1] = incl - b;
+        pre[lane] = incl - a;
     }
     __syncthreads();
     const uint2 off = tile_off[blockIdx.x];
@@ -634,10 +638,11 @@ __global__ void __launch_bounds__(kSmThreads) k_flush_small(const int64_t* __res
     if (tid == 0) bad = *err & (kErrOutOfDomain | kErrPoolOverflow);
     K key[kSmItems];
     uint32_t idx[kSmItems], rank[kSmItems];
-    const int base = warp * 32 * kSmItems + lane;  // items in (warp, round, lane) order
+    const int rounds = (n + kSmThreads - 1) / kSmThreads;  // the same for every warp
+    const int base = warp * 32 * rounds + lane;  // items in (warp, round, lane) order
 #pragma unroll
     for (int r = 0; r < kSmItems; ++r) {
-        const int i = base + 32 * r;
+        const int i = r < rounds ? base + 32 * r : n;
         key[r] = i < n ? (K)lin[i] : K(0);
         idx[r] = (uint32_t)i;
     }
@@ -647,6 +652,7 @@ __global__ void __launch_bounds__(kSmThreads) k_flush_small(const int64_t* __res
         __syncthreads();
 #pragma unroll
         for (int r = 0; r < kSmItems; ++r) {
+            if (r >= rounds) break;  // uniform
             const bool valid = base + 32 * r < n;
             const unsigned d = (unsigned)(key[r] >> shift) & dmask;
             const unsigned peers = digit_peers(d, valid, dmask);
@@ -694,7 +700,7 @@ __global__ void __launch_bounds__(kSmThreads) k_flush_small(const int64_t* __res
         __syncthreads();
 #pragma unroll
         for (int r = 0; r < kSmItems; ++r)
-            if (base + 32 * r < n) {
+            if (r < rounds && base + 32 * r < n) {
                 const unsigned d = (unsigned)(key[r] >> shift) & dmask;
                 const uint32_t pos = dstart[d] + wcnt[warp][d] + rank[r];
                 sk[pos] = key[r];
@@ -704,7 +710,7 @@ __global__ void __launch_bounds__(kSmThreads) k_flush_small(const int64_t* __res
         if (ps + 1 < passes)
 #pragma unroll
             for (int r = 0; r < kSmItems; ++r)
-                if (base + 32 * r < n) {
+                if (r < rounds && base + 32 * r < n) {
                     key[r] = sk[base + 32 * r];
                     idx[r] = si[base + 32 * r];
                 }
@@ -791,20 +797,20 @@ __global__ void __launch_bounds__(kSmThreads) k_flush_small(const int64_t* __res
 
 static inline unsigned nblk(int64_t n, int t = 256) { return (unsigned)((n + t - 1) / t); }
 
-template <typename T, typename K>
+template <int RR, typename T, typename K>
 static int radix_pass(const T* kin, const uint32_t* vin, K* kout, uint32_t* vout, int64_t n, int shift, unsigned dmask,
                       int nbuckets, uint32_t* hist, uint32_t* tot, int ntiles, cudaStream_t s) {
-    k_rs_hist<T, K><<<ntiles, kRsThreads, 0, s>>>(kin, n, shift, dmask, nbuckets, hist);
+    k_rs_hist<RR, T, K><<<ntiles, kRsThreads, 0, s>>>(kin, n, shift, dmask, nbuckets, hist);
     k_rs_rowscan<<<(nbuckets + 31) / 32, 1024, 0, s>>>(hist, ntiles, nbuckets, tot);
-    constexpr size_t smem = rs_scatter_smem<K>();
+    constexpr size_t smem = rs_scatter_smem<RR, K>();
     if (smem > 48 * 1024)
-        SGB_CUDA(cudaFuncSetAttribute(k_rs_scatter<T, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_rs_scatter<T, K><<<ntiles, kRsThreads, smem, s>>>(kin, vin, kout, vout, n, shift, dmask, nbuckets, hist, tot);
+        SGB_CUDA(cudaFuncSetAttribute(k_rs_scatter<RR, T, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    k_rs_scatter<RR, T, K><<<ntiles, kRsThreads, smem, s>>>(kin, vin, kout, vout, n, shift, dmask, nbuckets, hist, tot);
     SGB_CUDA(cudaGetLastError());
     return SGB_OK;
 }
 
-template <typename K>
+template <int RR, typename K>
 static int radix_sort(sgb_grid* g, int64_t n, int bits, K** keys_out, uint32_t** vals_out, cudaStream_t s) {
     DevBuf& kA = g->scratch[0];
     DevBuf& kB = g->scratch[1];
@@ -815,7 +821,7 @@ static int radix_sort(sgb_grid* g, int64_t n, int bits, K** keys_out, uint32_t**
     SGB_TRY(kB.ensure((size_t)n * sizeof(K)));
     SGB_TRY(vA.ensure((size_t)n * 4));
     SGB_TRY(vB.ensure((size_t)n * 4));
-    const int ntiles = (int)((n + kRsTile - 1) / kRsTile);
+    const int ntiles = (int)((n + kRsThreads * RR - 1) / (kRsThreads * RR));
     // as few passes as digits of at most 10 bits allow, the digit width spread evenly over them
     const int passes = bits <= 0 ? 1 : (bits + 9) / 10;
     const int dbits = bits <= 0 ? 1 : (bits + passes - 1) / passes;
@@ -827,10 +833,10 @@ static int radix_sort(sgb_grid* g, int64_t n, int bits, K** keys_out, uint32_t**
     K* kbuf[2] = {kA.as<K>(), kB.as<K>()};
     uint32_t* vbuf[2] = {vA.as<uint32_t>(), vB.as<uint32_t>()};
     // pass 0 takes the staged ids as they are and ranks the insertion index itself
-    SGB_TRY((radix_pass<int64_t, K>(g->pend_lin.as<int64_t>(), nullptr, kbuf[0], vbuf[0], n, 0, dmask, nbuckets, h, tot,
+    SGB_TRY((radix_pass<RR, int64_t, K>(g->pend_lin.as<int64_t>(), nullptr, kbuf[0], vbuf[0], n, 0, dmask, nbuckets, h, tot,
                                     ntiles, s)));
     for (int ps = 1; ps < passes; ++ps)
-        SGB_TRY((radix_pass<K, K>(kbuf[(ps + 1) & 1], vbuf[(ps + 1) & 1], kbuf[ps & 1], vbuf[ps & 1], n, ps * dbits, dmask,
+        SGB_TRY((radix_pass<RR, K, K>(kbuf[(ps + 1) & 1], vbuf[(ps + 1) & 1], kbuf[ps & 1], vbuf[ps & 1], n, ps * dbits, dmask,
                                   nbuckets, h, tot, ntiles, s)));
     *vals_out = vbuf[(passes + 1) & 1];
     *keys_out = kbuf[(passes + 1) & 1];
@@ -889,7 +895,10 @@ static int flush_impl(sgb_grid* g, const int* ops, int bits, cudaStream_t s) {
     } else {
         K* sk = nullptr;
         uint32_t* sidx = nullptr;
-        SGB_TRY(radix_sort<K>(g, n, bits, &sk, &sidx, s));
+        if (n <= (int64_t)g->num_sms * 4 * kRsThreads * kRsRoundsFew)
+            SGB_TRY((radix_sort<kRsRoundsFew, K>(g, n, bits, &sk, &sidx, s)));
+        else
+            SGB_TRY((radix_sort<kRsRounds, K>(g, n, bits, &sk, &sidx, s)));
         k_heads_count<K><<<(unsigned)htiles, kHdThreads, 0, s>>>(sk, n, bs_shift, htile);
         k_tile_scan<0><<<1, 1024, 0, s>>>(htile, htiles, counters, nullptr);
         k_fold<K><<<(unsigned)htiles, kHdThreads, 0, s>>>(sk, sidx, n, bs_shift, htile, vals, upv, upt, ublk_key);
