@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1)
 #pragma unroll
             for (int z = 0; z < 4; ++z)
                 if (mz[z])
-                    star_store<KIND, NP>(cv[z], lap[z], mz[z], active_bits<false>(mz[z], StencilParams{}, 0, 0, 0), gi, bd,
+                    star_store<KIND, NP>(cv[z], lap[z], mz[z], active_bits<false>(mz[z], 0, 0, 0, 0), gi, bd,
                                          D + z * 64, D + (NP - 1) * fstride + z * 64);
         }
         cluster_barrier();  // also: no CTA leaves while another may still read its tiles

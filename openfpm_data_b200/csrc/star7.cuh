@@ -156,16 +156,16 @@ __device__ __forceinline__ void star_store(const float4 (&c)[NP], const Quad (&l
 }
 
 // Bits of the quad's active points: EXIST and not PADDING, inside the box.
-template <bool BOX>
-__device__ __forceinline__ uint32_t active_bits(uint32_t m4, const StencilParams& prm, int x, int y, int z) {
+template <bool BOX, typename Args>
+__device__ __forceinline__ uint32_t active_bits(uint32_t m4, const Args& box, int x, int y, int z) {
     // per byte: bit 0 set and bit 1 clear
     if (!BOX && m4 == 0x01010101u) return 0xfu;
     uint32_t a = m4 & ~(m4 >> 1) & 0x01010101u;
     a = (a | a >> 7 | a >> 14 | a >> 21) & 0xfu;
-    if (BOX) {
+    if constexpr (BOX) {
 #pragma unroll
         for (int k = 0; k < 4; ++k)
-            if (!in_box(prm, x + k, y, z)) a &= ~(1u << k);
+            if (!in_box(box.prm, x + k, y, z)) a &= ~(1u << k);
     }
     return a;
 }

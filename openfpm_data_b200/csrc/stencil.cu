@@ -507,12 +507,14 @@ int sgb_run_steps(sgb_grid* g, int kind, const int* src, const int* dst, const f
     }
     // One launch per step, whether or not the caller asked for a graph: capturing and instantiating a graph for
     // every call took 5-10 us per step on the host before the first step ran (31 heat steps of 6.2 us: 524 us),
-    // a launch takes about 2 us beside the step before it.  use_graph also asks for the wait at the end.
+    // a launch takes about 2 us beside the step before it.  use_graph also asks for the wait at the end, which
+    // 7-point solves of at most 4 chunks per SM do without, so that their next call's launches overlap.
     for (int k = 0; k < nsteps; ++k) {
         if (k % 2 == 0) SGB_TRY(launch_stencil(g, kind, src, dst, fwd, s, k > 0));
         else SGB_TRY(launch_stencil(g, kind, dst, src, bwd, s, k > 0));
     }
-    if (use_graph) SGB_CUDA(cudaStreamSynchronize(s));
+    const bool small = (kind == SGB_HEAT7 || kind == SGB_GS7) && g->n <= (int64_t)g->num_sms * 4 && nsteps >= 2;
+    if (use_graph && !small) SGB_CUDA(cudaStreamSynchronize(s));
     return SGB_OK;
 }
 
