@@ -224,7 +224,9 @@ int sgb_apply_stencil(sgb_grid* g, int kind, const int* src, const int* dst, con
  * reference's ping-pong loop, src/SparseGridGpu/tests/
  * SparseGridGpu_tests.cu:499-503): one launch per step, each overlapping the
  * tail of the one before, or one launch for all steps of a small grid.
- * use_graph != 0: the call waits for a grid of one launch per step.  On return *final_is_dst is 1 when the last step wrote the dst properties. */
+ * use_graph != 0: the call waits for the steps, except for 7-point solves of
+ * at most 4 chunks per SM, which return without waiting.  On return
+ * *final_is_dst is 1 when the last step wrote the dst properties. */
 int sgb_run_steps(sgb_grid* g, int kind, const int* src, const int* dst, const float* params, int nparams,
                   int nsteps, int use_graph, int* final_is_dst, sgb_stream s);
 
@@ -324,6 +326,10 @@ int sgb_calc_existing_points(sgb_grid* g, int64_t* count, sgb_stream s);
 
 /* The same list's device array (valid until existence changes) and length. */
 int sgb_existing_point_list(sgb_grid* g, const uint32_t** ids_dev, int64_t* count, sgb_stream s);
+
+/* The same list as 64-bit ids in the caller's memory: ids_dev [capacity] is
+ * written when capacity >= *count, so a first call with capacity 0 sizes it. */
+int sgb_existing_point_ids(sgb_grid* g, int64_t* ids_dev, int64_t capacity, int64_t* count, sgb_stream s);
 
 /* Links between the levels of a multi-resolution hierarchy
  * (construct_link_dw / construct_link_up, SparseGridGpu.hpp:2113-2262;

@@ -43,6 +43,7 @@ SIGNATURES = {
     "sgb_existing_points": (_i32, [_vp, _vp, _vp, _i64, _vp, _vp]),
     "sgb_calc_existing_points": (_i32, [_vp, _vp, _vp]),
     "sgb_existing_point_list": (_i32, [_vp, _vp, _vp, _vp]),
+    "sgb_existing_point_ids": (_i32, [_vp, _vp, _i64, _vp, _vp]),
     "sgb_set_linearizer": (_i32, [_vp, _i32]),
     "sgb_release_scratch": (_i32, [_vp]),
     "sgb_existence_changed": (_i32, [_vp]),

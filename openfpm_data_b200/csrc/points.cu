@@ -174,6 +174,20 @@ __global__ void __launch_bounds__(256) k_box27_points(const float* __restrict__ 
     dst[id] = tot;
 }
 
+// The list as 64-bit ids, four per thread: one pass (a conversion and a mask over it took 31 us for 6.7 M points,
+// 14 us so; 81 MB moved).
+__global__ void __launch_bounds__(256) k_ep_widen(const uint32_t* __restrict__ in, int64_t n, int64_t* __restrict__ out,
+                                                   int vec) {
+    const int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) * 4;
+    if (vec && i + 4 <= n) {
+        const uint4 v = *reinterpret_cast<const uint4*>(in + i);
+        reinterpret_cast<longlong2*>(out + i)[0] = make_longlong2(v.x, v.y);
+        reinterpret_cast<longlong2*>(out + i)[1] = make_longlong2(v.z, v.w);
+    } else {
+        for (int k = 0; k < 4 && i + k < n; ++k) out[i + k] = (int64_t)in[i + k];
+    }
+}
+
 static int launch_points(sgb_grid* g, const int* src, const int* dst, const StencilParams& prm, bool xouter,
                          cudaStream_t s) {
     if (g->n == 0) return SGB_OK;
@@ -232,5 +246,18 @@ extern "C" int sgb_existing_point_list(sgb_grid* g, const uint32_t** ids_dev, in
     SGB_TRY(ensure_point_list(g, (cudaStream_t)stream));
     *ids_dev = g->epts.as<uint32_t>();
     *count = g->nepts;
+    return SGB_OK;
+}
+
+extern "C" int sgb_existing_point_ids(sgb_grid* g, int64_t* ids_dev, int64_t capacity, int64_t* count, sgb_stream stream) {
+    if (!g || !count || capacity < 0 || (capacity > 0 && !ids_dev)) return SGB_EINVAL;
+    cudaStream_t s = (cudaStream_t)stream;
+    SGB_TRY(ensure_point_list(g, s));
+    *count = g->nepts;
+    if (g->nepts == 0 || capacity < g->nepts) return SGB_OK;  // the caller sizes the buffer from *count
+    const int64_t threads = (g->nepts + 3) / 4;
+    k_ep_widen<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(g->epts.as<uint32_t>(), g->nepts, ids_dev,
+                                                                 (uintptr_t)ids_dev % 16 == 0);
+    SGB_CUDA(cudaGetLastError());
     return SGB_OK;
 }

@@ -44,8 +44,19 @@ def _stream(stream=None) -> int:
     return stream.cuda_stream if hasattr(stream, "cuda_stream") else int(stream)
 
 
+# array types by length (looking them up costs a third of making them per call)
+_I32 = [C.c_int * k for k in range(33)]
+_F32 = [C.c_float * k for k in range(33)]
+
+
 def _i32arr(vals):
-    return (C.c_int * len(vals))(*vals)
+    n = len(vals)
+    return (_I32[n] if n < 33 else C.c_int * n)(*vals)
+
+
+def _f32arr(vals):
+    n = len(vals)
+    return (_F32[n] if n < 33 else C.c_float * n)(*vals)
 
 
 class _DevView:
@@ -200,13 +211,14 @@ class SparseGridGpu:
 
     def existing_point_list(self, stream=None) -> torch.Tensor:
         """The e_points list: int64 copy of the uint32 ids chunk position * bs + offset."""
-        p, cnt = C.c_void_p(), C.c_int64()
-        L.check(self._lib.sgb_existing_point_list(self._h, C.byref(p), C.byref(cnt), _stream(stream)),
-                "sgb_existing_point_list")
-        if cnt.value == 0:
-            return torch.empty(0, dtype=torch.int64, device=f"cuda:{self.device}")
-        v = torch.as_tensor(_DevView(p.value, (cnt.value,), "<i4"), device=f"cuda:{self.device}")
-        return v.to(torch.int64) & 0xFFFFFFFF
+        cnt = C.c_int64()
+        fn = self._lib.sgb_existing_point_ids
+        L.check(fn(self._h, None, 0, C.byref(cnt), _stream(stream)), "sgb_existing_point_ids")
+        out = torch.empty(cnt.value, dtype=torch.int64, device=f"cuda:{self.device}")
+        if cnt.value:
+            # on torch's current stream, the one its users read it on
+            L.check(fn(self._h, out.data_ptr(), cnt.value, C.byref(cnt), _stream()), "sgb_existing_point_ids")
+        return out
 
     # ---------------------------------------------------------------- stencils
     @staticmethod
@@ -218,14 +230,14 @@ class SparseGridGpu:
 
     def applyStencils(self, kind: int, src: Sequence[int], dst: Sequence[int], params: Sequence[float],
                       box=None, stream=None, tiled: bool = False) -> None:
-        prm = (C.c_float * len(params))(*params)
+        prm = _f32arr(params)
         fn = self._lib.sgb_apply_stencil_tiled if tiled else self._lib.sgb_apply_stencil
         L.check(fn(self._h, kind, _i32arr(src), _i32arr(dst), prm, len(params), self._box(box), _stream(stream)),
                 "sgb_apply_stencil")
 
     def run_steps(self, kind: int, src, dst, params, nsteps: int, use_graph: bool = True, stream=None) -> bool:
         """nsteps ping-pong applications; returns True when the result is in dst."""
-        prm = (C.c_float * len(params))(*params)
+        prm = _f32arr(params)
         fin = C.c_int(0)
         L.check(self._lib.sgb_run_steps(self._h, kind, _i32arr(src), _i32arr(dst), prm, len(params), nsteps,
                                         int(use_graph), C.byref(fin), _stream(stream)), "sgb_run_steps")
@@ -567,7 +579,7 @@ class Batch:
         L.check(self._lib.sgb_batch_set_launch_config(self._h, ctas_per_sm, stages), "sgb_batch_set_launch_config")
 
     def add(self, g: SparseGridGpu, kind: int, src, dst, params, nsteps: int, stream=None) -> int:
-        prm = (C.c_float * len(params))(*params)
+        prm = _f32arr(params)
         slot = C.c_int(-1)
         L.check(self._lib.sgb_batch_add(self._h, g.handle, kind, _i32arr(src), _i32arr(dst), prm, len(params),
                                         int(nsteps), C.byref(slot), _stream(stream)), "sgb_batch_add")
