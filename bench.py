@@ -467,7 +467,7 @@ def run_heat128(args, dist: Dist):
     te = dist.max(e0.elapsed_time(e1) / 1e3)
     e2e = {"value": round(dist.world * npts * 100 * nsolve / te / 1e9, 3), "unit": "Gpts/s",
            "h2d_bytes_per_step": int(hk.nbytes + hu.nbytes + hm.nbytes), "d2h_bytes_per_step": int(out.numel() * 4),
-           "step": "one solve: upload, 100 heat steps (sgb_run_steps: one cooperative launch on this small grid), download"}
+           "step": "one solve: upload, 100 heat steps (sgb_run_steps), download"}
     cpu = None
     if dist.rank == 0 and dist.world == 1 and not args.no_cpu_baseline:
         from oracle import oracle as O
@@ -656,7 +656,7 @@ def run_batched256(args, dist: Dist):
     p1.record()
     torch.cuda.synchronize()
     tp = dist.max(p0.elapsed_time(p1) / 1e3)
-    # per-grid sgb_run_steps (grids of at most 4 chunks per SM run all steps in one cooperative launch)
+    # per-grid sgb_run_steps (small grids run all steps in one launch)
     q0, q1 = _events()
     q0.record()
     for g in grids:
