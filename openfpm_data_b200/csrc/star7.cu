@@ -239,17 +239,22 @@ __global__ void __launch_bounds__(kStarThreads, MINB)
     }
     const int l16 = threadIdx.x & 15, y = l16 & 3, z = l16 >> 2;
     const int64_t c = (int64_t)blockIdx.x * kStarGroups + (threadIdx.x >> 4);
-    if (c >= n) return;
+    bool live = c < n;
     GridInfo gb;
     int par = 0;
-    if (BATCH) {
+    if (BATCH && live) {
         gb = grids[gid[c]];
-        if (!(t >= gb.start && t < gb.start + gb.nsteps)) return;
+        live = t >= gb.start && t < gb.start + gb.nsteps;
         par = (int)((t - gb.start) & 1);
     }
     const GridInfo& gi = BATCH ? gb : g0;
-    const uint32_t m = __ldg(reinterpret_cast<const uint32_t*>(mask + c * 64 + l16 * 4));
-    if (!m && !(KIND == SGB_HEAT7 && fill)) return;  // the row holds no point
+    const uint32_t m = live ? __ldg(reinterpret_cast<const uint32_t*>(mask + c * 64 + l16 * 4)) : 0u;
+    if (!m && !(KIND == SGB_HEAT7 && fill && live)) {
+        // The row holds no point.  No thread leaves without the wait: a launch of idle rows only would be over
+        // before the step ahead of it, and what follows in the stream waits for this launch alone.
+        grid_dependency_wait();
+        return;
+    }
     const int4 na = __ldg(reinterpret_cast<const int4*>(nn + c * 8));
     const int2 nz = __ldg(reinterpret_cast<const int2*>(nn + c * 8 + 4));
     const int64_t oc = c * 64 + l16 * 4;

@@ -93,3 +93,30 @@ def test_solve_in_one_launch_equals_steps(sgb, kind, nchunks):
         for q in a + b:  # the last state and the one before it
             x, w = g.private_get_data_array(q)[ex], h.private_get_data_array(q)[ex]
             assert torch.equal(x.view(torch.int32), w.view(torch.int32))
+
+
+@pytest.mark.parametrize("use_graph", [True, False])
+@pytest.mark.parametrize("kind", ["HEAT7", "GS7"])
+def test_batch_stepped_past_its_slots(sgb, kind, use_graph):
+    """4^3 chunks: most launches of the call find no slot with a step left; what is read behind them is the last
+    live step's result, of a step long enough for the idle launches to overtake it."""
+    prm = [0.1] if kind == "HEAT7" else [0.16, 0.08, 0.035, 0.065, 1.0]
+    a, b = ([0], [2]) if kind == "HEAT7" else ([0, 1], [2, 3])
+    batch = sgb.Batch()
+    slots, want = [], []
+    for nchunks, nsteps in ((40000, 4), (500, 3)):
+        size = (240, 240, 240) if nchunks > 1000 else (64, 60, 52)
+        g, h = (_grid(sgb, size, nchunks, "smb", 5, density=0.9, e=4) for _ in range(2))
+        slots.append((batch.add(g, getattr(sgb, kind), a, b, prm, nsteps), g))
+        for k in range(nsteps):
+            h.applyStencils(getattr(sgb, kind), a if k % 2 == 0 else b, b if k % 2 == 0 else a, prm, tiled=True)
+        want.append(h)
+    for _ in range(2):  # the second call has idle launches only
+        batch.step(24, use_graph=use_graph)
+        for (slot, g), h in zip(slots, want):
+            batch.extract(slot, g)
+            ex = (h.private_get_mask_array() & 1).bool()
+            for q in a + b:
+                x, w = g.private_get_data_array(q)[ex], h.private_get_data_array(q)[ex]
+                assert torch.equal(x.view(torch.int32), w.view(torch.int32))
+    batch.close()
