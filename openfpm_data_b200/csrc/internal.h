@@ -37,6 +37,16 @@ int cuda_status(cudaError_t e, const char* what);
         if (s_ != SGB_OK) return s_;  \
     } while (0)
 
+// Dynamic shared memory of a launch, at most.  A kernel's limit belongs to the device and not to the call: host
+// threads that launch one kernel with different sizes all set this same value, so that none of them lowers the limit
+// between another's setting and its launch.
+constexpr int kMaxDynamicSmem = 227 * 1024;
+template <typename Kernel>
+inline int allow_max_smem(Kernel kern) {
+    SGB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem));
+    return SGB_OK;
+}
+
 // Makes `dev` the current device for the lifetime of the guard and gives the
 // caller's current device back on every return path, so an entry point that
 // works on a grid of another GPU leaves the caller's CUDA state as it was.

@@ -175,8 +175,8 @@ static int launch_solve(const FieldSet& fs, const uint8_t* mask, const int32_t* 
     while (ctas < kSolveCtas && ctas < n) ctas *= 2;
     const int cap = (n + ctas - 1) / ctas;
     const size_t smem = solve_smem<NP>(cap);
-    if (smem > 227 * 1024) return SGB_ENOTSUP;
-    SGB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > kMaxDynamicSmem) return SGB_ENOTSUP;
+    SGB_TRY(allow_max_smem(kern));
     SGB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)ctas);

@@ -321,8 +321,8 @@ static int launch_star(const LaunchDesc& L, cudaStream_t s) {
     const int64_t items = L.n * (8 / ZS);
     size_t smem = sizeof(StarTile<NP, ZS>) * kStarGroups;
     // a caller's limit on the CTAs per SM: each CTA takes its share of the SM's shared memory
-    if (L.ctas_per_sm > 0) smem = std::max(smem, (size_t)(227 * 1024 / L.ctas_per_sm - 1024) & ~(size_t)127);
-    if (smem > 48 * 1024) SGB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (L.ctas_per_sm > 0) smem = std::max(smem, (size_t)(kMaxDynamicSmem / L.ctas_per_sm - 1024) & ~(size_t)127);
+    if (smem > 48 * 1024) SGB_TRY(allow_max_smem(kern));
     StarLaunch l(items, smem, s);
     const int ahead = L.num_sms * 7 * kStarGroups;  // about the groups resident at a time
     SGB_CUDA(cudaLaunchKernelEx(&l.cfg, kern, L.fs, L.mask, L.nn, box_args<BOX>(L), L.gid, L.grids, L.g0, L.n, L.t,

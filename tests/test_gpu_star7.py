@@ -120,3 +120,51 @@ def test_batch_stepped_past_its_slots(sgb, kind, use_graph):
                 x, w = g.private_get_data_array(q)[ex], h.private_get_data_array(q)[ex]
                 assert torch.equal(x.view(torch.int32), w.view(torch.int32))
     batch.close()
+
+
+@pytest.mark.parametrize("what", ["solve", "step"])
+def test_threads_with_different_shared_memory(sgb, what):
+    """Host threads, each with its own grid and stream, launch one kernel with different amounts of shared memory:
+    none may lower another's limit between its setting and its launch."""
+    import threading
+    # chunks, CTAs per SM, steps a call: small grids run in one cluster launch, larger ones by a launch per step
+    plans = [(256, -1, 2), (20, -1, 2), (120, -1, 2), (3, -1, 2)] if what == "solve" else [(400, 1, 50), (400, 3, 50)]
+    calls = 2000 if what == "solve" else 100
+    want, got, bad = {}, {}, []
+    together = threading.Barrier(len(plans), timeout=120)
+
+    def grid(n):
+        return _grid(sgb, (75, 80, 70), n, "smb", n, density=0.9)
+
+    for n, _, steps in plans:
+        g = grid(n)
+        for k in range(steps):
+            g.applyStencils(sgb.HEAT7, [2 * (k % 2)], [2 - 2 * (k % 2)], [0.1], tiled=True)
+        want[n] = g.deviceToHost()[1][0]
+
+    def work(k):
+        try:
+            n, ctas, steps = plans[k]
+            stream = torch.cuda.Stream()
+            g = grid(n)
+            g.setLaunchConfig(ctas, -1)
+            first = g.deviceToHost()[1][0]
+            together.wait()
+            for _ in range(calls):
+                g.run_steps(sgb.HEAT7, [0], [2], [0.1], steps, use_graph=False, stream=stream)
+            stream.synchronize()
+            g.private_get_data_array(0).copy_(torch.from_numpy(first))
+            torch.cuda.synchronize()
+            g.run_steps(sgb.HEAT7, [0], [2], [0.1], steps, use_graph=False, stream=stream)
+            got[k] = g.deviceToHost(stream)[1][0]
+        except Exception as e:  # noqa: BLE001
+            bad.append(e)
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(len(plans))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad, bad
+    for k, (n, _, _) in enumerate(plans):
+        assert np.array_equal(want[n].view(np.uint32), got[k].view(np.uint32))
