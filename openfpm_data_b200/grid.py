@@ -210,14 +210,23 @@ class SparseGridGpu:
         return cnt.value
 
     def existing_point_list(self, stream=None) -> torch.Tensor:
-        """The e_points list: int64 copy of the uint32 ids chunk position * bs + offset."""
+        """The e_points list: int64 copy of the uint32 ids chunk position * bs + offset, built
+        and copied on `stream` and ready on torch's current stream."""
         cnt = C.c_int64()
         fn = self._lib.sgb_existing_point_ids
-        L.check(fn(self._h, None, 0, C.byref(cnt), _stream(stream)), "sgb_existing_point_ids")
+        built = _stream(stream)
+        L.check(fn(self._h, None, 0, C.byref(cnt), built), "sgb_existing_point_ids")
         out = torch.empty(cnt.value, dtype=torch.int64, device=f"cuda:{self.device}")
         if cnt.value:
-            # on torch's current stream, the one its users read it on
-            L.check(fn(self._h, out.data_ptr(), cnt.value, C.byref(cnt), _stream()), "sgb_existing_point_ids")
+            # `out` is memory of torch's current stream; the copy runs behind the list's last kernel, which the call
+            # above leaves queued
+            here = torch.cuda.current_stream()
+            other = None if built == here.cuda_stream else torch.cuda.ExternalStream(built, device=self.device)
+            if other is not None:
+                other.wait_stream(here)
+            L.check(fn(self._h, out.data_ptr(), cnt.value, C.byref(cnt), built), "sgb_existing_point_ids")
+            if other is not None:
+                here.wait_stream(other)
         return out
 
     # ---------------------------------------------------------------- stencils
