@@ -285,9 +285,9 @@ int sgb_batch_add(sgb_batch* b, sgb_grid* g, int kind, const int* src, const int
     }
     SGB_TRY(batch_compact(b, s));
     SGB_TRY(ensure_neighbours(g, SGB_NN_STAR, s));
-    for (int p = 0; p < b->np; ++p) {  // batched kernels rely on background-filled empty points
-        SGB_TRY(ensure_clean(g, src[p], s));
-        SGB_TRY(ensure_clean(g, dst[p], s));
+    {  // batched kernels rely on background-filled empty points
+        const int props[4] = {src[0], dst[0], src[b->np - 1], dst[b->np - 1]};
+        SGB_TRY(ensure_clean_f32(g, props, 2 * b->np, true, s));
     }
     const int bs = g->geo.bs;
     SGB_TRY(batch_reserve(b, b->n + g->n));

@@ -111,6 +111,15 @@ __device__ __forceinline__ void cp_async_wait_group() {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
+// The next launch may begin while this one drains.
+__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Waits for the launch before this one; the returned value orders the loads that use it behind the wait.
+__device__ __forceinline__ int64_t grid_dependency_wait() {
+    int64_t z;
+    asm volatile("griddepcontrol.wait;\n\tmov.u64 %0, 0;" : "=l"(z)::"memory");
+    return z;
+}
+
 __device__ __forceinline__ unsigned lanemask_lt() {
     unsigned m;
     asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));

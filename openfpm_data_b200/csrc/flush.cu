@@ -962,7 +962,10 @@ static int flush_impl(sgb_grid* g, const int* ops, int bits, cudaStream_t s) {
         // swap buffer sets
         std::swap(g->keys, g->keys2);
         std::swap(g->mask, g->mask2);
-        for (int p = 0; p < g->nprop; ++p) std::swap(g->data[p], g->data2[p]);
+        for (int p = 0; p < g->nprop; ++p) {
+            std::swap(g->data[p], g->data2[p]);
+            g->exposed[p] = false;
+        }
         g->cap = cap2;
         g->n = nn_;
     }

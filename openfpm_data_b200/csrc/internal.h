@@ -314,6 +314,10 @@ struct sgb_grid {
     // keeping them filled lets the stencils read chunk data without a mask
     // test per neighbour.  Cleared when the caller gets a writable pointer.
     bool clean[sgb::kMaxProps] = {true, true, true, true, true, true, true, true};
+    // exposed[p]: since the map's buffers were last exchanged (which ends the caller's pointers) the caller has had a
+    // pointer that can write property p or the masks.  It may still write through it, so clean[p] stands for the call
+    // that established it and not for the next one: a step then writes the backgrounds of its destination again.
+    bool exposed[sgb::kMaxProps] = {};
 
     // flush / scan / sort scratch
     sgb::DevBuf scratch[12];
@@ -338,9 +342,6 @@ int launch_points_box27_sparse(sgb_grid* g, const int* src, const int* dst, cons
                                cudaStream_t s);
 
 // stencil.cu
-// chained: follows a launch over the same masks and neighbours in the same call
-int launch_stencil(sgb_grid* g, int kind, const int* src, const int* dst, const StencilParams& prm,
-                   cudaStream_t s, bool chained = false);
 int make_params(sgb_grid* g, int kind, const int* src, const int* dst, const float* params, int nparams,
                 const int64_t* box, StencilParams& prm);
 
@@ -355,6 +356,8 @@ int sanitize_prop(sgb_grid* g, int p, cudaStream_t s);
 // fill every point (n + 1 chunks) of property p with its background
 int fill_background_all(sgb_grid* g, int p, cudaStream_t s);
 int ensure_clean(sgb_grid* g, int p, cudaStream_t s);
+// the same for up to four float32 properties in one launch; again: also those that are exposed
+int ensure_clean_f32(sgb_grid* g, const int* props, int count, bool again, cudaStream_t s);
 // fill count elements of esize bytes with the low esize bytes of pattern
 int fill(void* dst, int64_t count, int esize, uint64_t pattern, cudaStream_t s);
 // the background of property p as an element_size-byte pattern

@@ -58,7 +58,7 @@ __host__ __device__ constexpr size_t solve_smem(int cap) {
 template <int KIND, int NP>
 __global__ void __launch_bounds__(kSolveThreads, 1)
     k_solve_cluster(FieldSet fs, const uint8_t* __restrict__ mask, const int32_t* __restrict__ nn, int n, GridInfo gi,
-                    int nsteps, int cap) {
+                    int nsteps, int cap, int again) {
     extern __shared__ __align__(16) unsigned char solve_raw[];
     float* const F = reinterpret_cast<float*>(solve_raw);                   // [2][NP][cap][512]
     uint8_t* const mk = solve_raw + (size_t)cap * 2 * NP * 2048;            // [cap][512]
@@ -76,13 +76,22 @@ __global__ void __launch_bounds__(kSolveThreads, 1)
         bq[threadIdx.x] = splat4(b ? (p ? gi.bck[1][NP - 1] : gi.bck[1][0]) : (p ? gi.bck[0][NP - 1] : gi.bck[0][0]));
     }
     const uint32_t bqa = map_cluster(smem_u32(bq), rank);
-    for (int i = threadIdx.x; i < m * 128; i += kSolveThreads)
+    for (int i = threadIdx.x; i < m * 128; i += kSolveThreads) {
+        const uint32_t m4 = again ? reinterpret_cast<const uint32_t*>(mask + (int64_t)a * 512)[i] : 0x01010101u;
 #pragma unroll
-        for (int p = 0; p < NP; ++p) {
-            reinterpret_cast<float4*>(F + p * fstride)[i] = reinterpret_cast<const float4*>(fs.in[0][p] + (int64_t)a * 512)[i];
-            reinterpret_cast<float4*>(F + (NP + p) * fstride)[i] =
-                reinterpret_cast<const float4*>(fs.in[1][p] + (int64_t)a * 512)[i];
-        }
+        for (int p = 0; p < NP; ++p)
+#pragma unroll
+            for (int b = 0; b < 2; ++b) {
+                float4 v = reinterpret_cast<const float4*>(fs.in[b][p] + (int64_t)a * 512)[i];
+                if (m4 != 0x01010101u) {
+                    v.x = m4 & 0xffu ? v.x : gi.bck[b][p];
+                    v.y = m4 & 0xff00u ? v.y : gi.bck[b][p];
+                    v.z = m4 & 0xff0000u ? v.z : gi.bck[b][p];
+                    v.w = m4 & 0xff000000u ? v.w : gi.bck[b][p];
+                }
+                reinterpret_cast<float4*>(F + (b * NP + p) * fstride)[i] = v;
+            }
+    }
     for (int i = threadIdx.x; i < m * 32; i += kSolveThreads)
         reinterpret_cast<uint4*>(mk)[i] = reinterpret_cast<const uint4*>(mask + (int64_t)a * 512)[i];
     // cluster addresses of the neighbours' tiles (field 0, buffer 0); the owner of position q is (P (q + 1) - 1) / n
@@ -169,7 +178,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1)
 
 template <int KIND, int NP>
 static int launch_solve(const FieldSet& fs, const uint8_t* mask, const int32_t* nn, int n, const GridInfo& gi, int nsteps,
-                        cudaStream_t s) {
+                        bool again, cudaStream_t s) {
     auto kern = k_solve_cluster<KIND, NP>;
     int ctas = 1;
     while (ctas < kSolveCtas && ctas < n) ctas *= 2;
@@ -195,12 +204,12 @@ static int launch_solve(const FieldSet& fs, const uint8_t* mask, const int32_t* 
         cudaGetLastError();  // the device has no room for such a cluster: one launch per step
         return SGB_ENOTSUP;
     }
-    SGB_CUDA(cudaLaunchKernelEx(&cfg, kern, fs, mask, nn, n, gi, nsteps, cap));
+    SGB_CUDA(cudaLaunchKernelEx(&cfg, kern, fs, mask, nn, n, gi, nsteps, cap, again ? 1 : 0));
     return SGB_OK;
 }
 
 int run_steps_cluster(sgb_grid* g, int kind, const int* src, const int* dst, const StencilParams& fwd, int nsteps,
-                      cudaStream_t s) {
+                      bool again, cudaStream_t s) {
     if ((kind != SGB_HEAT7 && kind != SGB_GS7) || g->geo.edge != 8) return SGB_ENOTSUP;
     // Heat while a CTA's half chunks take one round of its 32 groups; Gray-Scott, with twice the rows a point, up to
     // the size where a launch per step is as fast.  A launch per step costs 2.64 us (heat) / 2.8-3.0 us
@@ -218,8 +227,8 @@ int run_steps_cluster(sgb_grid* g, int kind, const int* src, const int* dst, con
     const GridInfo gi = grid_info_of(fwd);
     const uint8_t* mask = g->mask.as<uint8_t>();
     const int32_t* nn = g->nn[SGB_NN_STAR].as<int32_t>();
-    return kind == SGB_GS7 ? launch_solve<SGB_GS7, 2>(fs, mask, nn, (int)g->n, gi, nsteps, s)
-                           : launch_solve<SGB_HEAT7, 1>(fs, mask, nn, (int)g->n, gi, nsteps, s);
+    return kind == SGB_GS7 ? launch_solve<SGB_GS7, 2>(fs, mask, nn, (int)g->n, gi, nsteps, again, s)
+                           : launch_solve<SGB_HEAT7, 1>(fs, mask, nn, (int)g->n, gi, nsteps, again, s);
 }
 
 }  // namespace sgb

@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(kStarThreads, MINB)
             if (in_cta) xo = xs[(p * ZS + z) * 80];
             lap[p] = lap_quad<KIND>(cv[p], xq ? got : xo, xq ? xo : got, ym, yp, zm[p], zp[p]);
         }
-        if (m[z] || (KIND == SGB_HEAT7 && fill && live)) {
+        if (m[z] || (fill && live)) {
             const uint32_t act = active_bits<BOX>(m[z], box, cx, cy, cz + z);
             star_store<KIND, NP>(cv, lap, m[z], act, gi, bd, dst[0] + z * 64, dst[NP - 1] + z * 64);
         }
@@ -249,7 +249,7 @@ __global__ void __launch_bounds__(kStarThreads, MINB)
     }
     const GridInfo& gi = BATCH ? gb : g0;
     const uint32_t m = live ? __ldg(reinterpret_cast<const uint32_t*>(mask + c * 64 + l16 * 4)) : 0u;
-    if (!m && !(KIND == SGB_HEAT7 && fill && live)) {
+    if (!m && !(fill && live)) {
         // The row holds no point.  No thread leaves without the wait: a launch of idle rows only would be over
         // before the step ahead of it, and what follows in the stream waits for this launch alone.
         grid_dependency_wait();

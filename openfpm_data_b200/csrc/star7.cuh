@@ -19,15 +19,6 @@ __device__ __forceinline__ float ldf1(const float* p) {
     asm("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
     return v;
 }
-// The next launch may begin while this one drains.
-__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-// Waits for the launch before this one; the returned value orders the loads that use it behind the wait.
-__device__ __forceinline__ int64_t grid_dependency_wait() {
-    int64_t z;
-    asm volatile("griddepcontrol.wait;\n\tmov.u64 %0, 0;" : "=l"(z)::"memory");
-    return z;
-}
-
 __device__ __forceinline__ float4 splat4(float b) { return make_float4(b, b, b, b); }
 
 // Two float32 values in one 64-bit register pair and the packed arithmetic on them (each half rounds as the

@@ -407,8 +407,16 @@ int launch_fields(const LaunchDesc& L, cudaStream_t s) {
     return SGB_OK;
 }
 
-int launch_stencil_impl(sgb_grid* g, int kind, const int* src, const int* dst, const StencilParams& prm,
-                        cudaStream_t s, bool use_tile, bool chained) {
+// A caller may keep a pointer to a property and write points that do not exist.  As the destination of a 7-point step
+// such a property takes its backgrounds again; as a source it does so in every call on 4^3 chunks and Morton ids (one
+// more launch while a pointer is out), and on 8^3 chunks with x-fastest ids when a pointer to it has been taken since
+// its last use.
+static bool cleans_sources(const sgb_grid* g) { return g->geo.edge == 4 || g->geo.zorder; }
+
+// step: -1 for a call of one step; else the step's number in run_steps, which has cleaned the properties.  Steps
+// before `refills` write the backgrounds of an exposed destination.
+static int launch_stencil(sgb_grid* g, int kind, const int* src, const int* dst, const StencilParams& prm,
+                          cudaStream_t s, int step, int refills, bool use_tile = false) {
     if (g->n == 0) return SGB_OK;
     if (kind == SGB_BOX27_NS) return launch_points_box27(g, src, dst, prm, s);
     if (kind == SGB_BOX27 && !use_tile) {  // sparse chunks: the point list
@@ -418,7 +426,8 @@ int launch_stencil_impl(sgb_grid* g, int kind, const int* src, const int* dst, c
     const int nnk = kind == SGB_BOX27 ? SGB_NN_FULL : SGB_NN_STAR;
     SGB_TRY(ensure_neighbours(g, nnk, s));
     const int np = kind == SGB_GS7 ? 2 : 1;
-    for (int j = 0; j < np; ++j) SGB_TRY(ensure_clean(g, src[j], s));
+    // (the tile kernel tests the masks itself)
+    SGB_TRY(ensure_clean_f32(g, src, np, step < 0 && kind != SGB_BOX27 && !use_tile && cleans_sources(g), s));
     LaunchDesc L;
     std::memset(&L, 0, sizeof(L));
     L.kind = kind;
@@ -443,17 +452,13 @@ int launch_stencil_impl(sgb_grid* g, int kind, const int* src, const int* dst, c
     L.geo = g->geo;
     L.prm = prm;
     L.t = 0;
-    L.chained = chained;
-    L.fill = kind == SGB_HEAT7 && !g->clean[dst[0]];
+    L.chained = step > 0;
+    L.fill = (step < refills && (g->exposed[dst[0]] || g->exposed[dst[np - 1]])) ||
+             (kind == SGB_HEAT7 && !g->clean[dst[0]]);
     L.err = g->err.as<unsigned>();
     SGB_TRY(launch_fields(L, s));
     if (kind == SGB_HEAT7) g->clean[dst[0]] = true;  // every point of dst was written from the tile
     return SGB_OK;
-}
-
-int launch_stencil(sgb_grid* g, int kind, const int* src, const int* dst, const StencilParams& prm, cudaStream_t s,
-                   bool chained) {
-    return launch_stencil_impl(g, kind, src, dst, prm, s, false, chained);
 }
 
 }  // namespace sgb
@@ -467,7 +472,7 @@ int sgb_apply_stencil(sgb_grid* g, int kind, const int* src, const int* dst, con
     if (!g) return SGB_EINVAL;
     StencilParams prm;
     SGB_TRY(make_params(g, kind, src, dst, params, nparams, box, prm));
-    return launch_stencil(g, kind, src, dst, prm, (cudaStream_t)s);
+    return launch_stencil(g, kind, src, dst, prm, (cudaStream_t)s, -1, 0);
 }
 
 // Same as sgb_apply_stencil through the generic one-chunk-per-CTA kernel
@@ -477,7 +482,7 @@ int sgb_apply_stencil_tiled(sgb_grid* g, int kind, const int* src, const int* ds
     if (!g) return SGB_EINVAL;
     StencilParams prm;
     SGB_TRY(make_params(g, kind, src, dst, params, nparams, box, prm));
-    return launch_stencil_impl(g, kind, src, dst, prm, (cudaStream_t)s, true, false);
+    return launch_stencil(g, kind, src, dst, prm, (cudaStream_t)s, -1, 0, true);
 }
 
 int sgb_run_steps(sgb_grid* g, int kind, const int* src, const int* dst, const float* params, int nparams, int nsteps,
@@ -492,13 +497,15 @@ int sgb_run_steps(sgb_grid* g, int kind, const int* src, const int* dst, const f
     SGB_TRY(ensure_neighbours(g, kind == SGB_BOX27 || kind == SGB_BOX27_NS ? SGB_NN_FULL : SGB_NN_STAR, s));
     if (kind == SGB_BOX27_NS || kind == SGB_BOX27) SGB_TRY(ensure_point_list(g, s));
     // both halves of the ping-pong are read as sources
-    for (int j = 0; j < (kind == SGB_GS7 ? 2 : 1); ++j) {
-        SGB_TRY(ensure_clean(g, src[j], s));
-        SGB_TRY(ensure_clean(g, dst[j], s));
-    }
+    const int np = kind == SGB_GS7 ? 2 : 1;
+    const int props[4] = {src[0], dst[0], src[np - 1], dst[np - 1]};
+    SGB_TRY(ensure_clean_f32(g, props, 2 * np, false, s));
+    const bool star = kind == SGB_HEAT7 || kind == SGB_GS7;
+    bool exposed = false;
+    for (int j = 0; j < 2 * np; ++j) exposed |= g->exposed[props[j]];
     // a small grid: all steps in one launch
     {
-        const int st = run_steps_cluster(g, kind, src, dst, fwd, nsteps, s);
+        const int st = run_steps_cluster(g, kind, src, dst, fwd, nsteps, exposed, s);
         if (st == SGB_OK) {
             if (kind == SGB_HEAT7) g->clean[nsteps % 2 ? dst[0] : src[0]] = true;
             return SGB_OK;
@@ -509,11 +516,17 @@ int sgb_run_steps(sgb_grid* g, int kind, const int* src, const int* dst, const f
     // every call took 5-10 us per step on the host before the first step ran (31 heat steps of 6.2 us: 524 us),
     // a launch takes about 2 us beside the step before it.  use_graph also asks for the wait at the end, which
     // 7-point solves of at most 4 chunks per SM do without, so that their next call's launches overlap.
-    for (int k = 0; k < nsteps; ++k) {
-        if (k % 2 == 0) SGB_TRY(launch_stencil(g, kind, src, dst, fwd, s, k > 0));
-        else SGB_TRY(launch_stencil(g, kind, dst, src, bwd, s, k > 0));
+    const bool small = star && g->n <= (int64_t)g->num_sms * 4 && nsteps >= 2;
+    int refills = 2;  // each half of the ping-pong once
+    if (star && (small || cleans_sources(g))) {
+        // heat's first step puts the destination in order; Gray-Scott's leaves x quads with padding points alone
+        SGB_TRY(ensure_clean_f32(g, props, kind == SGB_HEAT7 ? 1 : 4, true, s));
+        refills = kind == SGB_HEAT7 ? 1 : 0;
     }
-    const bool small = (kind == SGB_HEAT7 || kind == SGB_GS7) && g->n <= (int64_t)g->num_sms * 4 && nsteps >= 2;
+    for (int k = 0; k < nsteps; ++k) {
+        if (k % 2 == 0) SGB_TRY(launch_stencil(g, kind, src, dst, fwd, s, k, refills));
+        else SGB_TRY(launch_stencil(g, kind, dst, src, bwd, s, k, refills));
+    }
     if (use_graph && !small) SGB_CUDA(cudaStreamSynchronize(s));
     return SGB_OK;
 }

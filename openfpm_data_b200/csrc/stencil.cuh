@@ -79,7 +79,7 @@ struct LaunchDesc {
     Geometry geo;
     StencilParams prm;
     int64_t t;
-    int fill;                // HEAT7: quads without an existing point are written too (dst may hold anything there)
+    int fill;                // quads without an existing point are written too (dst may hold anything there)
     int chained;             // follows a launch over the same masks and neighbours in the same call
     unsigned* err;
 };
@@ -87,8 +87,9 @@ struct LaunchDesc {
 int launch_fields(const LaunchDesc& L, cudaStream_t s);
 int launch_star7(const LaunchDesc& L, cudaStream_t s);  // 7-point kernels, any chunk ids (star7.cu)
 // All steps of a small grid's solve in one launch (solve.cu); SGB_ENOTSUP: not for this grid.
+// again: points that do not exist may hold anything (the caller kept a pointer).
 int run_steps_cluster(sgb_grid* g, int kind, const int* src, const int* dst, const StencilParams& fwd, int nsteps,
-                      cudaStream_t s);
+                      bool again, cudaStream_t s);
 GridInfo grid_info_of(const StencilParams& prm);
 
 }  // namespace sgb

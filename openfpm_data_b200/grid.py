@@ -268,13 +268,17 @@ class SparseGridGpu:
         return torch.as_tensor(_DevView(p.value or 0, (self.nchunks,), "<i8"), device=f"cuda:{self.device}")
 
     def private_get_data_array(self, prop: int) -> torch.Tensor:
-        """Chunk data of one property, (nchunks + 1) * bs elements, background chunk last."""
+        """Chunk data of one property, (nchunks + 1) * bs elements, background chunk last; valid until the
+        next flush.  After writing points that do not exist through a view that was kept, take it again
+        before a step reads the property (a step that writes it puts the background back itself)."""
         p = C.c_void_p()
         L.check(self._lib.sgb_data_buffer(self._h, prop, C.byref(p)), "sgb_data_buffer")
         return torch.as_tensor(_DevView(p.value, ((self.nchunks + 1) * self.bs,), _TS[self.ptypes[prop]]),
                                device=f"cuda:{self.device}")
 
     def private_get_mask_array(self) -> torch.Tensor:
+        """Mask bytes, (nchunks + 1) * bs; valid until the next flush.  Take it again for every change of
+        which points exist: the point lists, bitmaps and backgrounds are renewed by this call."""
         p = C.c_void_p()
         L.check(self._lib.sgb_mask_buffer(self._h, C.byref(p)), "sgb_mask_buffer")
         return torch.as_tensor(_DevView(p.value, ((self.nchunks + 1) * self.bs,), "|u1"), device=f"cuda:{self.device}")
