@@ -995,6 +995,7 @@ extern "C" int sgb_flush(sgb_grid* g, const int* ops, sgb_stream stream) {
     if (bits <= 32) st = flush_impl<uint32_t>(g, ops, bits, s);
     else st = flush_impl<uint64_t>(g, ops, bits, s);
     g->npend = 0;
+    if (st == SGB_ERANGE) return st;  // rejected: the map is as it was, and so is what was made from it
     g->nn_valid[0] = g->nn_valid[1] = false;
     g->nnhash_ok = false;
     g->bits_valid = false;

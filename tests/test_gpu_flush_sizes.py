@@ -54,3 +54,30 @@ def test_flush_drops_out_of_domain(sgb):
         g.flush(["sRight_"])
     g.flush(["sRight_"])
     assert g.countExistingElements() == 2 and g.nchunks == 2
+
+
+def test_rejected_flush_keeps_what_was_made_from_the_map(sgb):
+    """A mark in the existing-point list's memory is still there after a flush that was refused (the list stands),
+    and gone after one that was taken (it is built again)."""
+    import ctypes as C
+    from openfpm_data_b200 import _lib as L
+    from openfpm_data_b200.grid import _DevView
+    g = sgb.SparseGridGpu((40, 40, 40), ["f32"], edge=8)
+    g.insert(torch.tensor([[1, 2, 3], [9, 9, 9]], dtype=torch.int32, device="cuda"), [torch.ones(2, device="cuda")])
+    g.flush(["sRight_"])
+
+    def ids():
+        p, n = C.c_void_p(), C.c_int64()
+        L.check(g._lib.sgb_existing_point_list(g.handle, C.byref(p), C.byref(n), 0), "sgb_existing_point_list")
+        torch.cuda.synchronize()
+        return torch.as_tensor(_DevView(p.value, (n.value,), "<i4"), device="cuda")
+
+    want = ids().clone()
+    ids()[0] = -7
+    g.insert(torch.tensor([[20, 20, 20], [40, 0, 0]], dtype=torch.int32, device="cuda"), [torch.ones(2, device="cuda")])
+    with pytest.raises(sgb.SgbError):
+        g.flush(["sRight_"])
+    assert ids()[0].item() == -7
+    g.insert(torch.tensor([[1, 2, 3]], dtype=torch.int32, device="cuda"), [torch.ones(1, device="cuda")])
+    g.flush(["sRight_"])
+    assert torch.equal(ids(), want)
