@@ -38,7 +38,10 @@ struct UBoxes {
 // A CTA takes 32 chunks: its first warp tests them against the boxes, one chunk per lane, then the warps share
 // the chunks that a box touches, bs / 32 consecutive points per lane.  (A CTA per chunk, tests and all: 53 us
 // for six one-layer slabs of a 512^3 grid of 18.9 K chunks, 17 us so.)  A box cuts a chunk's x rows to one bit
-// mask, so a touched chunk costs a few operations per box and row.
+// mask, so a touched chunk costs a few operations per box and row.  Boxes are taken 64 at a time through shared
+// memory, with a bit per chunk for each that meets it: a grid of few chunks has few CTAs, and each would wait for
+// memory box by box (1000 boxes on 216 chunks, the whole call: 582 us, 1009 with boxes read from memory, 660 with a
+// CTA per chunk).
 template <int P>  // points per lane: 16 (8^3 chunks) or 2 (4^3)
 __global__ void __launch_bounds__(256) k_remove_boxes(const int64_t* __restrict__ keys, int64_t n, Geometry geo, uint8_t* mask,
                                                        const __grid_constant__ UBoxes pb, const UBox* __restrict__ db, int nb,
@@ -46,92 +49,91 @@ __global__ void __launch_bounds__(256) k_remove_boxes(const int64_t* __restrict_
     constexpr int bs = P * 32, e = P == 16 ? 8 : 4;
     __shared__ int hits[32];
     __shared__ uint32_t org[32][3];
-    __shared__ int nhits, range[32][2];
-    // indexed reads of the parameters go through memory: staged once
-    __shared__ UBox sb[kParamBoxes];
-    for (int i = threadIdx.x; i < nb * 6 && nb <= kParamBoxes; i += 256)
-        reinterpret_cast<uint32_t*>(sb)[i] = reinterpret_cast<const uint32_t*>(pb.b)[i];
-    __syncthreads();
-    const UBox* boxes = nb <= kParamBoxes ? sb : db;
+    __shared__ unsigned long long touched[32];  // the boxes of the round that meet the chunk
+    __shared__ int nhits;
+    __shared__ UBox boxes[kParamBoxes];  // indexed reads of the parameters would go through memory
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t c0 = (int64_t)blockIdx.x * 32;
-    if (warp == 0) {
-        bool touch = false;
-        if (c0 + lane < n) {
-            int64_t o[3];
-            chunk_origin(geo, keys[c0 + lane], o);
-            for (int d = 0; d < 3; ++d) org[lane][d] = (uint32_t)o[d];
-            int lo = nb, hi = -1;  // the boxes that touch the chunk lie in [lo, hi]
-            for (int k = 0; k < nb; ++k) {
-                bool t = true;
-                for (int d = 0; d < 3; ++d) {
-                    const uint32_t clo = (uint32_t)o[d], chi = (uint32_t)(o[d] + e - 1);
-                    t = t && !(chi < boxes[k].lo[d] || clo > boxes[k].hi[d]);
-                }
-                if (t) {
-                    if (hi < 0) lo = k;
-                    hi = k;
-                }
-            }
-            range[lane][0] = lo;
-            range[lane][1] = hi;
-            touch = hi >= 0;
-        }
-        const unsigned t = __ballot_sync(0xffffffffu, touch);
-        if (touch) hits[__popc(t & lanemask_lt())] = lane;
-        if (lane == 0) nhits = __popc(t);
+    if (warp == 0 && c0 + lane < n) {
+        int64_t o[3];
+        chunk_origin(geo, keys[c0 + lane], o);
+        for (int d = 0; d < 3; ++d) org[lane][d] = (uint32_t)o[d];
     }
-    __syncthreads();
-    for (int h = warp; h < nhits; h += 8) {
-        const int j = hits[h];
-        const int64_t first = (c0 + j) * bs + lane * P;
-        union {
-            uint4 v;
-            uint16_t s;
-            uint8_t b[16];
-        } m;
-        if (P == 16) m.v = *reinterpret_cast<const uint4*>(mask + first);
-        else m.s = *reinterpret_cast<const uint16_t*>(mask + first);
-        uint32_t gone = 0;  // the lane's points inside a box, then the existing ones of them
-        for (int k = range[j][0]; k <= range[j][1]; ++k) {
-            int lo[3], hi[3];  // the box in the chunk's coordinates, clipped to it
-#pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                const int64_t o = org[j][d], l = (int64_t)boxes[k].lo[d] - o, u = (int64_t)boxes[k].hi[d] - o;
-                lo[d] = l < 0 ? 0 : l > e ? e : (int)l;
-                hi[d] = u < -1 ? -1 : u > e - 1 ? e - 1 : (int)u;
-            }
-            if (lo[0] > hi[0]) continue;
-            const uint32_t xm = (2u << hi[0]) - (1u << lo[0]);
-            if (P == 16) {  // two x rows
-#pragma unroll
-                for (int r = 0; r < 2; ++r) {
-                    const int y = (2 * lane + r) & 7, z = (2 * lane + r) >> 3;
-                    if (y >= lo[1] && y <= hi[1] && z >= lo[2] && z <= hi[2]) gone |= xm << (8 * r);
+    for (int k0 = 0; k0 < nb; k0 += kParamBoxes) {
+        const int nk = nb - k0 < kParamBoxes ? nb - k0 : kParamBoxes;
+        const uint32_t* from = reinterpret_cast<const uint32_t*>(nb <= kParamBoxes ? pb.b : db + k0);
+        __syncthreads();  // the round before has read its boxes
+        for (int i = threadIdx.x; i < nk * 6; i += 256) reinterpret_cast<uint32_t*>(boxes)[i] = from[i];
+        __syncthreads();
+        if (warp == 0) {
+            unsigned long long in = 0;
+            if (c0 + lane < n) {
+                uint32_t clo[3];
+                for (int d = 0; d < 3; ++d) clo[d] = org[lane][d];
+                for (int k = 0; k < nk; ++k) {
+                    bool t = true;
+                    for (int d = 0; d < 3; ++d) t = t && !(clo[d] + (e - 1) < boxes[k].lo[d] || clo[d] > boxes[k].hi[d]);
+                    in |= (unsigned long long)t << k;
                 }
-            } else {  // half an x row
-                const int y = lane >> 1 & 3, z = lane >> 3;
-                if (y >= lo[1] && y <= hi[1] && z >= lo[2] && z <= hi[2]) gone |= xm >> (2 * (lane & 1)) & 3u;
+                touched[lane] = in;
             }
+            const unsigned t = __ballot_sync(0xffffffffu, in != 0);
+            if (in) hits[__popc(t & lanemask_lt())] = lane;
+            if (lane == 0) nhits = __popc(t);
         }
-        uint32_t ex = 0;
+        __syncthreads();
+        for (int h = warp; h < nhits; h += 8) {
+            const int j = hits[h];
+            const int64_t first = (c0 + j) * bs + lane * P;
+            union {
+                uint4 v;
+                uint16_t s;
+                uint8_t b[16];
+            } m;
+            if (P == 16) m.v = *reinterpret_cast<const uint4*>(mask + first);
+            else m.s = *reinterpret_cast<const uint16_t*>(mask + first);
+            uint32_t gone = 0;  // the lane's points inside a box, then the existing ones of them
+            for (unsigned long long left = touched[j]; left; left &= left - 1) {
+                const int k = __ffsll((long long)left) - 1;
+                int lo[3], hi[3];  // the box in the chunk's coordinates, clipped to it
 #pragma unroll
-        for (int i = 0; i < P; ++i) ex |= (uint32_t)(m.b[i] & 1) << i;
-        gone &= ex;
-        if (!gone) continue;
+                for (int d = 0; d < 3; ++d) {
+                    const int64_t o = org[j][d], l = (int64_t)boxes[k].lo[d] - o, u = (int64_t)boxes[k].hi[d] - o;
+                    lo[d] = l < 0 ? 0 : l > e ? e : (int)l;
+                    hi[d] = u < -1 ? -1 : u > e - 1 ? e - 1 : (int)u;
+                }
+                if (lo[0] > hi[0]) continue;
+                const uint32_t xm = (2u << hi[0]) - (1u << lo[0]);
+                if (P == 16) {  // two x rows
 #pragma unroll
-        for (int i = 0; i < P; ++i)
-            if (gone >> i & 1u) m.b[i] = 0;
-        if (P == 16) *reinterpret_cast<uint4*>(mask + first) = m.v;
-        else *reinterpret_cast<uint16_t*>(mask + first) = m.s;
-        for (int p = 0; p < bck.nprop; ++p) {
-            unsigned char* q = bck.p[p] + (size_t)first * bck.es[p];
-            const uint64_t pat = bck.pat[p];
-            for (uint32_t w = gone; w; w &= w - 1) {
-                const int i = __ffs(w) - 1;
-                if (bck.es[p] == 4) reinterpret_cast<uint32_t*>(q)[i] = (uint32_t)pat;
-                else if (bck.es[p] == 8) reinterpret_cast<uint64_t*>(q)[i] = pat;
-                else q[i] = (unsigned char)pat;
+                    for (int r = 0; r < 2; ++r) {
+                        const int y = (2 * lane + r) & 7, z = (2 * lane + r) >> 3;
+                        if (y >= lo[1] && y <= hi[1] && z >= lo[2] && z <= hi[2]) gone |= xm << (8 * r);
+                    }
+                } else {  // half an x row
+                    const int y = lane >> 1 & 3, z = lane >> 3;
+                    if (y >= lo[1] && y <= hi[1] && z >= lo[2] && z <= hi[2]) gone |= xm >> (2 * (lane & 1)) & 3u;
+                }
+            }
+            uint32_t ex = 0;
+#pragma unroll
+            for (int i = 0; i < P; ++i) ex |= (uint32_t)(m.b[i] & 1) << i;
+            gone &= ex;
+            if (!gone) continue;
+#pragma unroll
+            for (int i = 0; i < P; ++i)
+                if (gone >> i & 1u) m.b[i] = 0;
+            if (P == 16) *reinterpret_cast<uint4*>(mask + first) = m.v;
+            else *reinterpret_cast<uint16_t*>(mask + first) = m.s;
+            for (int p = 0; p < bck.nprop; ++p) {
+                unsigned char* q = bck.p[p] + (size_t)first * bck.es[p];
+                const uint64_t pat = bck.pat[p];
+                for (uint32_t w = gone; w; w &= w - 1) {
+                    const int i = __ffs(w) - 1;
+                    if (bck.es[p] == 4) reinterpret_cast<uint32_t*>(q)[i] = (uint32_t)pat;
+                    else if (bck.es[p] == 8) reinterpret_cast<uint64_t*>(q)[i] = pat;
+                    else q[i] = (unsigned char)pat;
+                }
             }
         }
     }

@@ -87,3 +87,27 @@ def test_existing_points_order_matches_oracle(sgb, edge):
     sub = g.existing_points(box).cpu().numpy().astype(np.int64)
     assert np.array_equal(sub, o.existing_points(box))
     assert len(list(g.getIterator((5, 7, 9), (33, 30, 40)))) == len(sub)
+
+
+@pytest.mark.parametrize("edge", [8, 4])
+@pytest.mark.parametrize("nboxes", [1, 64, 65, 128, 200])
+def test_remove_box_counts(sgb, edge, nboxes):
+    """As many boxes as launch parameters and one round of the kernel hold, and more: small overlapping ones, some
+    one layer thick, some across chunk faces or past the domain."""
+    size = (61, 50, 47)
+    g, o = _grid_pair(sgb, size, 40000, nboxes + edge, edge)
+    rng = np.random.default_rng(nboxes + edge)
+    lo = rng.integers(0, 55, size=(nboxes, 3))
+    hi = lo + rng.integers(0, 9, size=(nboxes, 3)) * (rng.random((nboxes, 3)) < 0.7)
+    for a, b in zip(lo.tolist(), hi.tolist()):
+        g.remove((a, b))
+    g.removePoints()
+    o.remove_boxes([a + b for a, b in zip(lo.tolist(), hi.tolist())])
+    keys, data, mask = g.deviceToHost()
+    okeys, odata, omask = o.export()
+    n = len(okeys)
+    assert np.array_equal(keys, okeys) and np.array_equal(mask[: n * g.bs], omask[: n * g.bs])
+    ex = (mask[: n * g.bs] & 1).astype(bool)
+    for p, b in enumerate([0.25, 0.5]):
+        assert np.array_equal(data[p][: n * g.bs][ex], odata[p][: n * g.bs][ex])
+        assert np.all(data[p][: n * g.bs][~ex] == np.float32(b))
