@@ -76,7 +76,9 @@ struct HitBox {
 // The packed points come from few chunks, so the chunks are found first: which chunks each box meets, as bitmaps
 // of 32 chunks (a warp per 32 chunks, a lane per chunk, all boxes), then a list of the hits in (box, chunk) order.
 // The point work that follows takes a warp per hit and not a warp per chunk of the grid (six one-layer slabs of a
-// 512^3 grid meet 1.7 K of 6 x 18.9 K (box, chunk) pairs: count 54 -> 28 us, emission 64 -> 14 us).
+// 512^3 grid meet 1.7 K of 6 x 18.9 K (box, chunk) pairs: count 54 -> 28 us, emission 64 -> 14 us).  The boxes are
+// split over the grid's second dimension, since few chunks make few warps (request and pack of 200 boxes on 216
+// chunks 555 us with all boxes in one warp, 335 so).
 __global__ void __launch_bounds__(256) k_pack_hits(const int64_t* __restrict__ keys, int64_t n, Geometry geo,
                                                     const HitBox* __restrict__ boxes, int nb, int64_t words,
                                                     uint32_t* __restrict__ bits, uint32_t* __restrict__ cnt) {
@@ -86,7 +88,7 @@ __global__ void __launch_bounds__(256) k_pack_hits(const int64_t* __restrict__ k
     const int64_t c = w * 32 + lane;
     int64_t bc[3] = {-1, -1, -1};  // below every box's range
     if (c < n) block_coords(geo, keys[c], bc);
-    for (int k = 0; k < nb; ++k) {
+    for (int k = blockIdx.y; k < nb; k += gridDim.y) {
         const HitBox& b = boxes[k];
         const bool in = bc[0] >= b.lo[0] && bc[0] <= b.hi[0] && bc[1] >= b.lo[1] && bc[1] <= b.hi[1] && bc[2] >= b.lo[2] &&
                         bc[2] <= b.hi[2];
@@ -565,7 +567,10 @@ static int pack_counts(sgb_grid* g, int64_t nboxes, const int64_t* boxes_host, s
     ps.rows = g->scratch[8].as<uint32_t>();
     SGB_CUDA(cudaMemcpyAsync(ps.boxes, hbx, (size_t)nboxes * sizeof(HitBox), cudaMemcpyHostToDevice, s));
     uint32_t* nhits = ps.start + ps.len;
-    k_pack_hits<<<(unsigned)((ps.words + 7) / 8), 256, 0, s>>>(g->keys.as<int64_t>(), n, g->geo, ps.boxes, (int)nboxes,
+    // boxes are shared out over the grid's second dimension until the chip holds no more CTAs
+    const int64_t hx = (ps.words + 7) / 8;
+    const int64_t hy = std::max<int64_t>(1, std::min<int64_t>({nboxes, (int64_t)g->num_sms * 8 / hx, 65535}));
+    k_pack_hits<<<dim3((unsigned)hx, (unsigned)hy), 256, 0, s>>>(g->keys.as<int64_t>(), n, g->geo, ps.boxes, (int)nboxes,
                                                                ps.words, ps.bits, ps.cnt);
     SGB_CUDA(cudaGetLastError());
     SGB_TRY(scan_exclusive_u32(ps.cnt, ps.start, ps.len, nhits, &g->scratch[6], s));

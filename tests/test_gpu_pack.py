@@ -225,3 +225,21 @@ def test_unpack_boxes_equals_box_by_box(sgb, with_starts):
     b.removeAddUnpackFinalize(props)
     assert b.countExistingElements() == n_before
     b.check_device_errors()
+
+
+@pytest.mark.parametrize("nboxes", [1, 31, 300])
+@pytest.mark.parametrize("edge", [8, 4])
+def test_pack_many_boxes_on_few_chunks(sgb, edge, nboxes):
+    """More boxes than chunks, overlapping, some empty or outside the grid: byte-identical to the oracle."""
+    size = (30, 26, 22)
+    rng = np.random.default_rng(nboxes + edge)
+    pts = np.unique(rng.integers(0, size, size=(5000, 3)), axis=0).astype(np.int64)
+    vals = [rng.random(len(pts)).astype(np.float32)]
+    g = sgb.SparseGridGpu(size, ["f32"], edge=edge)
+    o = O.OracleGrid(size, edge=edge, ptypes=[O.T_F32])
+    g.insert(torch.from_numpy(pts).cuda(), [torch.from_numpy(vals[0]).cuda()])
+    g.flush(["smax_"])
+    o.insert_flush(pts, vals, [O.OP_MAX])
+    lo = rng.integers(-4, 30, size=(nboxes, 3))
+    boxes = [a + b for a, b in zip(lo.tolist(), (lo + rng.integers(0, 12, size=(nboxes, 3))).tolist())]
+    assert bytes(g.pack_boxes(boxes, [0]).cpu().numpy()) == o.pack(boxes, [0])
