@@ -43,6 +43,30 @@ def test_flush_sizes(sgb, edge, n, spread):
         assert np.array_equal(a[ex], np.asarray(b)[ex])
 
 
+@pytest.mark.parametrize("n,distinct", [(5, 1), (8192, 1), (8192, 3), (8193, 1), (20001, 1), (33000, 6)])
+def test_points_inserted_many_times(sgb, n, distinct):
+    """Long runs of one point in the sorted list, in the one-launch flush and in the tiles of the other; the sums are
+    taken in insertion order, so they are exact too."""
+    rng = np.random.default_rng(n)
+    size = (40, 40, 40)
+    g = sgb.SparseGridGpu(size, ["f32", "f64", "i32", "u8"], edge=8)
+    o = O.OracleGrid(size, edge=8, ptypes=[O.T_F32, O.T_F64, O.T_I32, O.T_U8])
+    pool = np.array([[9, 9, 9], [1, 2, 3], [10, 9, 9], [39, 39, 39], [0, 0, 0], [16, 8, 8]], dtype=np.int64)[:distinct]
+    for _ in range(2):
+        pts = pool[rng.integers(0, distinct, n)]
+        vals = [rng.standard_normal(n).astype(np.float32), rng.standard_normal(n),
+                rng.integers(0, 2 ** 31 - 1, n).astype(np.int32), rng.integers(0, 255, n).astype(np.uint8)]
+        g.insert(torch.from_numpy(pts.astype(np.int32)).cuda(), [torch.from_numpy(v).cuda() for v in vals])
+        g.flush(["sadd_", "smin_", "sBitwiseOr_", "smax_"])
+        o.insert_flush(pts, vals, [O.OP_ADD, O.OP_MIN, O.OP_OR, O.OP_MAX])
+    keys, data, mask = g.deviceToHost()
+    okeys, odata, omask = o.export()
+    assert np.array_equal(keys, okeys) and np.array_equal(mask, omask)
+    ex = (mask & 1).astype(bool)
+    for a, b in zip(data, odata):
+        assert np.array_equal(a[ex], np.asarray(b)[ex])
+
+
 def test_flush_drops_out_of_domain(sgb):
     """The staged points are dropped and the map stays as it was when one of them lies outside."""
     g = sgb.SparseGridGpu((40, 40, 40), ["f32"], edge=8)
