@@ -1,4 +1,4 @@
-// All steps of a small grid's heat or Gray-Scott solve in one launch.
+// All steps of a small grid's heat or Gray-Scott solve in one launch: first 8^3 chunks, 4^3 chunks below.
 //
 // A grid of a few hundred 8^3 chunks runs a step in less time than a launch
 // costs.  Here one cluster of up to 16 CTAs keeps the whole solve in its
@@ -208,15 +208,118 @@ static int launch_solve(const FieldSet& fs, const uint8_t* mask, const int32_t* 
     return SGB_OK;
 }
 
-int run_steps_cluster(sgb_grid* g, int kind, const int* src, const int* dst, const StencilParams& fwd, int nsteps,
+// 4^3 chunks: all steps in one cooperative launch (all CTAs resident).  Each CTA takes chunks blockIdx.x + k *
+// gridDim.x, a thread per cell of the 6^3 tile with the mask tested for each, and the CTAs meet at a grid barrier (an
+// arrival counter, a bounded wait) before the next step reads what the last one wrote.  Field reads bypass L1 (other
+// SMs wrote them during the launch).  Arithmetic and stores are those of k_stencil_tile.
+template <int KIND>
+__global__ void __launch_bounds__(256) k_steps_coop4(FieldSet fs, const uint8_t* __restrict__ mask,
+                                                     const int32_t* __restrict__ nn, int64_t n, GridInfo gi, int nsteps,
+                                                     unsigned* bar, unsigned* err) {
+    constexpr int E = 4, T = E + 2, TT = T * T * T, BS = E * E * E;
+    constexpr int NP = KIND == SGB_GS7 ? 2 : 1;
+    __shared__ float tile[NP][TT];
+    __shared__ int abort_run;
+    if (threadIdx.x == 0) abort_run = 0;
+    // the thread's cell of the tile: its neighbour slot (6: the chunk itself, -1: an edge, which 7 points do not use)
+    // and its offset there
+    const int tx = threadIdx.x % T, ty = threadIdx.x / T % T, tz = threadIdx.x / (T * T);
+    const int dx = tx == 0 ? -1 : (tx == T - 1), dy = ty == 0 ? -1 : (ty == T - 1), dz = tz == 0 ? -1 : (tz == T - 1);
+    const int out = (dx != 0) + (dy != 0) + (dz != 0);
+    const int slot = threadIdx.x >= TT || out > 1 ? -1 : !out ? 6 : dx ? (dx > 0) : dy ? 2 + (dy > 0) : 4 + (dz > 0);
+    const int off = (tx + E - 1) % E + E * ((ty + E - 1) % E + E * ((tz + E - 1) % E));
+    for (int t = 0; t < nsteps; ++t) {
+        const int par = t & 1;
+        const float* src[2] = {par ? fs.in[1][0] : fs.in[0][0], par ? fs.in[1][NP - 1] : fs.in[0][NP - 1]};
+        float* d0 = par ? fs.out[1][0] : fs.out[0][0];
+        float* d1 = par ? fs.out[1][NP - 1] : fs.out[0][NP - 1];
+        for (int64_t chunk = blockIdx.x; chunk < n; chunk += gridDim.x) {
+            if (slot >= 0) {
+                const int64_t sc = slot == 6 ? chunk : nn[chunk * 8 + slot];
+                const int64_t idx = sc * BS + off;
+                const bool ex = sc >= 0 && mask[idx] != 0;
+#pragma unroll
+                for (int p = 0; p < NP; ++p)
+                    tile[p][threadIdx.x] = ex ? __ldcg(src[p] + idx) : (par ? gi.bck[1][p] : gi.bck[0][p]);
+            }
+            __syncthreads();
+            if (threadIdx.x < BS) {
+                const int x = threadIdx.x % E, y = threadIdx.x / E % E, z = threadIdx.x / (E * E);
+                const int64_t gidx = chunk * BS + threadIdx.x;
+                const uint8_t m = mask[gidx];
+                const bool act = (m & 1) && !(m & 2);
+                const int c = (x + 1) + T * ((y + 1) + T * (z + 1));
+                auto lap_of = [&](const float* f) {
+                    return lap7k<KIND>(f[c], f[c - 1], f[c + 1], f[c - T], f[c + T], f[c - T * T], f[c + T * T]);
+                };
+                if (KIND == SGB_HEAT7) {
+                    const float cur = tile[0][c];
+                    d0[gidx] = act ? __fmaf_rn(gi.dt, lap_of(tile[0]), cur) : (m ? cur : (par ? gi.bck[0][0] : gi.bck[1][0]));
+                } else if (act) {
+                    float un, vn;
+                    gs_update(tile[0][c], tile[NP - 1][c], lap_of(tile[0]), lap_of(tile[NP - 1]), gi, un, vn);
+                    d0[gidx] = un;
+                    d1[gidx] = vn;
+                }
+            }
+            __syncthreads();
+        }
+        if (t + 1 < nsteps) {
+            // arrival t + 1 of every CTA; the counter only grows.  Every thread fences its stores of this step
+            // before the CTA arrives.
+            __threadfence();
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                __threadfence();
+                atomicAdd(bar, 1u);
+                const unsigned target = (unsigned)(t + 1) * gridDim.x;
+                const uint64_t t0 = global_timer_ns();
+                for (uint32_t it = 0;; ++it) {
+                    if (*reinterpret_cast<volatile unsigned*>(bar) >= target) break;
+                    if ((it & 63u) == 63u && global_timer_ns() - t0 > 2000000000ull) {
+                        atomicOr(err, kErrWaitTimeout);
+                        abort_run = 1;
+                        break;
+                    }
+                }
+                __threadfence();
+            }
+            __syncthreads();
+            if (abort_run) return;
+        }
+    }
+}
+
+static int run_steps_coop4(sgb_grid* g, int kind, const FieldSet& fields, const StencilParams& fwd, int nsteps, cudaStream_t s) {
+    // Where it is the faster one (whole calls in us, here / a launch per step, heat; Gray-Scott within 10 %): 8 chunks
+    // 100 steps 197 / 221, 12 chunks 232 / 221; 148 chunks 8 steps 24 / 24, 5 steps 17 / 18, 3 steps 11 / 14; 444 chunks
+    // 3 steps 13 / 13, 592 chunks 15 / 14.
+    const int64_t sms = g->num_sms;
+    if (!(g->n <= 8 || (g->n <= sms && nsteps <= 8) || (g->n <= 3 * sms && nsteps <= 3))) return SGB_ENOTSUP;
+    if ((int64_t)nsteps * g->n >= (int64_t(1) << 31)) return SGB_ENOTSUP;  // arrival counter range
+    FieldSet fs = fields;
+    GridInfo gi = grid_info_of(fwd);
+    const uint8_t* mask = g->mask.as<uint8_t>();
+    const int32_t* nn = g->nn[SGB_NN_STAR].as<int32_t>();
+    int64_t n = g->n;
+    unsigned* err = g->err.as<unsigned>();
+    SGB_TRY(g->scratch[11].ensure(64));
+    unsigned* bar = g->scratch[11].as<unsigned>();
+    const void* kern = kind == SGB_GS7 ? (const void*)k_steps_coop4<SGB_GS7> : (const void*)k_steps_coop4<SGB_HEAT7>;
+    int per_sm = 0;
+    SGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, 0));
+    if (per_sm < 1) return SGB_ENOTSUP;
+    SGB_CUDA(cudaMemsetAsync(bar, 0, 4, s));
+    const int64_t blocks = std::min<int64_t>(n, (int64_t)per_sm * g->num_sms);
+    void* args[] = {&fs, &mask, &nn, &n, &gi, &nsteps, &bar, &err};
+    SGB_CUDA(cudaLaunchCooperativeKernel(kern, dim3((unsigned)blocks), dim3(256), args, 0, s));
+    return SGB_OK;
+}
+
+int run_steps_one_launch(sgb_grid* g, int kind, const int* src, const int* dst, const StencilParams& fwd, int nsteps,
                       bool again, cudaStream_t s) {
-    if ((kind != SGB_HEAT7 && kind != SGB_GS7) || g->geo.edge != 8) return SGB_ENOTSUP;
-    // Heat while a CTA's half chunks take one round of its 32 groups; Gray-Scott, with twice the rows a point, up to
-    // the size where a launch per step is as fast.  A launch per step costs 2.64 us (heat) / 2.8-3.0 us
-    // (Gray-Scott) whatever the size; here (us per step, 100 steps): heat 36 chunks 1.15, 122 1.56, 219 2.07,
-    // 301 2.93, 391 3.22; Gray-Scott 36 chunks 1.66, 122 2.36, 174 2.97, 219 3.50.
+    if ((kind != SGB_HEAT7 && kind != SGB_GS7) || nsteps < 2) return SGB_ENOTSUP;
     const int np = kind == SGB_GS7 ? 2 : 1;
-    if (g->n > (np == 1 ? 16 : 10) * kSolveCtas || nsteps < 2 || nsteps > (1 << 20)) return SGB_ENOTSUP;
     FieldSet fs;
     for (int j = 0; j < 2; ++j) {
         fs.in[0][j] = g->data[src[j < np ? j : 0]].as<float>();
@@ -224,6 +327,12 @@ int run_steps_cluster(sgb_grid* g, int kind, const int* src, const int* dst, con
         fs.in[1][j] = g->data[dst[j < np ? j : 0]].as<float>();
         fs.out[1][j] = g->data[src[j < np ? j : 0]].as<float>();
     }
+    if (g->geo.edge == 4) return run_steps_coop4(g, kind, fs, fwd, nsteps, s);
+    // Heat while a CTA's half chunks take one round of its 32 groups; Gray-Scott, with twice the rows a point, up to
+    // the size where a launch per step is as fast.  A launch per step costs 2.64 us (heat) / 2.8-3.0 us
+    // (Gray-Scott) whatever the size; here (us per step, 100 steps): heat 36 chunks 1.15, 122 1.56, 219 2.07,
+    // 301 2.93, 391 3.22; Gray-Scott 36 chunks 1.66, 122 2.36, 174 2.97, 219 3.50.
+    if (g->n > (np == 1 ? 16 : 10) * kSolveCtas || nsteps > (1 << 20)) return SGB_ENOTSUP;
     const GridInfo gi = grid_info_of(fwd);
     const uint8_t* mask = g->mask.as<uint8_t>();
     const int32_t* nn = g->nn[SGB_NN_STAR].as<int32_t>();

@@ -413,8 +413,8 @@ int launch_fields(const LaunchDesc& L, cudaStream_t s) {
 // its last use.
 static bool cleans_sources(const sgb_grid* g) { return g->geo.edge == 4 || g->geo.zorder; }
 
-// step: -1 for a call of one step; else the step's number in run_steps, which has cleaned the properties.  Steps
-// before `refills` write the backgrounds of an exposed destination.
+// step: -1 for a call of one step; else the step's number in run_steps, which has the tables and the properties in
+// order.  Steps before `refills` write the backgrounds of an exposed destination.
 static int launch_stencil(sgb_grid* g, int kind, const int* src, const int* dst, const StencilParams& prm,
                           cudaStream_t s, int step, int refills, bool use_tile = false) {
     if (g->n == 0) return SGB_OK;
@@ -424,10 +424,11 @@ static int launch_stencil(sgb_grid* g, int kind, const int* src, const int* dst,
         if (st != SGB_ENOTSUP) return st;
     }
     const int nnk = kind == SGB_BOX27 ? SGB_NN_FULL : SGB_NN_STAR;
-    SGB_TRY(ensure_neighbours(g, nnk, s));
     const int np = kind == SGB_GS7 ? 2 : 1;
-    // (the tile kernel tests the masks itself)
-    SGB_TRY(ensure_clean_f32(g, src, np, step < 0 && kind != SGB_BOX27 && !use_tile && cleans_sources(g), s));
+    if (step < 0) {  // (the tile kernel tests the masks itself)
+        SGB_TRY(ensure_neighbours(g, nnk, s));
+        SGB_TRY(ensure_clean_f32(g, src, np, kind != SGB_BOX27 && !use_tile && cleans_sources(g), s));
+    }
     LaunchDesc L;
     std::memset(&L, 0, sizeof(L));
     L.kind = kind;
@@ -505,7 +506,7 @@ int sgb_run_steps(sgb_grid* g, int kind, const int* src, const int* dst, const f
     for (int j = 0; j < 2 * np; ++j) exposed |= g->exposed[props[j]];
     // a small grid: all steps in one launch
     {
-        const int st = run_steps_cluster(g, kind, src, dst, fwd, nsteps, exposed, s);
+        const int st = run_steps_one_launch(g, kind, src, dst, fwd, nsteps, exposed, s);
         if (st == SGB_OK) {
             if (kind == SGB_HEAT7) g->clean[nsteps % 2 ? dst[0] : src[0]] = true;
             return SGB_OK;

@@ -88,7 +88,7 @@ int launch_fields(const LaunchDesc& L, cudaStream_t s);
 int launch_star7(const LaunchDesc& L, cudaStream_t s);  // 7-point kernels, any chunk ids (star7.cu)
 // All steps of a small grid's solve in one launch (solve.cu); SGB_ENOTSUP: not for this grid.
 // again: points that do not exist may hold anything (the caller kept a pointer).
-int run_steps_cluster(sgb_grid* g, int kind, const int* src, const int* dst, const StencilParams& fwd, int nsteps,
+int run_steps_one_launch(sgb_grid* g, int kind, const int* src, const int* dst, const StencilParams& fwd, int nsteps,
                       bool again, cudaStream_t s);
 GridInfo grid_info_of(const StencilParams& prm);
 

@@ -95,6 +95,26 @@ def test_solve_in_one_launch_equals_steps(sgb, kind, nchunks):
             assert torch.equal(x.view(torch.int32), w.view(torch.int32))
 
 
+@pytest.mark.parametrize("per_sm,more", [(0, 1), (0, 8), (0, 9), (1, 0), (1, 1), (3, 0), (3, 1)])
+@pytest.mark.parametrize("kind,lin", [("HEAT7", "smb"), ("GS7", "smb"), ("GS7", "zmb")])
+def test_solve_of_4_chunks_equals_steps(sgb, kind, lin, per_sm, more):
+    """run_steps on 4^3 chunks, both sides of the limits in chunks and steps, against steps of the tile kernel."""
+    prm = [0.1] if kind == "HEAT7" else [0.16, 0.08, 0.035, 0.065, 1.0]
+    a, b = ([0], [2]) if kind == "HEAT7" else ([0, 1], [2, 3])
+    nchunks = per_sm * torch.cuda.get_device_properties(0).multi_processor_count + more
+    for nsteps in (2, 3, 4, 8, 9):
+        g, h = (_grid(sgb, (40, 33, 38), nchunks, lin, 13, density=0.9, e=4) for _ in range(2))
+        fin = g.run_steps(getattr(sgb, kind), a, b, prm, nsteps)
+        for k in range(nsteps):
+            h.applyStencils(getattr(sgb, kind), a if k % 2 == 0 else b, b if k % 2 == 0 else a, prm, tiled=True)
+        assert fin == (nsteps % 2 == 1)
+        g.check_device_errors()
+        ex = (g.private_get_mask_array() & 1).bool()
+        for q in a + b:
+            x, w = g.private_get_data_array(q)[ex], h.private_get_data_array(q)[ex]
+            assert torch.equal(x.view(torch.int32), w.view(torch.int32))
+
+
 @pytest.mark.parametrize("use_graph", [True, False])
 @pytest.mark.parametrize("kind", ["HEAT7", "GS7"])
 def test_batch_stepped_past_its_slots(sgb, kind, use_graph):
