@@ -70,8 +70,10 @@ __global__ void k_scan_tiles(const uint32_t* in, int64_t n, const uint32_t* offs
 }
 
 // Short arrays: one CTA walks them, 16384 items a round (three launches of a few CTAs each cost 10.5 us for 19 K
-// items, this 8.1 us).  VEC: 16-byte accesses, for 16-byte aligned arrays.
-constexpr int64_t kScanOneMax = 65536;
+// items, this 8.1 us).  VEC: 16-byte accesses, for 16-byte aligned arrays.  At both ends the other kernels are the
+// faster ones (the point list of n chunks in us, with a tile's CTA / this / three launches): 512 chunks 38 / 41 / -,
+// 1024 40 / 39 / -, 4096 - / 40 / 45, 32768 - / 51 / 50, 46656 - / 57 / 58, 65536 - / 74 / 68.
+constexpr int64_t kScanOneMin = 512, kScanOneMax = 49152;
 constexpr int kScanOneItems = 16;
 template <bool VEC>
 __global__ void __launch_bounds__(1024) k_scan_one(const uint32_t* __restrict__ in, int64_t n, uint32_t* __restrict__ out,
@@ -139,6 +141,11 @@ int scan_exclusive_u32(const uint32_t* in, uint32_t* out, int64_t n, uint32_t* t
                        cudaStream_t s) {
     if (n <= 0) {
         if (total_dev) SGB_CUDA(cudaMemsetAsync(total_dev, 0, 4, s));
+        return SGB_OK;
+    }
+    if (n <= kScanOneMin) {
+        k_scan_tiles<<<1, kScanThreads, 0, s>>>(in, n, nullptr, out, total_dev);
+        SGB_CUDA(cudaGetLastError());
         return SGB_OK;
     }
     if (n <= kScanOneMax) {

@@ -41,3 +41,18 @@ def test_point_list_on_another_stream(sgb, other):
     torch.cuda.synchronize()
     for a, m in zip(lists, want):
         assert torch.equal(a, m.nonzero().squeeze(1))
+
+
+@pytest.mark.parametrize("n", [1, 511, 512, 513, 16384, 16385, 49151, 49152, 49153])
+def test_point_offsets_at_the_limits_of_the_prefix_sums(sgb, n):
+    """First existing point of every chunk, and the list made from it, for chunk counts at which the prefix sum
+    changes its kernel or takes another round."""
+    g = sgb.SparseGridGpu((8 * n, 8, 8), ["u8"], edge=8)
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(n)
+    m = (torch.rand(n * 512, generator=gen, device="cuda") < 0.02).to(torch.uint8)
+    g.load_map_dev(torch.arange(n, device="cuda"), [m], m)
+    per = m.reshape(n, 512).sum(dim=1)
+    want = torch.cat([torch.zeros(1, dtype=torch.int64, device="cuda"), per.cumsum(0)])
+    assert torch.equal(g.existing_offsets(), want)
+    assert torch.equal(g.existing_point_list(), m.nonzero().squeeze(1))
