@@ -20,7 +20,7 @@ def sgb():
 
 
 PRM = {"HEAT7": [0.1], "GS7": [0.16, 0.08, 0.035, 0.065, 1.0]}
-GRIDS = [(8, "smb", (75, 50, 61), 200), (8, "smb", (100, 99, 75), 900), (8, "zmb", (64, 64, 64), 300),
+GRIDS = [(8, "smb", (75, 50, 61), 100), (8, "smb", (75, 50, 61), 200), (8, "smb", (100, 99, 75), 900), (8, "zmb", (64, 64, 64), 300),
          (4, "smb", (64, 60, 52), 700), (4, "zmb", (64, 64, 64), 30)]
 
 

@@ -75,7 +75,7 @@ def test_star7_eight_slices_by_size(sgb):
     g.check_device_errors()
 
 
-@pytest.mark.parametrize("nchunks", [1, 2, 5, 17, 33, 160, 161, 256, 257])
+@pytest.mark.parametrize("nchunks", [1, 2, 5, 17, 33, 144, 145, 160, 161, 256, 257])
 @pytest.mark.parametrize("kind", ["HEAT7", "GS7"])
 def test_solve_in_one_launch_equals_steps(sgb, kind, nchunks):
     """run_steps of a small grid (both sides of the size limit) against single steps of the tile kernel."""
