@@ -625,7 +625,12 @@ __global__ void k_scatter(const uint2* __restrict__ upt, int64_t nu, int bs_shif
 // Up to 8192 staged points: one CTA sorts them in shared memory (digits of at most 8 bits, eight items per thread),
 // folds the points' inserts, looks the touched chunks up and, when none of them is new, writes the results back --
 // what the kernels above do in 14 launches of a few CTAs, each bound by its launch and memory latency.  (5003
-// points into a 128^3 map, whole call: 123 us with those, 92 us so.)
+// points into a 128^3 map, whole call: 123 us with those, 92 us so.)  The limit is what the CTA's shared memory holds;
+// the kernels above are as fast from fewer points on when many properties are listed, since one CTA folds and writes
+// them all.  Insert and flush in us, here / by those kernels, points in existing chunks and in new ones: 1 property
+// 8192 points 86 / 103 and 89 / 117; 3 properties 5120 points 102 / 111 and 99 / 129, 8192 points 129 / 111 and
+// 114 / 129; 6 properties 4096 points 128 / 123 and 118 / 147, 8192 points 188 / 124 and 154 / 146 (8^3 chunks; 4^3
+// chunks and 64-bit ids within 15 %).
 constexpr int kSmThreads = 1024, kSmItems = 8, kSmMax = kSmThreads * kSmItems, kSmBuckets = 256;
 
 template <typename K>

@@ -1,5 +1,6 @@
-"""Flush at the sizes where its kernels' tiles end: 2048 items (segment heads), 4096 keys (sort), 1024 touched
-chunks (lookup), against the CPU oracle; block maps, masks and values are exact."""
+"""Flush at the sizes where its kernels change or their tiles end, against the CPU oracle; block maps, masks and values
+are exact.  One launch takes up to 8192 points; above, the sort's tiles hold 1024 keys, 4096 past 4096 points per SM,
+and the heads' and lookup's tiles 1024 points and chunks.  Ids above 32 bits have kernels of their own."""
 import numpy as np
 import pytest
 import torch
@@ -17,7 +18,7 @@ def sgb():
 
 
 @pytest.mark.parametrize("edge", [8, 4])
-@pytest.mark.parametrize("n", [1, 31, 2047, 2048, 2049, 4096, 4097, 12289, 70000])
+@pytest.mark.parametrize("n", [1, 31, 1023, 1024, 1025, 2047, 2048, 2049, 4096, 4097, 8191, 8192, 8193, 9215, 9216, 9217, 12289, 70000])
 @pytest.mark.parametrize("spread", [6, 120])
 def test_flush_sizes(sgb, edge, n, spread):
     """n inserts with duplicates in a small or large part of the domain, then as many again (merge into the map).
@@ -41,6 +42,49 @@ def test_flush_sizes(sgb, edge, n, spread):
     ex = (mask & 1).astype(bool)
     for a, b in zip(data, odata):
         assert np.array_equal(a[ex], np.asarray(b)[ex])
+
+
+def _one_property(sgb, size, edge, rounds, rng):
+    g = sgb.SparseGridGpu(size, ["f32"], edge=edge)
+    o = O.OracleGrid(size, edge=edge, ptypes=[O.T_F32])
+    for pts in rounds:
+        v = rng.standard_normal(len(pts)).astype(np.float32)
+        g.insert(torch.from_numpy(pts.astype(np.int32)).cuda(), [torch.from_numpy(v).cuda()])
+        g.flush(["sLeft_"])
+        o.insert_flush(pts, [v], [O.OP_LEFT])
+    keys, data, mask = g.deviceToHost()
+    okeys, odata, omask = o.export()
+    assert np.array_equal(keys, okeys) and np.array_equal(mask, omask)
+    ex = (mask & 1).astype(bool)
+    assert np.array_equal(data[0][ex], np.asarray(odata[0])[ex])
+
+
+@pytest.mark.parametrize("n", [8191, 8192, 8193])
+@pytest.mark.parametrize("spread", [20, 125])
+def test_flush_at_the_limit_of_one_launch(sgb, n, spread):
+    rng = np.random.default_rng(n + spread)
+    _one_property(sgb, (130, 121, 125), 8, [rng.integers(0, [min(spread, s) for s in (130, 121, 125)], size=(n, 3)) for _ in range(3)], rng)
+
+
+@pytest.mark.parametrize("more", [0, 1])
+def test_flush_at_the_limit_of_small_sort_tiles(sgb, more):
+    rng = np.random.default_rng(more)
+    n = torch.cuda.get_device_properties(0).multi_processor_count * 4096 + more
+    _one_property(sgb, (130, 121, 125), 8, [rng.integers(0, 121, size=(n, 3)), rng.integers(0, 121, size=(5000, 3))], rng)
+
+
+@pytest.mark.parametrize("edge", [8, 4])
+@pytest.mark.parametrize("n", [1, 3000, 8192, 8193, 700000])
+def test_flush_with_ids_above_32_bits(sgb, edge, n):
+    """A 2000^3 domain: points at both ends of it, so that ids below and above 2^32 are sorted together."""
+    rng = np.random.default_rng(n + edge)
+    size = np.array([2000, 1990, 2010])
+    rounds = []
+    for _ in range(2):
+        p = rng.integers(0, 90, size=(n, 3))
+        p[n // 2:] += size - 90
+        rounds.append(p[rng.permutation(n)])
+    _one_property(sgb, tuple(int(v) for v in size), edge, rounds, rng)
 
 
 @pytest.mark.parametrize("n,distinct", [(5, 1), (8192, 1), (8192, 3), (8193, 1), (20001, 1), (33000, 6)])
