@@ -110,9 +110,8 @@ int sgb_destroy(sgb_grid* g);
  * coordinate, SparseGridGpu_z, src/Grid/Geometry/grid_zmb.hpp:25-104,
  * src/SparseGridGpu/SparseGridGpu.hpp:3948-3960); offsets inside a chunk
  * are x fastest for both.  Chosen while the grid is empty; SGB_LIN_ZMB needs
- * 3-D and at most 2^21 blocks per dimension.  Stencils on Morton grids run
- * the one-chunk-per-CTA kernel; batches and the scene builder take
- * SGB_LIN_SMB grids only. */
+ * 3-D and at most 2^21 blocks per dimension.  Stencils run the same kernels
+ * on both; batches and the scene builder take SGB_LIN_SMB grids only. */
 typedef enum { SGB_LIN_SMB = 0, SGB_LIN_ZMB = 1 } sgb_linearizer;
 int sgb_set_linearizer(sgb_grid* g, int kind);
 
@@ -124,9 +123,9 @@ int sgb_set_linearizer(sgb_grid* g, int kind);
 int sgb_release_scratch(sgb_grid* g);
 
 /* Self-check of failure detection (no reference counterpart): runs the
- * library's two kinds of bounded wait -- on an mbarrier phase and on an
- * arrival counter -- on conditions nothing satisfies, with a limit of
- * limit_ns (at most 1 s).  Returns SGB_ETIMEOUT when both gave up as they
+ * bounded wait of the library's one kernel that has one -- on an arrival
+ * counter -- and one on an mbarrier phase, on conditions nothing satisfies,
+ * with a limit of limit_ns (at most 1 s).  Returns SGB_ETIMEOUT when both gave up as they
  * should, with the device still usable. */
 int sgb_probe_bounded_waits(int64_t limit_ns, int device, sgb_stream s);
 

@@ -1,5 +1,5 @@
-// Batched form: many independent grids advanced by one persistent launch per
-// step over their concatenated block maps.  No reference counterpart (the
+// Batched form: many independent grids advanced by one launch per step
+// over their concatenated block maps.  No reference counterpart (the
 // reference launches one applyStencils per grid,
 // src/SparseGridGpu/SparseGridGpu.hpp:2704-2734).
 //
@@ -37,7 +37,6 @@ struct sgb_batch {
     bool dirty = true;     // grids table must be uploaded
     bool holes = false;    // removed slots to compact
     int num_sms = 148, ctas_per_sm = 0, stages = 0;  // 0: automatic
-    sgb::DevBuf err;
     // the instantiated graph of the last sgb_batch_step call with use_graph, updated in place for the
     // next call of the same step count (kernel arguments change, the graph's shape does not)
     cudaGraphExec_t exec = nullptr;
@@ -200,12 +199,10 @@ static int batch_launch(sgb_batch* b, int64_t t, cudaStream_t s, bool chained) {
     L.gid = b->gid.as<int32_t>();
     L.grids = b->grids.as<GridInfo>();
     L.n = b->n;
-    L.arr_chunks = b->n;
     L.geo.edge = b->edge;
     L.geo.bs = b->edge * b->edge * b->edge;
     L.t = t;
     L.chained = chained;
-    L.err = b->err.as<unsigned>();
     return launch_fields(L, s);
 }
 
@@ -222,10 +219,6 @@ int sgb_batch_create(sgb_batch** out, int device) {
     sgb_batch* b = new sgb_batch();
     b->device = device;
     cudaDeviceGetAttribute(&b->num_sms, cudaDevAttrMultiProcessorCount, device);
-    if (b->err.ensure(16) != SGB_OK || cudaMemset(b->err.p, 0, 16) != cudaSuccess) {
-        delete b;
-        return SGB_ENOMEM;
-    }
     *out = b;
     return SGB_OK;
 }
@@ -241,7 +234,7 @@ int sgb_batch_destroy(sgb_batch* b) {
         }
         if (b->grids_host[k]) cudaFreeHost(b->grids_host[k]);
     }
-    for (DevBuf* d : {&b->keys, &b->mask, &b->nn, &b->gid, &b->grids, &b->keys2, &b->mask2, &b->nn2, &b->gid2, &b->err})
+    for (DevBuf* d : {&b->keys, &b->mask, &b->nn, &b->gid, &b->grids, &b->keys2, &b->mask2, &b->nn2, &b->gid2})
         d->release();
     for (int k = 0; k < 2; ++k)
         for (int p = 0; p < 2; ++p) {

@@ -1,17 +1,52 @@
 // Self-check of the bounded waits (failure detection without a GPU fault).
 //
-// Every wait in the library's kernels is bounded: on an mbarrier phase
-// (mbar_wait_bounded) and on the grid barrier of the one-launch multi-step
-// kernel (an arrival counter watched against the global timer).  When the
-// limit passes, the kernel raises kErrWaitTimeout in the grid's error word
-// and returns, and the host reports SGB_ETIMEOUT with the context intact.
-// This entry point runs both kinds of wait on conditions that nothing ever
-// satisfies (an mbarrier phase with no arrivals, a counter nobody
-// increments), each with a short limit, so a test can see that path work.
+// A wait in a kernel of this library has a limit; when it passes, the kernel
+// raises kErrWaitTimeout in the grid's error word and returns, and the host
+// reports SGB_ETIMEOUT with the context intact.  The one such wait is the grid
+// barrier of the small-solve kernel for 4^3 chunks (counter_wait_bounded);
+// everything else is ordered by hardware cluster barriers, CTA barriers and
+// launches.  This entry point runs that wait, and one on an mbarrier phase, on
+// conditions that nothing ever satisfies (a counter nobody increments, a phase
+// with no arrivals), each with a short limit, so a test can see the path work.
 #include "common.cuh"
 #include "internal.h"
 
 namespace sgb {
+
+__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
+}
+
+__device__ __forceinline__ void mbar_fence_init() {
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+}
+
+__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+
+// Bounded wait on an mbarrier phase: gives up after about `limit_ns`
+// nanoseconds, raises kErrWaitTimeout in *err and returns false.
+__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, unsigned* err,
+                                                  uint64_t limit_ns = 2000000000ull) {
+    if (mbar_try_wait(bar, parity)) return true;
+    const uint64_t t0 = global_timer_ns();
+    for (uint32_t it = 0;; ++it) {
+        if (mbar_try_wait(bar, parity)) return true;
+        if ((it & 63u) == 63u && global_timer_ns() - t0 > limit_ns) {
+            atomicOr(err, kErrWaitTimeout);
+            return false;
+        }
+    }
+}
 
 __global__ void k_probe_waits(uint64_t limit_ns, unsigned* err, unsigned* counter) {
     __shared__ uint64_t bar;
@@ -21,14 +56,7 @@ __global__ void k_probe_waits(uint64_t limit_ns, unsigned* err, unsigned* counte
     // phase 0 never completes: nobody arrives
     mbar_wait_bounded(&bar, 0, err, limit_ns);
     // the counter stays 0: nobody increments it
-    const uint64_t t0 = global_timer_ns();
-    for (uint32_t it = 0;; ++it) {
-        if (*reinterpret_cast<volatile unsigned*>(counter) >= 1u) break;
-        if ((it & 63u) == 63u && global_timer_ns() - t0 > limit_ns) {
-            atomicOr(err, kErrWaitTimeout);
-            break;
-        }
-    }
+    counter_wait_bounded(counter, 1u, err, limit_ns);
 }
 
 }  // namespace sgb

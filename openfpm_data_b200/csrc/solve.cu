@@ -272,16 +272,7 @@ __global__ void __launch_bounds__(256) k_steps_coop4(FieldSet fs, const uint8_t*
             if (threadIdx.x == 0) {
                 __threadfence();
                 atomicAdd(bar, 1u);
-                const unsigned target = (unsigned)(t + 1) * gridDim.x;
-                const uint64_t t0 = global_timer_ns();
-                for (uint32_t it = 0;; ++it) {
-                    if (*reinterpret_cast<volatile unsigned*>(bar) >= target) break;
-                    if ((it & 63u) == 63u && global_timer_ns() - t0 > 2000000000ull) {
-                        atomicOr(err, kErrWaitTimeout);
-                        abort_run = 1;
-                        break;
-                    }
-                }
+                if (!counter_wait_bounded(bar, (unsigned)(t + 1) * gridDim.x, err)) abort_run = 1;
                 __threadfence();
             }
             __syncthreads();

@@ -449,14 +449,12 @@ static int launch_stencil(sgb_grid* g, int kind, const int* src, const int* dst,
     L.grids = nullptr;
     L.g0 = grid_info_of(prm);
     L.n = g->n;
-    L.arr_chunks = g->n + 1;
     L.geo = g->geo;
     L.prm = prm;
     L.t = 0;
     L.chained = step > 0;
     L.fill = (step < refills && (g->exposed[dst[0]] || g->exposed[dst[np - 1]])) ||
              (kind == SGB_HEAT7 && !g->clean[dst[0]]);
-    L.err = g->err.as<unsigned>();
     SGB_TRY(launch_fields(L, s));
     if (kind == SGB_HEAT7) g->clean[dst[0]] = true;  // every point of dst was written from the tile
     return SGB_OK;

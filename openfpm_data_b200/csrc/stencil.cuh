@@ -75,13 +75,11 @@ struct LaunchDesc {
     const GridInfo* grids;   // per grid entries (NULL: single grid g0)
     GridInfo g0;
     int64_t n;
-    int64_t arr_chunks;      // chunks held by the field arrays (n + background chunk for grids)
     Geometry geo;
     StencilParams prm;
     int64_t t;
     int fill;                // quads without an existing point are written too (dst may hold anything there)
     int chained;             // follows a launch over the same masks and neighbours in the same call
-    unsigned* err;
 };
 
 int launch_fields(const LaunchDesc& L, cudaStream_t s);
