@@ -280,7 +280,9 @@ int sgb_batch_add(sgb_batch* b, sgb_grid* g, int kind, const int* src, const int
     SGB_TRY(ensure_neighbours(g, SGB_NN_STAR, s));
     {  // batched kernels rely on background-filled empty points
         const int props[4] = {src[0], dst[0], src[b->np - 1], dst[b->np - 1]};
-        SGB_TRY(ensure_clean_f32(g, props, 2 * b->np, true, s));
+        bool again = false;
+        for (int k = 0; k < 2 * b->np; ++k) again |= g->exposed[props[k]];
+        SGB_TRY(ensure_clean_f32(g, props, 2 * b->np, again, s));
     }
     const int bs = g->geo.bs;
     SGB_TRY(batch_reserve(b, b->n + g->n));

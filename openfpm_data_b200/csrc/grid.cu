@@ -386,7 +386,7 @@ int ensure_clean_f32(sgb_grid* g, const int* props, int count, bool again, cudaS
     CleanSet cs{};
     for (int k = 0; k < count; ++k) {
         const int p = props[k];
-        if (g->clean[p] && !(again && g->exposed[p])) continue;
+        if (g->clean[p] && !again) continue;
         cs.data[cs.count] = g->data[p].as<float>();
         std::memcpy(&cs.bck[cs.count++], g->bck[p], 4);
         g->clean[p] = true;

@@ -47,6 +47,11 @@ inline int allow_max_smem(Kernel kern) {
     return SGB_OK;
 }
 
+inline bool is_capturing(cudaStream_t s) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(s, &st) == cudaSuccess && st == cudaStreamCaptureStatusActive;
+}
+
 // Makes `dev` the current device for the lifetime of the guard and gives the
 // caller's current device back on every return path, so an entry point that
 // works on a grid of another GPU leaves the caller's CUDA state as it was.
@@ -356,7 +361,7 @@ int sanitize_prop(sgb_grid* g, int p, cudaStream_t s);
 // fill every point (n + 1 chunks) of property p with its background
 int fill_background_all(sgb_grid* g, int p, cudaStream_t s);
 int ensure_clean(sgb_grid* g, int p, cudaStream_t s);
-// the same for up to four float32 properties in one launch; again: also those that are exposed
+// the same for up to four float32 properties in one launch; again: whether or not they count as clean
 int ensure_clean_f32(sgb_grid* g, const int* props, int count, bool again, cudaStream_t s);
 // fill count elements of esize bytes with the low esize bytes of pattern
 int fill(void* dst, int64_t count, int esize, uint64_t pattern, cudaStream_t s);

@@ -288,6 +288,7 @@ static int run_steps_coop4(sgb_grid* g, int kind, const FieldSet& fields, const 
     const int64_t sms = g->num_sms;
     if (!(g->n <= 8 || (g->n <= sms && nsteps <= 8) || (g->n <= 3 * sms && nsteps <= 3))) return SGB_ENOTSUP;
     if ((int64_t)nsteps * g->n >= (int64_t(1) << 31)) return SGB_ENOTSUP;  // arrival counter range
+    if (is_capturing(s)) return SGB_ENOTSUP;  // the counter is allocated by the first call
     FieldSet fs = fields;
     GridInfo gi = grid_info_of(fwd);
     const uint8_t* mask = g->mask.as<uint8_t>();

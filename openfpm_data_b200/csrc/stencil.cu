@@ -413,10 +413,18 @@ int launch_fields(const LaunchDesc& L, cudaStream_t s) {
 // its last use.
 static bool cleans_sources(const sgb_grid* g) { return g->geo.edge == 4 || g->geo.zorder; }
 
+// May a caller write one of these properties, through a pointer, between this call and its steps?  It may if it has
+// had one; and a captured step runs again and again, with pointers that are taken later.
+static bool may_be_written(const sgb_grid* g, const int* props, int count, cudaStream_t s) {
+    for (int k = 0; k < count; ++k)
+        if (g->exposed[props[k]]) return true;
+    return is_capturing(s);
+}
+
 // step: -1 for a call of one step; else the step's number in run_steps, which has the tables and the properties in
-// order.  Steps before `refills` write the backgrounds of an exposed destination.
+// order.  refill: the step writes the backgrounds of its destination.
 static int launch_stencil(sgb_grid* g, int kind, const int* src, const int* dst, const StencilParams& prm,
-                          cudaStream_t s, int step, int refills, bool use_tile = false) {
+                          cudaStream_t s, int step, bool refill, bool use_tile = false) {
     if (g->n == 0) return SGB_OK;
     if (kind == SGB_BOX27_NS) return launch_points_box27(g, src, dst, prm, s);
     if (kind == SGB_BOX27 && !use_tile) {  // sparse chunks: the point list
@@ -427,7 +435,9 @@ static int launch_stencil(sgb_grid* g, int kind, const int* src, const int* dst,
     const int np = kind == SGB_GS7 ? 2 : 1;
     if (step < 0) {  // (the tile kernel tests the masks itself)
         SGB_TRY(ensure_neighbours(g, nnk, s));
-        SGB_TRY(ensure_clean_f32(g, src, np, kind != SGB_BOX27 && !use_tile && cleans_sources(g), s));
+        const bool star = kind != SGB_BOX27 && !use_tile;
+        SGB_TRY(ensure_clean_f32(g, src, np, star && cleans_sources(g) && may_be_written(g, src, np, s), s));
+        refill = star && may_be_written(g, dst, np, s);
     }
     LaunchDesc L;
     std::memset(&L, 0, sizeof(L));
@@ -453,8 +463,7 @@ static int launch_stencil(sgb_grid* g, int kind, const int* src, const int* dst,
     L.prm = prm;
     L.t = 0;
     L.chained = step > 0;
-    L.fill = (step < refills && (g->exposed[dst[0]] || g->exposed[dst[np - 1]])) ||
-             (kind == SGB_HEAT7 && !g->clean[dst[0]]);
+    L.fill = refill || (kind == SGB_HEAT7 && !g->clean[dst[0]]);
     SGB_TRY(launch_fields(L, s));
     if (kind == SGB_HEAT7) g->clean[dst[0]] = true;  // every point of dst was written from the tile
     return SGB_OK;
@@ -471,7 +480,7 @@ int sgb_apply_stencil(sgb_grid* g, int kind, const int* src, const int* dst, con
     if (!g) return SGB_EINVAL;
     StencilParams prm;
     SGB_TRY(make_params(g, kind, src, dst, params, nparams, box, prm));
-    return launch_stencil(g, kind, src, dst, prm, (cudaStream_t)s, -1, 0);
+    return launch_stencil(g, kind, src, dst, prm, (cudaStream_t)s, -1, false);
 }
 
 // Same as sgb_apply_stencil through the generic one-chunk-per-CTA kernel
@@ -481,7 +490,7 @@ int sgb_apply_stencil_tiled(sgb_grid* g, int kind, const int* src, const int* ds
     if (!g) return SGB_EINVAL;
     StencilParams prm;
     SGB_TRY(make_params(g, kind, src, dst, params, nparams, box, prm));
-    return launch_stencil(g, kind, src, dst, prm, (cudaStream_t)s, -1, 0, true);
+    return launch_stencil(g, kind, src, dst, prm, (cudaStream_t)s, -1, false, true);
 }
 
 int sgb_run_steps(sgb_grid* g, int kind, const int* src, const int* dst, const float* params, int nparams, int nsteps,
@@ -500,11 +509,10 @@ int sgb_run_steps(sgb_grid* g, int kind, const int* src, const int* dst, const f
     const int props[4] = {src[0], dst[0], src[np - 1], dst[np - 1]};
     SGB_TRY(ensure_clean_f32(g, props, 2 * np, false, s));
     const bool star = kind == SGB_HEAT7 || kind == SGB_GS7;
-    bool exposed = false;
-    for (int j = 0; j < 2 * np; ++j) exposed |= g->exposed[props[j]];
+    const bool written = star && may_be_written(g, props, 2 * np, s);
     // a small grid: all steps in one launch
     {
-        const int st = run_steps_one_launch(g, kind, src, dst, fwd, nsteps, exposed, s);
+        const int st = run_steps_one_launch(g, kind, src, dst, fwd, nsteps, written, s);
         if (st == SGB_OK) {
             if (kind == SGB_HEAT7) g->clean[nsteps % 2 ? dst[0] : src[0]] = true;
             return SGB_OK;
@@ -516,15 +524,15 @@ int sgb_run_steps(sgb_grid* g, int kind, const int* src, const int* dst, const f
     // a launch takes about 2 us beside the step before it.  use_graph also asks for the wait at the end, which
     // 7-point solves of at most 4 chunks per SM do without, so that their next call's launches overlap.
     const bool small = star && g->n <= (int64_t)g->num_sms * 4 && nsteps >= 2;
-    int refills = 2;  // each half of the ping-pong once
-    if (star && (small || cleans_sources(g))) {
+    int refills = written ? 2 : 0;  // each half of the ping-pong once
+    if (written && (small || cleans_sources(g))) {
         // heat's first step puts the destination in order; Gray-Scott's leaves x quads with padding points alone
         SGB_TRY(ensure_clean_f32(g, props, kind == SGB_HEAT7 ? 1 : 4, true, s));
         refills = kind == SGB_HEAT7 ? 1 : 0;
     }
     for (int k = 0; k < nsteps; ++k) {
-        if (k % 2 == 0) SGB_TRY(launch_stencil(g, kind, src, dst, fwd, s, k, refills));
-        else SGB_TRY(launch_stencil(g, kind, dst, src, bwd, s, k, refills));
+        if (k % 2 == 0) SGB_TRY(launch_stencil(g, kind, src, dst, fwd, s, k, k < refills));
+        else SGB_TRY(launch_stencil(g, kind, dst, src, bwd, s, k, k < refills));
     }
     if (use_graph && !small) SGB_CUDA(cudaStreamSynchronize(s));
     return SGB_OK;

@@ -124,3 +124,37 @@ def test_points_taken_out_through_a_kept_mask(sgb, kind, e, lin, size, n):
     h.applyStencils(getattr(sgb, kind), b, a, PRM[kind], tiled=True)
     h.applyStencils(getattr(sgb, kind), a, b, PRM[kind], tiled=True)
     _same(g, h, a + b)
+
+
+@pytest.mark.parametrize("kind", ["HEAT7", "GS7"])
+@pytest.mark.parametrize("e,lin,size,n", GRIDS)
+@pytest.mark.parametrize("how", ["steps", "run_steps"])
+def test_captured_before_the_view_was_taken(sgb, how, kind, e, lin, size, n):
+    """Two steps in a graph, captured while nobody has had a view of the grid, replayed after writes through one."""
+    g, h = (_grid(sgb, size, n, lin, 3, e=e) for _ in range(2))
+    if kind == "GS7":  # no padding points, and a map whose views nobody has had
+        keys, data, mask = h.deviceToHost()
+        for x in (g, h):
+            x.load_map(keys, [d[: n * x.bs] for d in data], mask[: n * x.bs] & 1)
+    a, b = _fields(kind)
+    graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    g.findNeighbours(sgb.NN_STAR)
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=side):
+        if how == "steps":
+            g.applyStencils(getattr(sgb, kind), a, b, PRM[kind])
+            g.applyStencils(getattr(sgb, kind), b, a, PRM[kind])
+        else:
+            g.run_steps(getattr(sgb, kind), a, b, PRM[kind], 2, use_graph=False)
+    graph.replay()
+    torch.cuda.synchronize()
+    views = [g.private_get_data_array(p) for p in range(4)]
+    gone = g.private_get_mask_array() == 0
+    gone[g.nchunks * g.bs:] = False
+    for p in b:
+        views[p].masked_fill_(gone, float("nan"))
+    graph.replay()
+    torch.cuda.synchronize()
+    _twin_steps(sgb, h, kind, a, b, 2)
+    _twin_steps(sgb, h, kind, a, b, 2)
+    _same(g, h, a + b)
