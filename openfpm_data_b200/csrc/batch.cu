@@ -431,7 +431,10 @@ int sgb_batch_extract(sgb_batch* b, int slot, sgb_grid* g, int* final_is_dst, sg
         }
     }
     const int64_t words = sl.n * bs / 4;
-    if (words > 0) {
+    if (g->device != b->device) {  // a grid on another GPU: copies, which need no peer mapping
+        for (int k = 0; k < cs.count; ++k)
+            SGB_CUDA(cudaMemcpyAsync(cs.dst[k], cs.src[k], (size_t)words * 16, cudaMemcpyDeviceToDevice, s));
+    } else if (words > 0) {
         k_copy_set<<<(unsigned)std::min<int64_t>((words + 255) / 256, (int64_t)b->num_sms * 8), 256, 0, s>>>(cs, words);
         SGB_CUDA(cudaGetLastError());
     }
