@@ -600,8 +600,8 @@ def served_shard(rate: float, seconds: float, rank: int, world: int):
 def run_batched256(args, dist: Dist):
     """256 heat grids of uneven size (edges log-uniform in [32, 384], one
     centred ball of radius 0.25-0.5 edge, seed 3), 200 steps per solve.
-    value: solves/s of the batched form (one persistent launch per step over
-    the concatenated block maps, each solve's 200 steps one CUDA graph) with
+    value: solves/s of the batched form (one launch per step over the
+    concatenated block maps, each solve's 200 steps one CUDA graph) with
     the autotuned launch; beside it the same solves with per-grid plain
     launches (one applyStencils per grid per step), with the reference's
     one-CTA-per-chunk execution model, and with one sgb_run_steps per grid."""

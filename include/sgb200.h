@@ -426,9 +426,9 @@ int sgb_device_bytes(const sgb_grid* g, int64_t* bytes);
 int sgb_set_launch_config(sgb_grid* g, int ctas_per_sm, int stages);
 
 /* ---------------------------------------------------------------- batches
- * Many independent grids advanced by one persistent launch per step over
- * their concatenated block maps (no reference counterpart: the reference
- * launches one applyStencils per grid).  All member grids share dim, edge,
+ * Many independent grids advanced by one launch per step over their
+ * concatenated block maps (no reference counterpart: the reference launches
+ * one applyStencils per grid).  All member grids share dim, edge,
  * property types and stencil kind; each keeps its own parameters and
  * background values. */
 int sgb_batch_create(sgb_batch** out, int device);
@@ -441,8 +441,8 @@ int sgb_batch_add(sgb_batch* b, sgb_grid* g, int kind, const int* src, const int
                   int nparams, int64_t nsteps, int* slot, sgb_stream s);
 /* Drop a slot; its chunks are compacted away before the next step. */
 int sgb_batch_remove(sgb_batch* b, int slot, sgb_stream s);
-/* Advance the batch by nsteps global steps: one persistent launch per step
- * over all chunks, captured as one CUDA graph when use_graph != 0.  The batch
+/* Advance the batch by nsteps global steps: one launch per step over all
+ * chunks, captured as one CUDA graph when use_graph != 0.  The batch
  * keeps the instantiated graph and updates it in place on the next call with
  * the same nsteps.  The call returns without waiting for the GPU: the steps
  * run on stream s in order with the batch's other calls on that stream. */

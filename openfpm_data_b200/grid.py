@@ -569,7 +569,7 @@ class SparseGridGpu:
 
 
 class Batch:
-    """Many grids advanced by one persistent launch per step (sgb_batch_*)."""
+    """Many grids advanced by one launch per step (sgb_batch_*)."""
 
     def __init__(self, device: int = 0):
         lib = L.load()

@@ -4,8 +4,8 @@ Requests (workloads.Request: kind, domain edge, balls, steps) arrive over
 time.  Each arrived request is admitted when its device footprint fits the
 HBM budget: its block map is built on the device (sgb_build_balls) in a
 pooled staging grid, copied into the resident batch of its kind and
-advanced together with every other admitted request by one persistent
-launch per step (sgb_batch_step).  Between quanta of steps, finished
+advanced together with every other admitted request by one launch per
+step (sgb_batch_step).  Between quanta of steps, finished
 requests are read back (their final fields: the response), removed from
 the batch and their memory returned to the budget.  Latency is measured
 from the request's arrival time to the end of its read-back.

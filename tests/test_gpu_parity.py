@@ -236,10 +236,9 @@ def test_heat_pipelined_equals_tiled(sgb):
 
 @pytest.mark.parametrize("box", [None, ((5, 9, 13), (60, 70, 50))])
 def test_gray_scott_pipelined_equals_tiled(sgb, box):
-    """The pipelined 8^3 kernel and the one-chunk-per-CTA kernel give the same
-    bits everywhere, existing points and the background-filled rest alike,
-    with padding points (tagBoundaries) and a box leaving existing points
-    untouched."""
+    """The 8^3 kernel and the one-chunk-per-CTA kernel give the same bits
+    everywhere, existing points and the background-filled rest alike, with
+    padding points (tagBoundaries) and a box leaving existing points untouched."""
     rng = np.random.default_rng(5)
     g1, _, _ = _sparse_grid(sgb, rng, (96, 80, 72), 8, 60000, ptypes=(O.T_F32,) * 4)
     keys, data, mask = g1.deviceToHost()
@@ -443,8 +442,9 @@ def test_existing_offsets_and_counts(sgb, edge):
 @pytest.mark.parametrize("kind", ["heat", "gs"])
 @pytest.mark.parametrize("nsteps", [2, 7, 64])
 def test_run_steps_small_grid_one_launch(sgb, edge, kind, nsteps):
-    """A small grid runs all steps in one cooperative launch: the result equals the
-    step-by-step applyStencils path bit for bit (ping-pong, distinct backgrounds)."""
+    """A small grid's run_steps, in one launch for all steps (8^3 chunks; 4^3 chunks at few
+    steps) or one per step: the result equals the step-by-step applyStencils path bit for
+    bit (ping-pong, distinct backgrounds)."""
     rng = np.random.default_rng(100 + edge + nsteps)
     size = (40, 36, 44) if edge == 8 else (24, 20, 28)
     pts = np.unique(rng.integers(0, size, size=(9000 if edge == 8 else 3000, 3)), axis=0).astype(np.int64)
