@@ -355,7 +355,7 @@ struct CleanSet {
 __global__ void __launch_bounds__(256) k_sanitize_f32(const uint32_t* __restrict__ mask, CleanSet cs, int64_t quads) {
     constexpr int R = 4;
     grid_dependency_wait();
-    grid_launch_dependents();  // the step behind this starts while it runs, and waits for it
+    grid_launch_dependents();  // a step behind this starts while it runs, and waits for it
     const int64_t q0 = blockIdx.x * (int64_t)(256 * R) + threadIdx.x;
     uint32_t m[R];
 #pragma unroll

@@ -321,7 +321,8 @@ struct sgb_grid {
     bool clean[sgb::kMaxProps] = {true, true, true, true, true, true, true, true};
     // exposed[p]: since the map's buffers were last exchanged (which ends the caller's pointers) the caller has had a
     // pointer that can write property p or the masks.  It may still write through it, so clean[p] stands for the call
-    // that established it and not for the next one: a step then writes the backgrounds of its destination again.
+    // that established it and not for the next one: a step then writes the backgrounds of its destination again, and
+    // some read their source through the masks (stencil.cu).
     bool exposed[sgb::kMaxProps] = {};
 
     // flush / scan / sort scratch

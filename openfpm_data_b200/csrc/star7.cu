@@ -23,6 +23,11 @@
 // HEAT7's stores keep), so a step moves about the bytes of the existing rows
 // and not of whole chunks.
 //
+// AGAIN: the source may hold anything at points that do not exist (a caller kept a pointer to it); each lane puts
+// the background into what it has copied or loaded, by the mask bytes.  A kernel of its own, for the first step of a
+// call: the tests in a uniform branch made the usual path a quarter slower (512^3 Gray-Scott, 50 steps, 1458 us,
+// 1813 so).  Heat on 16,384 Morton chunks 15.0 us a step, 12.8 without.
+//
 // What bounds it: HBM for large grids, where the power cap is reached with
 // it; latency and block turnover for one to four waves of blocks.  Measured
 // on one B200 (us per step, the earlier kernel, a ring of bulk copies per
@@ -63,7 +68,7 @@ struct StarTile {
     float row[NP][ZS][80];
 };
 
-template <int KIND, int NP, bool BOX, bool BATCH, int ZS, int MINB>
+template <int KIND, int NP, bool BOX, bool BATCH, bool AGAIN, int ZS, int MINB>
 __global__ void __launch_bounds__(kStarThreads, MINB)
     k_star7_e8(FieldSet fs, const uint8_t* __restrict__ mask, const int32_t* __restrict__ nn,
                BoxArgs<BOX> box, const int32_t* __restrict__ gid, const GridInfo* __restrict__ grids, GridInfo g0, int64_t n,
@@ -125,18 +130,23 @@ __global__ void __launch_bounds__(kStarThreads, MINB)
             else *reinterpret_cast<float4*>(d) = splat4(bs[p]);
         }
     // y faces: lanes 0..7 the -y side, 8..15 the +y side, quad xq of slice (l16 % 8) / 2 + 4 k
+    const int side = l16 >> 3, zq = (l16 & 7) >> 1;
+    uint32_t my[ZS / 4];  // AGAIN: their mask bytes
     {
-        const int side = l16 >> 3, zq = (l16 & 7) >> 1;
         const int32_t ny = side ? na.w : na.z;
 #pragma unroll
-        for (int z = zq; z < ZS; z += 4)
+        for (int k = 0; k < ZS / 4; ++k) {
+            const int z = zq + 4 * k;
+            const int64_t oy = (int64_t)ny * 512 + (zb + z) * 64 + (side ? 0 : 56) + xq * 4;
+            const bool there = live && ny >= 0;
+            my[k] = AGAIN && there ? ldm4(mask + oy) : 0x01010101u;
 #pragma unroll
             for (int p = 0; p < NP; ++p) {
                 float* d = &T.row[p][z][(side ? 72 : 0) + xq * 4];
-                if (live && ny >= 0)
-                    cp_async16(d, src[p] + (int64_t)ny * 512 + (zb + z) * 64 + (side ? 0 : 56) + xq * 4);
+                if (there) cp_async16(d, src[p] + oy);
                 else *reinterpret_cast<float4*>(d) = splat4(bs[p]);
             }
+        }
     }
     cp_async_commit();
     // the group `ahead` items on: its mask bytes and neighbour row on their way to L2 (3 % at 512^3)
@@ -163,15 +173,25 @@ __global__ void __launch_bounds__(kStarThreads, MINB)
     for (int p = 0; p < NP; ++p) {
         zm[p] = splat4(bs[p]);
         zl[p] = splat4(bs[p]);
-        if (m[0] && ozm >= 0) zm[p] = ldf4(src[p] + ozm);
-        if (m[ZS - 1] && ozp >= 0) zl[p] = ldf4(src[p] + ozp);
+        if (m[0] && ozm >= 0) {
+            zm[p] = ldf4(src[p] + ozm);
+            if constexpr (AGAIN) zm[p] = masked4(zm[p], ldm4(mask + ozm), bs[p]);
+        }
+        if (m[ZS - 1] && ozp >= 0) {
+            zl[p] = ldf4(src[p] + ozp);
+            if constexpr (AGAIN) zl[p] = masked4(zl[p], ldm4(mask + ozp), bs[p]);
+        }
     }
 #pragma unroll
     for (int z = 0; z < ZS; ++z)
 #pragma unroll
         for (int p = 0; p < NP; ++p) {
             xh[z][p] = bs[p];
-            if (m[z] && nx >= 0 && !in_cta) xh[z][p] = ldf1(src[p] + ox + z * 64);
+            if (m[z] && nx >= 0 && !in_cta) {
+                xh[z][p] = ldf1(src[p] + ox + z * 64);
+                if constexpr (AGAIN)
+                    if (!__ldg(mask + ox + z * 64)) xh[z][p] = bs[p];
+            }
         }
     int32_t cx = 0, cy = 0, cz = 0;
     if constexpr (BOX) {
@@ -185,6 +205,19 @@ __global__ void __launch_bounds__(kStarThreads, MINB)
 #pragma unroll
     for (int p = 0; p < NP; ++p) dst[p] = (par ? fs.out[1][p] : fs.out[0][p]) + oc;
     cp_async_wait_all();
+    if constexpr (AGAIN) {  // backgrounds into what this lane has copied
+        auto mend = [&](float* d, uint32_t m4, float b) {
+            if (m4 != 0x01010101u) *reinterpret_cast<float4*>(d) = masked4(*reinterpret_cast<const float4*>(d), m4, b);
+        };
+#pragma unroll
+        for (int p = 0; p < NP; ++p) {
+#pragma unroll
+            for (int z = 0; z < ZS; ++z)
+                if (m[z]) mend(&T.row[p][z][8 + o0], m[z], bs[p]);
+#pragma unroll
+            for (int k = 0; k < ZS / 4; ++k) mend(&T.row[p][zq + 4 * k][(side ? 72 : 0) + xq * 4], my[k], bs[p]);
+        }
+    }
     __syncthreads();
 #pragma unroll
     for (int p = 0; p < NP; ++p) cv[p] = *reinterpret_cast<const float4*>(&T.row[p][0][8 + o0]);
@@ -206,6 +239,7 @@ __global__ void __launch_bounds__(kStarThreads, MINB)
         if (m[z] || (fill && live)) {
             const uint32_t act = active_bits<BOX>(m[z], box, cx, cy, cz + z);
             star_store<KIND, NP>(cv, lap, m[z], act, gi, bd, dst[0] + z * 64, dst[NP - 1] + z * 64);
+            if (KIND == SGB_GS7 && fill > 1) star_rest<NP>(m[z], bd, dst[0] + z * 64, dst[NP - 1] + z * 64);
         }
 #pragma unroll
         for (int p = 0; p < NP; ++p) {
@@ -220,7 +254,7 @@ __global__ void __launch_bounds__(kStarThreads, MINB)
 // that the block's other lanes load).  The one-CTA-per-chunk gather that served these chunks before kept 64 of
 // 256 threads busy: Gray-Scott 250x190x131, 24,003 chunks and 1.33 M points, 65.7 us per step, now 6.46 (3.5
 // TB/s of the points' bytes; 4 to 8 blocks per SM run the same).  Bound by latency: two waves of blocks.
-template <int KIND, int NP, bool BOX, bool BATCH, int MINB>
+template <int KIND, int NP, bool BOX, bool BATCH, bool AGAIN, int MINB>
 __global__ void __launch_bounds__(kStarThreads, MINB)
     k_star7_e4(FieldSet fs, const uint8_t* __restrict__ mask, const int32_t* __restrict__ nn,
                BoxArgs<BOX> box, const int32_t* __restrict__ gid, const GridInfo* __restrict__ grids, GridInfo g0, int64_t n,
@@ -285,6 +319,15 @@ __global__ void __launch_bounds__(kStarThreads, MINB)
         if (ozp >= 0) zp[p] = ldf4(src + ozp);
         if (na.x >= 0) xm[p] = ldf1(src + oxm);
         if (na.y >= 0) xp[p] = ldf1(src + oxp);
+        if constexpr (AGAIN) {
+            cv[p] = masked4(cv[p], m, bs);
+            ym[p] = masked4(ym[p], oym >= 0 ? ldm4(mask + oym) : 0u, bs);
+            yp[p] = masked4(yp[p], oyp >= 0 ? ldm4(mask + oyp) : 0u, bs);
+            zm[p] = masked4(zm[p], ozm >= 0 ? ldm4(mask + ozm) : 0u, bs);
+            zp[p] = masked4(zp[p], ozp >= 0 ? ldm4(mask + ozp) : 0u, bs);
+            if (na.x >= 0 && !__ldg(mask + oxm)) xm[p] = bs;
+            if (na.y >= 0 && !__ldg(mask + oxp)) xp[p] = bs;
+        }
     }
 #pragma unroll
     for (int p = 0; p < NP; ++p) lap[p] = lap_quad<KIND>(cv[p], xm[p], xp[p], ym[p], yp[p], zm[p], zp[p]);
@@ -297,6 +340,7 @@ __global__ void __launch_bounds__(kStarThreads, MINB)
         cz = (int32_t)o[2] + z;
     }
     star_store<KIND, NP>(cv, lap, m, active_bits<BOX>(m, box, cx, cy, cz), gi, bd, dst[0], dst[NP - 1]);
+    if (KIND == SGB_GS7 && fill > 1) star_rest<NP>(m, bd, dst[0], dst[NP - 1]);
 }
 
 // Consecutive steps overlap one launch's ramp-up with the previous one's tail.
@@ -315,9 +359,9 @@ struct StarLaunch {
     }
 };
 
-template <int KIND, int NP, bool BOX, bool BATCH, int ZS, int MINB>
+template <int KIND, int NP, bool BOX, bool BATCH, bool AGAIN, int ZS, int MINB>
 static int launch_star(const LaunchDesc& L, cudaStream_t s) {
-    auto kern = k_star7_e8<KIND, NP, BOX, BATCH, ZS, MINB>;
+    auto kern = k_star7_e8<KIND, NP, BOX, BATCH, AGAIN, ZS, MINB>;
     const int64_t items = L.n * (8 / ZS);
     size_t smem = sizeof(StarTile<NP, ZS>) * kStarGroups;
     // a caller's limit on the CTAs per SM: each CTA takes its share of the SM's shared memory
@@ -333,24 +377,29 @@ static int launch_star(const LaunchDesc& L, cudaStream_t s) {
 template <int KIND, int NP, int ZS, int MINB>
 static int launch_star_kind(const LaunchDesc& L, cudaStream_t s) {
     constexpr int BATCHB = KIND == SGB_GS7 && ZS == 4 ? MINB - 1 : MINB;  // the grid entry takes registers
-    if (L.grids) return launch_star<KIND, NP, false, true, ZS, BATCHB>(L, s);
-    if (L.prm.has_box) return launch_star<KIND, NP, true, false, ZS, MINB>(L, s);
-    return launch_star<KIND, NP, false, false, ZS, MINB>(L, s);
+    if (L.grids) return launch_star<KIND, NP, false, true, false, ZS, BATCHB>(L, s);
+    if (L.again) return L.prm.has_box ? launch_star<KIND, NP, true, false, true, ZS, MINB>(L, s)
+                                      : launch_star<KIND, NP, false, false, true, ZS, MINB>(L, s);
+    if (L.prm.has_box) return launch_star<KIND, NP, true, false, false, ZS, MINB>(L, s);
+    return launch_star<KIND, NP, false, false, false, ZS, MINB>(L, s);
 }
 
-template <int KIND, int NP, bool BOX, bool BATCH>
+template <int KIND, int NP, bool BOX, bool BATCH, bool AGAIN>
 static int launch_e4(const LaunchDesc& L, cudaStream_t s) {
     StarLaunch l(L.n, 0, s);
-    SGB_CUDA(cudaLaunchKernelEx(&l.cfg, k_star7_e4<KIND, NP, BOX, BATCH, KIND == SGB_GS7 ? 6 : 10>, L.fs, L.mask, L.nn,
+    // Gray-Scott held to 56 registers: 146.6 us for 20 steps on 24,003 chunks, 148.6 with the 64 it takes otherwise
+    constexpr int MINB = KIND == SGB_HEAT7 ? 10 : AGAIN || BATCH ? 6 : 9;
+    SGB_CUDA(cudaLaunchKernelEx(&l.cfg, k_star7_e4<KIND, NP, BOX, BATCH, AGAIN, MINB>, L.fs, L.mask, L.nn,
                                 box_args<BOX>(L), L.gid, L.grids, L.g0, L.n, L.t, L.fill, L.chained));
     return SGB_OK;
 }
 
 template <int KIND, int NP>
 static int launch_e4_kind(const LaunchDesc& L, cudaStream_t s) {
-    if (L.grids) return launch_e4<KIND, NP, false, true>(L, s);
-    if (L.prm.has_box) return launch_e4<KIND, NP, true, false>(L, s);
-    return launch_e4<KIND, NP, false, false>(L, s);
+    if (L.grids) return launch_e4<KIND, NP, false, true, false>(L, s);
+    if (L.again) return L.prm.has_box ? launch_e4<KIND, NP, true, false, true>(L, s) : launch_e4<KIND, NP, false, false, true>(L, s);
+    if (L.prm.has_box) return launch_e4<KIND, NP, true, false, false>(L, s);
+    return launch_e4<KIND, NP, false, false, false>(L, s);
 }
 
 // Slices per group.  Eight halve the z-face loads and the instructions per point, four fill the chip with half

@@ -20,6 +20,15 @@ __device__ __forceinline__ float ldf1(const float* p) {
     return v;
 }
 __device__ __forceinline__ float4 splat4(float b) { return make_float4(b, b, b, b); }
+__device__ __forceinline__ uint32_t ldm4(const uint8_t* m) { return __ldg(reinterpret_cast<const uint32_t*>(m)); }
+// The background b where a quad's mask byte is 0.
+__device__ __forceinline__ float4 masked4(float4 v, uint32_t m4, float b) {
+    v.x = m4 & 0xffu ? v.x : b;
+    v.y = m4 & 0xff00u ? v.y : b;
+    v.z = m4 & 0xff0000u ? v.z : b;
+    v.w = m4 & 0xff000000u ? v.w : b;
+    return v;
+}
 
 // Two float32 values in one 64-bit register pair and the packed arithmetic on them (each half rounds as the
 // scalar instruction does).
@@ -144,6 +153,17 @@ __device__ __forceinline__ void star_store(const float4 (&c)[NP], const Quad (&l
     }
     *reinterpret_cast<float4*>(d0) = o[0];
     if (NP > 1) *reinterpret_cast<float4*>(d1) = o[NP - 1];
+}
+
+// Backgrounds for a quad's points that do not exist, beside existing ones that star_store has left alone too.
+template <int NP>
+__device__ __forceinline__ void star_rest(uint32_t m4, const float (&bd)[NP], float* d0, float* d1) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        if (!(m4 >> 8 * k & 0xffu)) {
+            d0[k] = bd[0];
+            d1[k] = bd[NP - 1];
+        }
 }
 
 // Bits of the quad's active points: EXIST and not PADDING, inside the box.
