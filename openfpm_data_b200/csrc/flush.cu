@@ -294,26 +294,37 @@ __device__ __forceinline__ uint64_t op_raw(int type, int op, uint64_t a, uint64_
     }
 }
 
-// The rest of a point's inserts folded into its first one, in insertion order, four values in flight at a time (one
-// point inserted 8192 times with an addition, the whole flush: 2053 us with one at a time, 1680 so, 1361 with
-// run_end; eight at a time spill three times as much in the kernels that call this).  A call: inlined into the
+// The rest of a point's inserts folded into its first one, in insertion order: one branch on the operation per run and
+// three values in flight (one point inserted 8192 times with an addition, the whole flush: 2053 us with a branch per
+// insert and a value at a time, 898 so and with run_end).  With four values the kernels that call this spill more:
+// 0.3 % of the 1024^3 rebuild, whose points have few inserts, for 7-30 % of such runs.  A call: inlined into the
 // unrolled rounds of its users it takes 218 registers.
-template <typename T, typename I>
-__device__ __noinline__ T fold_rest(int type, int op, T first, const T* vals, const I* sidx, uint32_t len) {
+template <int OP, typename T, typename I>
+__device__ __forceinline__ T fold_loop(int type, T first, const T* vals, const I* sidx, uint32_t len) {
+    constexpr int N = 3;
     uint64_t acc = first;
-    for (uint32_t j = 1; j < len; j += 4) {
-        T v[4];
+    for (uint32_t j = 1; j < len; j += N) {
+        T v[N];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) v[k] = j + k < len ? vals[sidx[j + k]] : T(0);
+        for (int k = 0; k < N; ++k) v[k] = j + k < len ? vals[sidx[j + k]] : T(0);
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
-            if (j + k < len) acc = op_raw(type, op, acc, (uint64_t)v[k]);
+        for (int k = 0; k < N; ++k)
+            if (j + k < len) acc = op_raw(type, OP, acc, (uint64_t)v[k]);
     }
     return (T)acc;
 }
+template <typename T, typename I>
+__device__ __noinline__ T fold_rest(int type, int op, T first, const T* vals, const I* sidx, uint32_t len) {
+    switch (op) {  // one branch per run and not per insert
+        case SGB_OP_ADD: return fold_loop<SGB_OP_ADD>(type, first, vals, sidx, len);
+        case SGB_OP_MAX: return fold_loop<SGB_OP_MAX>(type, first, vals, sidx, len);
+        case SGB_OP_MIN: return fold_loop<SGB_OP_MIN>(type, first, vals, sidx, len);
+        default: return fold_loop<SGB_OP_OR>(type, first, vals, sidx, len);
+    }
+}
 
 // The first item from e on (in sorted order) that is not k: doubling steps, as a point may fill the whole list (100 K
-// inserts of one point: 24.2 ms item by item, 17.5 so).
+// inserts of one point: a quarter of the flush's time item by item).
 template <typename K, typename I>
 __device__ __forceinline__ I run_end(const K* sk, I n, I e, K k) {
     while (e < n && sk[e] == k) {
