@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(kStarThreads, MINB)
         if (m[z] || (fill && live)) {
             const uint32_t act = active_bits<BOX>(m[z], box, cx, cy, cz + z);
             star_store<KIND, NP>(cv, lap, m[z], act, gi, bd, dst[0] + z * 64, dst[NP - 1] + z * 64);
-            if (KIND == SGB_GS7 && fill > 1) star_rest<NP>(m[z], bd, dst[0] + z * 64, dst[NP - 1] + z * 64);
+            if (KIND == SGB_GS7 && fill > 1 && (BOX || (m[z] & 0xfefefefeu))) star_rest<NP>(m[z], bd, dst[0] + z * 64, dst[NP - 1] + z * 64);
         }
 #pragma unroll
         for (int p = 0; p < NP; ++p) {
@@ -340,7 +340,7 @@ __global__ void __launch_bounds__(kStarThreads, MINB)
         cz = (int32_t)o[2] + z;
     }
     star_store<KIND, NP>(cv, lap, m, active_bits<BOX>(m, box, cx, cy, cz), gi, bd, dst[0], dst[NP - 1]);
-    if (KIND == SGB_GS7 && fill > 1) star_rest<NP>(m, bd, dst[0], dst[NP - 1]);
+    if (KIND == SGB_GS7 && fill > 1 && (BOX || (m & 0xfefefefeu))) star_rest<NP>(m, bd, dst[0], dst[NP - 1]);
 }
 
 // Consecutive steps overlap one launch's ramp-up with the previous one's tail.

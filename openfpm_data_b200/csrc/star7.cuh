@@ -155,7 +155,8 @@ __device__ __forceinline__ void star_store(const float4 (&c)[NP], const Quad (&l
     if (NP > 1) *reinterpret_cast<float4*>(d1) = o[NP - 1];
 }
 
-// Backgrounds for a quad's points that do not exist, beside existing ones that star_store has left alone too.
+// Backgrounds for a quad's points that do not exist beside existing ones that star_store leaves alone (mask bytes with
+// more than EXIST, or outside the box; it has written all other quads whole).
 template <int NP>
 __device__ __forceinline__ void star_rest(uint32_t m4, const float (&bd)[NP], float* d0, float* d1) {
 #pragma unroll

@@ -158,3 +158,20 @@ def test_captured_before_the_view_was_taken(sgb, how, kind, e, lin, size, n):
     _twin_steps(sgb, h, kind, a, b, 2)
     _twin_steps(sgb, h, kind, a, b, 2)
     _same(g, h, a + b)
+
+
+@pytest.mark.parametrize("kind,e,lin,size,n", [("HEAT7", *g) for g in GRIDS] +
+                         [("GS7", *g) for g in GRIDS if g[:2] != (8, "smb")])
+def test_boxed_steps(sgb, kind, e, lin, size, n):
+    g, h, views, mask = _pair(sgb, kind, e, lin, size, n)
+    a, b = _fields(kind)
+    box = ((3, 2, 5), (size[0] - 6, size[1] - 3, size[2] - 2))
+    gone = (mask == 0)
+    gone[g.nchunks * g.bs:] = False
+    for k in range(4):
+        x, y = (a, b) if k % 2 == 0 else (b, a)
+        g.applyStencils(getattr(sgb, kind), x, y, PRM[kind], box=box)
+        h.applyStencils(getattr(sgb, kind), x, y, PRM[kind], box=box, tiled=True)
+        for p in a if k % 2 == 0 else b:  # the source of this step, the destination of the next one
+            views[p].masked_fill_(gone, float("nan"))
+    _same(g, h, a + b)
