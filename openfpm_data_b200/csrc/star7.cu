@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(kStarThreads, MINB)
         if (m[z] || (fill && live)) {
             const uint32_t act = active_bits<BOX>(m[z], box, cx, cy, cz + z);
             star_store<KIND, NP>(cv, lap, m[z], act, gi, bd, dst[0] + z * 64, dst[NP - 1] + z * 64);
-            if (KIND == SGB_GS7 && fill > 1 && (BOX || (m[z] & 0xfefefefeu))) star_rest<NP>(m[z], bd, dst[0] + z * 64, dst[NP - 1] + z * 64);
+            if (KIND == SGB_GS7 && !BOX && fill > 1 && (m[z] & 0xfefefefeu)) star_rest<NP>(m[z], bd, dst[0] + z * 64, dst[NP - 1] + z * 64);
         }
 #pragma unroll
         for (int p = 0; p < NP; ++p) {
@@ -340,7 +340,7 @@ __global__ void __launch_bounds__(kStarThreads, MINB)
         cz = (int32_t)o[2] + z;
     }
     star_store<KIND, NP>(cv, lap, m, active_bits<BOX>(m, box, cx, cy, cz), gi, bd, dst[0], dst[NP - 1]);
-    if (KIND == SGB_GS7 && fill > 1 && (BOX || (m & 0xfefefefeu))) star_rest<NP>(m, bd, dst[0], dst[NP - 1]);
+    if (KIND == SGB_GS7 && !BOX && fill > 1 && (m & 0xfefefefeu)) star_rest<NP>(m, bd, dst[0], dst[NP - 1]);
 }
 
 // Consecutive steps overlap one launch's ramp-up with the previous one's tail.
@@ -388,7 +388,7 @@ template <int KIND, int NP, bool BOX, bool BATCH, bool AGAIN>
 static int launch_e4(const LaunchDesc& L, cudaStream_t s) {
     StarLaunch l(L.n, 0, s);
     // Gray-Scott held to 56 registers: 146.6 us for 20 steps on 24,003 chunks, 148.6 with the 64 it takes otherwise
-    constexpr int MINB = KIND == SGB_HEAT7 ? 10 : AGAIN || BATCH ? 6 : 9;
+    constexpr int MINB = KIND == SGB_HEAT7 ? 10 : AGAIN || BATCH || BOX ? 6 : 9;
     SGB_CUDA(cudaLaunchKernelEx(&l.cfg, k_star7_e4<KIND, NP, BOX, BATCH, AGAIN, MINB>, L.fs, L.mask, L.nn,
                                 box_args<BOX>(L), L.gid, L.grids, L.g0, L.n, L.t, L.fill, L.chained));
     return SGB_OK;

@@ -156,7 +156,7 @@ __device__ __forceinline__ void star_store(const float4 (&c)[NP], const Quad (&l
 }
 
 // Backgrounds for a quad's points that do not exist beside existing ones that star_store leaves alone (mask bytes with
-// more than EXIST, or outside the box; it has written all other quads whole).
+// more than EXIST; it has written all other quads whole).  Steps without a box only: solves.
 template <int NP>
 __device__ __forceinline__ void star_rest(uint32_t m4, const float (&bd)[NP], float* d0, float* d1) {
 #pragma unroll

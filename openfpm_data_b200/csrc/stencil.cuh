@@ -79,7 +79,8 @@ struct LaunchDesc {
     StencilParams prm;
     int64_t t;
     int fill;                // quads without an existing point are written too (dst may hold anything there); 2: so is
-                             // every other point that does not exist (1: Gray-Scott not beside points it leaves alone)
+                             // every other point that does not exist (1: Gray-Scott not beside points it leaves
+                             // alone); launches with a box take 0 or 1
     int again;               // single grids: the source may hold anything at points that do not exist
     int chained;             // follows a launch over the same masks and neighbours in the same call
 };
