@@ -234,12 +234,12 @@ int sgb_nchunks(const sgb_grid* g, int64_t* n);
 
 /* Non-owning device views (private_get_index_array / private_get_data_array,
  * SparseGridGpu.hpp:1959-1990).  Invalidated by sgb_flush.
- * Points that do not exist read as the property's background.  A caller that
- * keeps a view and writes such points: a 7-point step that writes the property
- * puts the background back; a step that reads it does so on 4^3 chunks and on
- * Morton ids, and so does sgb_run_steps on grids of at most 4 chunks per SM.
- * Elsewhere, and for the 27-point stencils, ask for the view again after the
- * writes and before the property is read as a source. */
+ * Points that do not exist read as the property's background, also when a
+ * caller writes them through a view that it keeps: in every property that a
+ * 7-point step writes, and in those that one reads on 4^3 chunks, on Morton
+ * ids and in sgb_run_steps on grids of at most 4 chunks per SM.  Elsewhere,
+ * and for the 27-point stencils, ask for the view again after such writes and
+ * before the property is read as a source. */
 int sgb_index_buffer(sgb_grid* g, const int64_t** dev);
 int sgb_data_buffer(sgb_grid* g, int prop, void** dev);
 int sgb_mask_buffer(sgb_grid* g, uint8_t** dev);

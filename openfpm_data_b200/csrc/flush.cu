@@ -994,6 +994,7 @@ static int flush_impl(sgb_grid* g, const int* ops, int bits, cudaStream_t s) {
         std::swap(g->mask, g->mask2);
         for (int p = 0; p < g->nprop; ++p) {
             std::swap(g->data[p], g->data2[p]);
+            if (g->exposed[p] && nold > 0) g->clean[p] = false;  // what the caller wrote has moved along
             g->exposed[p] = false;
         }
         g->cap = cap2;

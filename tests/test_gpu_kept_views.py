@@ -175,3 +175,31 @@ def test_boxed_steps(sgb, kind, e, lin, size, n):
         for p in a if k % 2 == 0 else b:  # the source of this step, the destination of the next one
             views[p].masked_fill_(gone, float("nan"))
     _same(g, h, a + b)
+
+
+@pytest.mark.parametrize("kind", ["HEAT7", "GS7"])
+@pytest.mark.parametrize("e,lin,size,n", GRIDS)
+def test_writes_before_the_map_grows(sgb, kind, e, lin, size, n):
+    """A flush with new chunks moves the map to other buffers, what the caller wrote included, and ends its views."""
+    g, h, views, mask = _pair(sgb, kind, e, lin, size, n)
+    a, b = _fields(kind)
+    gone = (mask == 0)
+    gone[g.nchunks * g.bs:] = False
+    g.applyStencils(getattr(sgb, kind), a, b, PRM[kind])
+    _twin_steps(sgb, h, kind, a, b, 1)
+    for p in a + b:
+        views[p].masked_fill_(gone, float("nan"))
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(n)
+    pts = torch.stack([torch.randint(0, s, (4000,), generator=gen, device="cuda") for s in size], 1).to(torch.int32)
+    vals = [torch.rand(4000, generator=gen, device="cuda") for _ in range(4)]
+    before = g.nchunks
+    for x in (g, h):
+        x.insert(pts, vals)
+        x.flush(["sRight_"] * 4)
+    assert g.nchunks > before
+    for k in range(2):
+        x, y = (a, b) if k == 0 else (b, a)
+        g.applyStencils(getattr(sgb, kind), x, y, PRM[kind])
+        h.applyStencils(getattr(sgb, kind), x, y, PRM[kind], tiled=True)
+    _same(g, h, a + b)
